@@ -63,6 +63,10 @@ static thread_local std::string g_noctx_err;
     tn::Ctx* _c = (ctxptr);         \
     try {
 #define TN_API_END                                                  \
+    if (_c && _c->tc_pending) {                                     \
+        _c->tc_pending = false;                                     \
+        tn::tc_check_error(_c);                                     \
+    }                                                               \
     return TN_OK;                                                   \
     }                                                               \
     catch (const tn::Error& e) {                                    \

@@ -70,7 +70,7 @@ struct Ctx {
     int sm_count = 0;
     // reusable scratch for the hot path
     Scratch s_gram, s_eigval, s_work, s_x, s_y, s_t1, s_t2, s_dot, s_coef, s_mixa, s_mixb, s_mixc,
-        s_mixd, s_mixe, s_mixf, s_eig, s_splitk;
+        s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz;
     int* d_info = nullptr;
     // grid-barrier words of the eigensolver's cooperative kernels: arrival
     // count, generation, and an error word set when a bounded wait ran out
@@ -82,6 +82,8 @@ struct Ctx {
     // split-K FP64 GEMMs draw partial buffers from the pool; callers that must
     // not allocate turn them off
     bool splitk = true;
+    // a tensor-core kernel of the FP64 path ran since d_err was last read
+    bool tc_pending = false;
     double* h_pinned = nullptr;  // small pinned staging area
     size_t h_pinned_n = 0;
     // kernel profiler: CUDA events around launches, per class
@@ -171,6 +173,13 @@ void zgemm(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha
            int64_t lda, int64_t strideA, const cplx* B, int64_t ldb, int64_t strideB, cplx beta,
            cplx* C, int64_t ldc, int64_t strideC, int64_t batch = 1, bool lower_only = false);
 
+// The same product on the tensor cores (tc_zgemm.cu), FP64 accurate, one batch;
+// false when it does not take the call (no room for its operand planes, K
+// above 2^16).
+bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
+              int64_t lda, const cplx* B, int64_t ldb, cplx beta, cplx* C, int64_t ldc,
+              bool lower_only);
+
 // out[a + lda_o*J + ldc_o*c] (=|+=) sum_I in[a + lda_i*I + ldc_i*c] * M[I + nI*J]
 void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int nJ, int64_t na,
                  int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o, int64_t ldc_o,
@@ -211,7 +220,8 @@ void scale_rows(Ctx* ctx, cplx* X, int64_t k, int64_t n, const double* s, int in
 // their sum.
 struct KeepResult { int64_t k; double total; double discarded; };
 // dinfo (device, optional): an eigensolver status read back in the same
-// synchronisation; nonzero raises TN_ERR_NUMERIC.
+// synchronisation with the tensor-core wait status; nonzero raises
+// TN_ERR_TIMEOUT.
 KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double cutoff,
                      int64_t maxdim, int64_t mindim, double* dS, const double* dtotal = nullptr,
                      const int* dinfo = nullptr);

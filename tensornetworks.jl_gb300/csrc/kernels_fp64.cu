@@ -113,36 +113,70 @@ __global__ void __launch_bounds__(256) zgemm_kernel(int64_t M, int64_t N, int64_
     }
 }
 
-// Thin or small products (min(m, n) < 48): one thread per output element, a
-// plain dot product over k.  The 64x64 tile kernel would spend GB300's scarce
-// FP64 issue slots on zero padding there (a 10 x 10 product costs a full tile).
+// Small and thin products: one thread per output element and K slice, a plain
+// dot product; blockDim = (outputs, S) and the S slices of an element are added
+// in slice order through shared memory.  GB300 issues one FP64 warp instruction
+// per 16 clocks and SM, so operands read straight from L1/L2 keep that pipe
+// busy and no tile is padded: what counts is that the outputs, times the
+// slices where they are few, reach every SM.
+constexpr int ZS_T = 512;  // most threads of a block
+
 template <int OPA, int OPB>
-__global__ void __launch_bounds__(64) zgemm_small_kernel(int64_t M, int64_t N, int64_t K, cplx alpha,
-                                                         const cplx* __restrict__ A, int64_t lda,
-                                                         int64_t sA, const cplx* __restrict__ B,
-                                                         int64_t ldb, int64_t sB, cplx beta,
-                                                         cplx* __restrict__ C, int64_t ldc,
-                                                         int64_t sC, int64_t batch, int lower) {
+__global__ void __launch_bounds__(ZS_T)
+    zgemm_small_kernel(int64_t M, int64_t N, int64_t K, cplx alpha, const cplx* __restrict__ A,
+                       int64_t lda, int64_t sA, const cplx* __restrict__ B, int64_t ldb, int64_t sB,
+                       cplx beta, cplx* __restrict__ C, int64_t ldc, int64_t sC, int64_t batch,
+                       int lower) {
+    __shared__ cplx part[ZS_T];
+    const int tx = threadIdx.x, ty = threadIdx.y, OX = blockDim.x, S = blockDim.y;
     const int64_t total = M * N * batch;
     const bool use_beta = (beta.x != 0.0 || beta.y != 0.0);
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t kc = (K + S - 1) / S, l0 = ty * kc, l1 = min(K, l0 + kc);
+    for (int64_t base = blockIdx.x * (int64_t)OX; base < total; base += (int64_t)gridDim.x * OX) {
+        const int64_t idx = base + tx;
         const int64_t i = idx % M, j = (idx / M) % N, b = idx / (M * N);
-        if (lower && i < j) continue;  // only the lower triangle is wanted
-        const cplx* a = A + b * sA;
-        const cplx* bb = B + b * sB;
+        const bool on = idx < total && !(lower && i < j);  // only the lower triangle is wanted
         cplx acc = cmk(0.0, 0.0);
-        for (int64_t l = 0; l < K; ++l) {
-            cplx x = (OPA == OP_N || OPA == OP_R) ? a[i + l * lda] : a[l + i * lda];
-            if (OPA == OP_C || OPA == OP_R) x.y = -x.y;
-            cplx y = (OPB == OP_N || OPB == OP_R) ? bb[l + j * ldb] : bb[j + l * ldb];
-            if (OPB == OP_C || OPB == OP_R) y.y = -y.y;
-            acc = cfma(x, y, acc);
+        if (on) {
+            const cplx* a = A + b * sA + ((OPA == OP_N || OPA == OP_R) ? i : i * lda);
+            const cplx* bb = B + b * sB + ((OPB == OP_N || OPB == OP_R) ? j * ldb : j);
+            const int64_t da = (OPA == OP_N || OPA == OP_R) ? lda : 1;
+            const int64_t db = (OPB == OP_N || OPB == OP_R) ? 1 : ldb;
+            cplx acc1 = cmk(0.0, 0.0);
+            auto step = [&](cplx x, cplx y, cplx& s) {
+                if (OPA == OP_C || OPA == OP_R) x.y = -x.y;
+                if (OPB == OP_C || OPB == OP_R) y.y = -y.y;
+                s = cfma(x, y, s);
+            };
+            int64_t l = l0;
+            for (; l + 3 < l1; l += 4) {  // four loads in flight, two FMA chains
+                cplx x[4], y[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    x[u] = a[(l + u) * da];
+                    y[u] = bb[(l + u) * db];
+                }
+                step(x[0], y[0], acc);
+                step(x[1], y[1], acc1);
+                step(x[2], y[2], acc);
+                step(x[3], y[3], acc1);
+            }
+            for (; l < l1; ++l) step(a[l * da], bb[l * db], acc);
+            acc = cadd(acc, acc1);
         }
-        cplx* c = C + b * sC + i + j * ldc;
-        cplx v = cmul(alpha, acc);
-        if (use_beta) v = cfma(beta, *c, v);
-        *c = v;
+        if (S > 1) {
+            part[ty * OX + tx] = acc;
+            __syncthreads();
+            if (ty == 0)
+                for (int s = 1; s < S; ++s) acc = cadd(acc, part[s * OX + tx]);
+        }
+        if (on && ty == 0) {
+            cplx* c = C + b * sC + i + j * ldc;
+            cplx v = cmul(alpha, acc);
+            if (use_beta) v = cfma(beta, *c, v);
+            *c = v;
+        }
+        if (S > 1) __syncthreads();
     }
 }
 
@@ -170,12 +204,19 @@ void zgemm_small_dispatch_b(Ctx* ctx, Op opb, int64_t m, int64_t n, int64_t k, c
                             const cplx* A, int64_t lda, int64_t sA, const cplx* B, int64_t ldb,
                             int64_t sB, cplx beta, cplx* C, int64_t ldc, int64_t sC, int64_t batch,
                             int lower) {
-    int64_t blocks = (m * n * batch + 63) / 64;
-    const int64_t cap = (int64_t)ctx->sm_count * 16;
-    if (blocks > cap) blocks = cap;
-    const unsigned g = (unsigned)(blocks < 1 ? 1 : blocks);
+    // Outputs per block: 32, fewer while the blocks would not reach every SM
+    // twice (16 x 16 outputs, K = 1024: 37 us on 8 SMs, 7 us on 128); then K
+    // slices of at least 16 terms up to a full warp, and on to eight warps per
+    // SM.
+    const int64_t outs = m * n * batch;
+    int OX = 32, S = 1;
+    while (OX > 2 && outs < 2 * OX * (int64_t)ctx->sm_count && k >= 16 * (64 / OX)) OX /= 2;
+    while (OX * S < 32 && k >= 32 * S) S *= 2;
+    while (OX * S < ZS_T && outs / OX * ((OX * S + 31) / 32) < 8 * (int64_t)ctx->sm_count && k >= 32 * S) S *= 2;
+    const unsigned g = (unsigned)std::min<int64_t>((outs + OX - 1) / OX, (int64_t)ctx->sm_count * 64);
+    const dim3 th((unsigned)OX, (unsigned)S);
     switch (opb) {
-#define TN_ZS(OB) case OB: zgemm_small_kernel<OPA, OB><<<g, 64, 0, ctx->stream>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, lower); break;
+#define TN_ZS(OB) case OB: zgemm_small_kernel<OPA, OB><<<g, th, 0, ctx->stream>>>(m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, lower); break;
         TN_ZS(OP_N) TN_ZS(OP_T) TN_ZS(OP_C) TN_ZS(OP_R)
 #undef TN_ZS
     }
@@ -444,6 +485,7 @@ __global__ void row_norms_kernel(const cplx* __restrict__ Y, int64_t k, int64_t 
 struct KeepDev {
     int64_t k;
     double total, discarded;
+    int64_t err;  // error words of the kernels before: grid barriers, tensor-core waits
 };
 
 __device__ inline double s2_at(const double* lam, int64_t n, int64_t i) {
@@ -455,6 +497,8 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
                                                          int64_t sz, double cutoff, int64_t maxdim,
                                                          int64_t mindim, double* __restrict__ S_out,
                                                          const double* __restrict__ dtotal,
+                                                         const int* __restrict__ dinfo,
+                                                         const int* __restrict__ derr,
                                                          KeepDev* __restrict__ res) {
     __shared__ double wsum[32];
     __shared__ long long wcnt[32];
@@ -531,8 +575,14 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
         double d = rest;
         for (int w = 0; w < nw; ++w) d += wsum[w];
         res->discarded = total > 0 ? d / total : 0.0;
+        res->err = (dinfo ? *dinfo : 0) | *derr;
     }
 }
+
+// Multiply-adds from which the tensor-core product is the faster one: it takes
+// five stream operations (27 us at any size up to 256 x 128 x 128 = 4.2 M, where
+// the per-output kernel takes 37 us; at 128^3 = 2.1 M it is 27 us against 23).
+constexpr double ZTC_MIN = 2.5e6;
 
 inline int grid_for(Ctx* ctx, int64_t n, int threads = 256) {
     int64_t g = (n + threads - 1) / threads;
@@ -556,7 +606,17 @@ void zgemm(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha
     }
     ProfScope ps(ctx, 1, (lower ? 0.5 : 1.0) * 8.0 * m * n * (double)std::max<int64_t>(k, 0) * batch,
                  16.0 * (double)(m * k + k * n + m * n) * batch);
-    if (std::min(m, n) < 48) {
+    // Large products run on the tensor cores.  Thin ones (a side below 16) read
+    // more than they multiply: there the operand conversion (64 bytes written
+    // per entry) costs more than the FP64 pipe.
+    const double work = (lower ? 0.5 : 1.0) * (double)m * n * k * batch;
+    const bool tc = ctx->splitk && batch == 1 && std::min(m, n) >= 16 && k >= 8 && work >= ZTC_MIN;
+    if (tc && zgemm_tc(ctx, opa, opb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only)) return;
+    // Otherwise (small products, and callers that must not allocate): a 64 x 64
+    // tile keeps one SM busy for 4.1 us per K entry at two FP64 FMAs per clock
+    // (64^3: 263 us), the per-output kernel spreads the same work over the SMs
+    // (64^3: 7 us).  Tiles, with their reuse, pay once they fill the SMs.
+    if (std::min(m, n) < 48 || work < 6.0e7) {
         switch (opa) {
             case OP_N: zgemm_small_dispatch_b<OP_N>(ctx, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, lower); break;
             case OP_T: zgemm_small_dispatch_b<OP_T>(ctx, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, lower); break;
@@ -774,22 +834,21 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
     TN_REQUIRE(sz <= n, "keep_rule: more singular values than eigenvalues");
     KeepDev* dres = static_cast<KeepDev*>(ctx->s_coef.get(ctx, 256));
     keep_rule_kernel<<<1, 1024, 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, dtotal,
-                                                  dres);
+                                                  dinfo, ctx->d_err, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
     double* h = ctx->pinned(4);
     TN_CHECK_CUDA(cudaMemcpyAsync(h, dres, sizeof(KeepDev), cudaMemcpyDeviceToHost, ctx->stream));
-    if (dinfo)
-        TN_CHECK_CUDA(cudaMemcpyAsync(reinterpret_cast<int*>(h + 3), dinfo, sizeof(int),
-                                      cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
-    if (dinfo && *reinterpret_cast<int*>(h + 3) != 0) {
-        // the eigensolver's error word: a bounded grid barrier ran out
-        TN_CHECK_CUDA(cudaMemsetAsync(const_cast<int*>(dinfo), 0, sizeof(int), ctx->stream));
-        throw Error(TN_ERR_TIMEOUT, "eigensolver: a bounded grid barrier ran out");
-    }
+    ctx->tc_pending = false;
     KeepDev r;
     memcpy(&r, h, sizeof(KeepDev));
+    if (r.err != 0) {
+        if (dinfo)
+            TN_CHECK_CUDA(cudaMemsetAsync(const_cast<int*>(dinfo), 0, sizeof(int), ctx->stream));
+        TN_CHECK_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+        throw Error(TN_ERR_TIMEOUT, "truncated split: a bounded device wait ran out");
+    }
     return KeepResult{r.k, r.total, r.discarded};
 }
 
