@@ -989,7 +989,7 @@ int32_t tn_eigh_top(tn_ctx* h, int64_t n, const double* G, int64_t want, double*
     Ctx* ctx = &h->c;
     DBuf dG(ctx, 16 * (size_t)n * n), dV(ctx, 16 * (size_t)n * want), dL(ctx, 8 * (size_t)want);
     h2d(ctx, dG.p, G, 16 * (size_t)n * n);
-    eig_top(ctx, dG.c(), n, want, dL.d(), dV.c());
+    eig_top(ctx, dG.c(), n, want, dL.d(), dV.c(), false);
     std::vector<double> asc(want);
     d2h(ctx, asc.data(), dL.p, 8 * (size_t)want);
     d2h(ctx, V, dV.p, 16 * (size_t)n * want);

@@ -70,11 +70,12 @@ struct Ctx {
     int sm_count = 0;
     // reusable scratch for the hot path
     Scratch s_gram, s_eigval, s_work, s_x, s_y, s_t1, s_t2, s_dot, s_coef, s_mixa, s_mixb, s_mixc,
-        s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz;
+        s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz, s_trd, s_bt, s_dc;
     int* d_info = nullptr;
     // grid-barrier words of the eigensolver's cooperative kernels: arrival
     // count, generation, and an error word set when a bounded wait ran out
     unsigned* d_bar = nullptr;
+    int trd_clusters = -1;  // 16-block clusters the GPU holds at once (-1: not asked yet)
     int* d_err = nullptr;  // set by device code when a bounded wait runs out
     // mixed precision on: environment updates and truncation projections run
     // on the tensor cores (set for the duration of a mixed-precision sweep)
@@ -239,8 +240,16 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
 // G destroyed), hand-written FP64 kernels (eig.cu): lam_asc[want-1-g] is the
 // g-th largest eigenvalue and X[:, g] (n x want) its eigenvector.  No host
 // synchronisation; a timed-out grid barrier leaves ctx->d_bar[2] nonzero.
-void eig_top(Ctx* ctx, cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X);
-// Full eigen-decomposition, ascending: eigenvalues in dlam[0..n), eigenvectors
+// psd: G is positive semidefinite (a Gram matrix).
+void eig_top(Ctx* ctx, cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X, bool psd);
+// Householder tridiagonalisation (hetrd.cu): T in (d, e), reflector j in column j
+// of G (rows j+1.., explicit first entry, zeros above), H_j = I - tau_j v_j v_j^H.
+void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool psd, int* perm);
+// Top `want` eigenpairs of the real symmetric tridiagonal (d, e) (dc.cu): lam_asc
+// ascending, Z (n x want) in descending order.
+void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t want,
+                 double* lam_asc, double* Z);
+// Full eigen-decomposition of a Gram matrix, ascending: eigenvalues in dlam[0..n), eigenvectors
 // overwrite G (column j belongs to dlam[j]); synchronises and checks.
 void heev_full(Ctx* ctx, cplx* G, int64_t n, double* dlam);
 

@@ -1,5 +1,4 @@
-// Device helpers shared by the Hermitian eigensolvers: the grid-wide one of
-// the truncated split (eig.cu) and the one-block one inside the trajectory
+// Device helpers of the one-block Hermitian eigensolver inside the trajectory
 // engine (qjmc_engine.cu).
 #pragma once
 
@@ -8,7 +7,6 @@
 namespace tn {
 namespace eigdev {
 
-constexpr int BIS_W = 4;  // lanes per eigenvalue in the bisection
 constexpr int BT_G = 4;   // reflectors per compact-WY group of the back-transformation
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -171,17 +169,9 @@ __device__ __forceinline__ void bisect_group_w(int g, int m, unsigned grp,
 
 }
 
-__device__ __forceinline__ void bisect_group(int g, int m, unsigned grp, const double* __restrict__ d,
-                                             const double* __restrict__ e2,
-                                             const float* __restrict__ d32,
-                                             const float* __restrict__ e2f, int t, int want,
-                                             const double* __restrict__ bounds,
-                                             double* __restrict__ lam_desc,
-                                             double* __restrict__ lam_asc) {
-    bisect_group_w<BIS_W>(g, m, grp, d, e2, d32, e2f, t, want, bounds, lam_desc, lam_asc);
-}
-
-// Inverse iteration for vector g; see stein_kernel.
+// Inverse iteration for vector g: (T - shift_g) z = b solved three times from a
+// pseudo-random b; factors and working vector stored [k][want], the normalised
+// vector column-major into Z (t x want).
 __device__ __forceinline__ void stein_vector(int g, const double* __restrict__ d,
                                              const double* __restrict__ e, int t, int want,
                                              const double* __restrict__ shift,
@@ -270,152 +260,6 @@ __device__ __forceinline__ void stein_vector(int g, const double* __restrict__ d
     const double inv = s2 > 0.0 ? 1.0 / sqrt(s2) : 0.0;
     double* z = Z + (size_t)g * t;
     for (int k = 0; k < t; ++k) z[k] = zw[(size_t)k * W + g] * inv;
-
-}
-
-// Column k-1-w of Q from the QR reflectors, by one warp (lane); see
-// qr_form_kernel.
-__device__ __forceinline__ void qr_form_column(int64_t w, int lane, const double* __restrict__ Zr,
-                                               int64_t t, int64_t k,
-                                               const double* __restrict__ qtau,
-                                               const double* __restrict__ rdiag,
-                                               double* __restrict__ Q) {
-    const int64_t c = k - 1 - w;  // column c costs c+1 reflectors: the heaviest start first
-    double* q = Q + c * t;
-    for (int64_t i = lane; i < t; i += 32) q[i] = (i == c) ? 1.0 : 0.0;
-    __syncwarp();
-    for (int64_t j = c; j >= 0; --j) {
-        const double tau = qtau[j];
-        if (tau == 0.0) continue;
-        const double* v = Zr + j * t;  // v[j] = 1 implicit
-        double s0 = (lane == 0) ? q[j] : 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int64_t i = j + 1 + lane;
-        for (; i + 96 < t; i += 128) {
-            s0 = fma(v[i], q[i], s0);
-            s1 = fma(v[i + 32], q[i + 32], s1);
-            s2 = fma(v[i + 64], q[i + 64], s2);
-            s3 = fma(v[i + 96], q[i + 96], s3);
-        }
-        for (; i < t; i += 32) s0 = fma(v[i], q[i], s0);
-        double s = warp_sum((s0 + s1) + (s2 + s3));
-        s = __shfl_sync(0xffffffffu, s, 0) * tau;
-        for (int64_t i = j + lane; i < t; i += 32) q[i] -= s * (i == j ? 1.0 : v[i]);
-        __syncwarp();
-    }
-    // R's diagonal carries the sign that maps the input column onto Q's column
-    if (rdiag[c] < 0.0)
-        for (int64_t i = lane; i < t; i += 32) q[i] = -q[i];
-
-}
-
-// Compact-WY factor of reflector group q by one warp (lane); see
-// wy_factor_kernel.
-__device__ __forceinline__ void wy_group(int64_t q, int lane, const cplx* __restrict__ A, int64_t n,
-                                         const cplx* __restrict__ tau,
-                                         cplx* __restrict__ Tg) {
-    const int64_t a = q * BT_G;
-    const int nr = (int)min((int64_t)BT_G, (n - 1) - a);
-    // S[c][r] = v_c^H v_r for c < r
-    double sre[BT_G][BT_G], sim[BT_G][BT_G];
-#pragma unroll
-    for (int c = 0; c < BT_G; ++c)
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) sre[c][r] = sim[c][r] = 0.0;
-    for (int64_t i = a + 1 + lane; i < n; i += 32) {
-        cplx v[BT_G];
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) v[r] = r < nr ? refl(A, n, a + r, i) : cmk(0, 0);
-#pragma unroll
-        for (int c = 0; c < BT_G; ++c)
-#pragma unroll
-            for (int r = c + 1; r < BT_G; ++r) {
-                sre[c][r] = fma(v[c].x, v[r].x, fma(v[c].y, v[r].y, sre[c][r]));
-                sim[c][r] = fma(v[c].x, v[r].y, fma(-v[c].y, v[r].x, sim[c][r]));
-            }
-    }
-#pragma unroll
-    for (int c = 0; c < BT_G; ++c)
-#pragma unroll
-        for (int r = c + 1; r < BT_G; ++r) {
-            sre[c][r] = warp_sum(sre[c][r]);
-            sim[c][r] = warp_sum(sim[c][r]);
-        }
-    if (lane != 0) return;
-    cplx T[BT_G][BT_G];
-#pragma unroll
-    for (int c = 0; c < BT_G; ++c)
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) T[c][r] = cmk(0, 0);
-    for (int r = 0; r < nr; ++r) {
-        const cplx tr = tau[a + r];
-        T[r][r] = tr;
-        cplx z[BT_G];
-        for (int c = 0; c < r; ++c) z[c] = cmul(cmk(-tr.x, -tr.y), cmk(sre[c][r], sim[c][r]));
-        for (int c = 0; c < r; ++c) {  // T[0:r, r] = T[0:r, 0:r] z
-            cplx acc = cmk(0, 0);
-            for (int u = c; u < r; ++u) acc = cfma(T[c][u], z[u], acc);
-            T[c][r] = acc;
-        }
-    }
-    for (int c = 0; c < BT_G; ++c)
-        for (int r = 0; r < BT_G; ++r) Tg[q * BT_G * BT_G + c + BT_G * r] = T[c][r];
-
-}
-
-// Column c of X = Q_trd Z by one warp (lane); see backtransform_kernel.
-__device__ __forceinline__ void bt_column(int64_t c, int lane, const cplx* __restrict__ A, int64_t n,
-                                          const cplx* __restrict__ Tg, int64_t ngroups,
-                                          const double* __restrict__ Z,
-                                          cplx* __restrict__ X) {
-    cplx* x = X + c * n;
-    const double* z = Z + c * n;
-    for (int64_t i = lane; i < n; i += 32) x[i] = cmk(z[i], 0.0);
-    __syncwarp();
-    for (int64_t q = ngroups - 1; q >= 0; --q) {
-        const int64_t a = q * BT_G;
-        const int nr = (int)min((int64_t)BT_G, (n - 1) - a);
-        double sr[BT_G], si[BT_G];
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) sr[r] = si[r] = 0.0;
-        for (int64_t i = a + 1 + lane; i < n; i += 32) {
-            const cplx xi = x[i];
-#pragma unroll
-            for (int r = 0; r < BT_G; ++r) {
-                if (r < nr) {
-                    const cplx v = refl(A, n, a + r, i);  // conj(v) x as two FMA chains
-                    sr[r] = fma(v.x, xi.x, fma(v.y, xi.y, sr[r]));
-                    si[r] = fma(v.x, xi.y, fma(-v.y, xi.x, si[r]));
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) {
-            sr[r] = __shfl_sync(0xffffffffu, warp_sum(sr[r]), 0);
-            si[r] = __shfl_sync(0xffffffffu, warp_sum(si[r]), 0);
-        }
-        // coefficients u = T s
-        const cplx* T = Tg + q * BT_G * BT_G;
-        cplx u[BT_G];
-#pragma unroll
-        for (int r = 0; r < BT_G; ++r) {
-            cplx acc = cmk(0, 0);
-#pragma unroll
-            for (int v = r; v < BT_G; ++v) acc = cfma(T[r + BT_G * v], cmk(sr[v], si[v]), acc);
-            u[r] = acc;
-        }
-        for (int64_t i = a + 1 + lane; i < n; i += 32) {
-            cplx xi = x[i];
-#pragma unroll
-            for (int r = 0; r < BT_G; ++r)
-                if (r < nr) {  // x -= u v, fused
-                    const cplx v = refl(A, n, a + r, i);
-                    xi.x = fma(-u[r].x, v.x, fma(u[r].y, v.y, xi.x));
-                    xi.y = fma(-u[r].x, v.y, fma(-u[r].y, v.x, xi.y));
-                }
-            x[i] = xi;
-        }
-        __syncwarp();
-    }
 
 }
 

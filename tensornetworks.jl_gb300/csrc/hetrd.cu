@@ -1,0 +1,708 @@
+// Householder reduction of a Hermitian matrix to a real symmetric tridiagonal,
+// G = Q T Q^H, in fixed point (fixp.cuh): step 1 of the eigensolver (eig.cu).
+//
+// One thread-block cluster holds the whole matrix in its shared memories up to
+// order 405 (sixteen blocks), one cooperative grid in global memory above.  Row
+// i belongs to block i mod C.  Step j:
+//   A. a warp per row applies the pending rank-2 update of step j-1 to the
+//      row and sums its product with v, in one pass, while a ninth warp forms
+//      the reflector's scalars in FP64 (its only FP64 work: about thirty
+//      instructions of 64 clocks); the row's product, its entry of column j+1
+//      and its share of v^H A v go to every block;
+//   B. after one barrier (cluster: 0.2 us, grid: 1.2 us) every block forms w,
+//      column j+1 with this step's update and its exact squared norm itself.
+// The FP64 version spent 8.7 us per step at order 256: a 1.9 us grid barrier,
+// five block sums of ten dependent 64-clock additions each and a serial
+// square root and two divisions (2,000 clocks).
+//
+// Reflector j is kept as V[j n + i] (i > j; integers of unit 2^-56 with the
+// first entry explicit) and tau[j]: H_j = I - tau_j v_j v_j^H.
+#include <climits>
+#include <cmath>
+
+#include "common.cuh"
+#include "fixp.cuh"
+#include "grid_dev.cuh"
+
+namespace tn {
+
+namespace {
+
+using namespace fixp;
+using namespace griddev;
+
+constexpr int HT = 288;       // threads: eight row warps and the scalar warp
+constexpr int HM = 256;       // threads of the row warps
+constexpr int HC = 16;        // blocks of a full cluster
+
+struct TrdOut {
+    zint* V;      // n x n, column j: reflector j
+    cplx* tau;    // n
+    ll* di;       // n: diagonal, unit 2^(f - 61 - dsh)
+    ll* ei;       // n: off-diagonal, unit 2^(f - 61 - esh)
+    int *dsh, *esh;  // n
+    int* f;       // exponent of the scale, or INT_MIN: the matrix is not finite
+    int* perm;    // n: row of G that became row l, when psd
+};
+
+struct TrdIn {
+    const cplx* G;  // n x n, lower triangle
+    int n, psd;
+    TrdOut o;
+    zint* A;          // grid form: n x n rows in global memory
+    zint* mp;         // grid form: mailbox, two buffers of n entries each
+    zint* ma;
+    ll *md, *mq;
+    zint* xr;         // grid form: a block's copy of the column
+    unsigned* part;   // grid form: per-block scale partials
+    unsigned* bar;    // grid form: arrival counter (zero at launch)
+    int* err;
+};
+
+__device__ __forceinline__ void bar_named(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// address in block `rank`'s shared memory of this block's address p
+__device__ __forceinline__ uint32_t map_shared(const void* p, unsigned rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+// stores that report their bytes to the receiving block's mbarrier
+__device__ __forceinline__ void st_async(uint32_t a, zint v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(a),
+                 "l"(v.x), "l"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t a, ll v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+                 "l"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, unsigned v) {
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// Waits for a phase of this block's mbarrier; false when the bound runs out.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
+    uint64_t t0 = 0;
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        const uint64_t t = hclock();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > HWAIT_NS) return false;
+    }
+}
+
+__device__ __forceinline__ ll warp_sum64(ll v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+struct ShCtl {
+    ll q[8];             // grid form: partial v^H A v of the warps
+    ll qt[2][8 * HC];    // cluster form: every warp's share, from every block
+    uint64_t mbar[2];    // cluster form: a step's exchange has arrived
+    int abort;
+    unsigned S[3][8];    // squared norm, 24-bit limbs, triple buffered by step
+    int vm[3];           // largest entry of v 2^-e, log2, likewise
+    int emin[3];         // smallest exponent of the rows left, likewise
+    int shift[3];        // whether any exponent changed, likewise
+    int em, c;           // smallest exponent of the rows left, the column's exponent
+    zint alpha;          // first entry of the column before the shift
+    ll beta;
+    zint v1, tau;
+    ll c2;
+    unsigned part[2 * HC];  // scale partials of the cluster's blocks
+};
+
+__device__ __forceinline__ zint ld_zint(const zint* p) {
+    const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(p));
+    return zint{v.x, v.y};
+}
+
+// x 2^s rounded to an integer (|x 2^s| < 2^62; denormal x counts as zero)
+__device__ __forceinline__ ll to_fix(double x, int s) {
+    const ll b = __double_as_longlong(x);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    if (ex == 0) return 0;
+    const ll m = (b & 0xfffffffffffffll) | 0x10000000000000ll;
+    const ll r = sft(m, ex - 1075 + s);
+    return b < 0 ? -r : r;
+}
+
+template <bool GRID>
+__global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
+    extern __shared__ __align__(16) unsigned char hsm[];
+    __shared__ ShCtl sh;
+    const int n = p.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int C = GRID ? (int)gridDim.x : (int)cluster_size();
+    const int b = GRID ? (int)blockIdx.x : (int)cluster_rank();
+    const int R = (n + C - 1) / C;
+    // shared memory: the column, v's limbs for products, v's and w's for the pending
+    // update, exponents and their pending change; in the cluster form the mailbox
+    // and the rows
+    int4* vD = reinterpret_cast<int4*>(hsm);
+    int4* vU = vD + n;
+    int4* wU = vU + n;
+    zint* mp = GRID ? p.mp : reinterpret_cast<zint*>(wU + n);
+    zint* ma = GRID ? p.ma : mp + 2 * n;
+    zint* xr = GRID ? p.xr + (size_t)b * n : ma + 2 * n;
+    zint* A = GRID ? p.A : xr + n;  // row i at A + row(i) n
+    ll* md = GRID ? p.md : reinterpret_cast<ll*>(A + (size_t)R * n);
+    signed char* ee = GRID ? reinterpret_cast<signed char*>(wU + n) : reinterpret_cast<signed char*>(md + 2 * n);
+    signed char* de = ee + n;
+    signed char* cap = de + n;  // largest exponent a row may get
+    ll* mq = p.mq;
+    auto row = [&](int i) { return GRID ? i : i / C; };
+    unsigned arrivals = 0;
+
+    // ---- scale: a power of two above the Frobenius norm -------------------------
+    if (tid < 24) (&sh.S[0][0])[tid] = 0;
+    if (tid == 0) {
+        sh.abort = 0;
+        for (int k = 0; k < 3; ++k) {
+            sh.emin[k] = INT_MAX;
+            sh.vm[k] = INT_MIN;
+            sh.shift[k] = 0;
+        }
+        if (!GRID) {  // the cluster barriers below come before the first exchange
+            for (int k = 0; k < 2; ++k)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                    (uint32_t)__cvta_generic_to_shared(&sh.mbar[k])));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+    }
+    unsigned hmax = 0;
+    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+        for (int l = lane; l <= i; l += 32) {
+            const cplx v = p.G[i + (size_t)n * l];
+            const double im = l == i ? 0.0 : v.y;
+            hmax = max(hmax, max((unsigned)__double2hiint(v.x) & 0x7fffffffu,
+                                 (unsigned)__double2hiint(im) & 0x7fffffffu));
+        }
+    hmax = __reduce_max_sync(0xffffffffu, hmax);
+    __shared__ unsigned s_max;
+    __shared__ float s_sum[8];
+    if (tid == 0) s_max = 0;
+    __syncthreads();
+    if (lane == 0 && warp < 8) atomicMax(&s_max, hmax);
+    __syncthreads();
+    auto share = [&](unsigned v, int slot) -> bool {  // this block's partial to all blocks
+        if (GRID) {
+            if (tid == 0) p.part[slot * C + b] = v;
+            arrivals += (unsigned)C;
+            return grid_sync(p.bar, p.err, arrivals);
+        }
+        if (tid < C) st_cluster(map_shared(&sh.part[slot * HC + b], tid), v);
+        cluster_sync();
+        return true;
+    };
+    auto shared_part = [&](int slot, int i) {
+        return GRID ? __ldcg(p.part + slot * C + i) : sh.part[slot * HC + i];
+    };
+    if (!share(s_max, 0)) return;
+    hmax = 0;
+    for (int i = 0; i < C; ++i) hmax = max(hmax, shared_part(0, i));
+    if (hmax >= 0x7ff00000u) {  // an infinity or NaN: no block goes on
+        if (b == 0 && tid == 0) *p.o.f = INT_MIN;
+        if (!GRID) cluster_sync();  // no block leaves while others read its memory
+        return;
+    }
+    const int emax = max((int)(hmax >> 20), 1) - 1022;  // |entries| < 2^emax
+    const double dn = scalbn(1.0, -max(emax, -1000));
+    float sum = 0.f;
+    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+        for (int l = lane; l <= i; l += 32) {
+            const cplx v = p.G[i + (size_t)n * l];
+            const float x = (float)(v.x * dn), y = l == i ? 0.f : (float)(v.y * dn);
+            sum += (l == i ? 1.f : 2.f) * (x * x + y * y);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && warp < 8) s_sum[warp] = sum;
+    __syncthreads();
+    sum = 0.f;
+    for (int w = 0; w < 8; ++w) sum += s_sum[w];
+    if (!share(__float_as_uint(sum), 1)) return;
+    sum = 0.f;
+    for (int i = 0; i < C; ++i) sum += __uint_as_float(shared_part(1, i));
+    // F^2 < 2^(2 f): the FP32 sum is good to 1e-3
+    int fe;
+    frexpf(sum * 1.01f, &fe);
+    const int f = max(emax, -1000) + (fe + 1) / 2;
+    if (b == 0 && tid == 0) *p.o.f = f;
+
+    // ---- order, exponents, this block's rows as integers --------------------------
+    // Rows of a graded matrix go by descending diagonal: eliminated in that order,
+    // small eigenvalues keep their relative accuracy (in the opposite order they
+    // lose it in FP64 too).
+    int* perm = reinterpret_cast<int*>(wU);
+    if (p.psd) {
+        float* key = reinterpret_cast<float*>(vD);
+        for (int l = tid; l < n; l += HT) key[l] = (float)scalbn(p.G[l + (size_t)n * l].x, -f);
+        __syncthreads();
+        for (int l = tid; l < n; l += HT) {
+            const float k = key[l];
+            int r = 0;
+            for (int i = 0; i < n; ++i) r += key[i] > k || (key[i] == k && i < l);
+            perm[r] = l;
+            if (b == 0) p.o.perm[r] = l;
+        }
+    } else {
+        for (int l = tid; l < n; l += HT) perm[l] = l;
+    }
+    __syncthreads();
+    int em = INT_MAX;
+    for (int l = tid; l < n; l += HT) {
+        const int64_t pl = perm[l];
+        const int e0 = p.psd ? next_exponent(0, EXP_MAX, (float)scalbn(p.G[pl + n * pl].x, -f), 0.f, 0.f, 0.f) : 0;
+        ee[l] = (signed char)e0;
+        cap[l] = (signed char)min(EXP_MAX, e0 + EXP_GAIN);
+        em = min(em, e0);
+    }
+    em = __reduce_min_sync(0xffffffffu, em);
+    if (lane == 0) atomicMin(&sh.emin[0], em);
+    __syncthreads();
+    em = sh.emin[0];  // over all rows: at most the smallest below row 0
+    int c = max(0, em - 6);
+    if (tid == 0) {
+        sh.em = em;
+        sh.c = c;
+    }
+    auto entry = [&](int i, int l) {  // (i, l) of the reordered matrix
+        const int64_t pi = perm[i], pl = perm[l];
+        cplx v = pl <= pi ? p.G[pi + n * pl] : p.G[pl + n * pi];
+        if (pl > pi) v.y = -v.y;
+        if (pl == pi) v.y = 0.0;
+        return v;
+    };
+    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+        for (int l = lane; l < n; l += 32) {
+            const cplx v = entry(i, l);
+            const int s = 61 - f + ee[i] + ee[l];
+            A[(size_t)row(i) * n + l] = zint{to_fix(v.x, s), to_fix(v.y, s)};
+        }
+
+    // One entry of the next column (rows left from l1 on): kept, its square added.
+    auto emit = [&](int l, int l1, zint x, int el, int emn, Norm2& S) {
+        xr[l] = x;
+        if (l == l1) sh.alpha = x;
+        norm_add(S, x, el - emn);
+    };
+    auto add_norm = [&](const Norm2& S, int buf) {  // exact: 24-bit limbs through warp adds
+        unsigned mine = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const unsigned t = __reduce_add_sync(0xffffffffu, norm_limb(S, k));
+            if (lane == k) mine = t;
+        }
+        if (lane < 8 && mine) atomicAdd(&sh.S[buf][lane], mine);
+    };
+    if (warp < 8) {  // column 0
+        Norm2 S{0, 0};
+        for (int l = tid; l < n; l += HM) {
+            const cplx v = entry(l, 0);
+            if (l == 0) {
+                if (b == 0) {
+                    p.o.di[0] = to_fix(v.x, 61 - f + 2 * c);
+                    p.o.dsh[0] = 2 * c;
+                }
+                continue;
+            }
+            const int s = 61 - f + ee[l] + c;
+            emit(l, 1, zint{to_fix(v.x, s), to_fix(v.y, s)}, ee[l], em, S);
+        }
+        add_norm(S, 0);
+    }
+    __syncthreads();  // perm gives way to w
+    bool pend = false;
+    for (int j = 0; j + 1 < n; ++j) {
+        __syncthreads();  // squared norm of the column, its entries and alpha
+        const NormTop S = norm_top(sh.S[j % 3]);
+        const int shf = S.bl ? norm_shift(S.bl) : 0;
+        em = sh.em;
+        c = sh.c;
+        const int l0 = j + 1, s0 = ee[l0] - em;  // first row left
+        const int buf = j & 1;
+        if (warp == 8) {
+            // beta and v's first entry for the row warps, then tau and c2 while
+            // the rows' results travel
+            double ar = 0.0, ai = 0.0, be = 0.0, sq = 0.0;
+            if (lane == 0) {
+                ll beta = 0;
+                zint al{0, 0};
+                if (S.bl) {
+                    // squared norm in v's unit: S 2^(2 shf - 112 - 56), in [1/4, 1)
+                    sq = scale2(__ull2double_rn(S.top), S.bl + 2 * shf - 232);
+                    al = zsft(sh.alpha, shf - s0);
+                    be = sq * rsqrt(sq);
+                    be = al.x < 0 ? be : -be;
+                    beta = __double2ll_rn(scale2(be, 56));
+                }
+                sh.beta = beta;
+                sh.v1 = zint{al.x - beta, al.y};
+                if (!GRID)
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(&sh.mbar[buf])),
+                                 "r"(40 * (n - j - 1) + 64 * C)
+                                 : "memory");
+                ar = scale2(__ll2double_rn(al.x), -56);
+                ai = scale2(__ll2double_rn(al.y), -56);
+            }
+            __syncwarp();
+            bar_named(2, HT);
+            if (lane == 0) {
+                zint tau{0, 0};
+                ll c2 = 0;
+                double tr = 0.0, ti = 0.0;
+                if (S.bl) {
+                    // |beta - alpha|^2 = s + |alpha|^2 + 2 |beta alpha_r| (no cancellation)
+                    const double D = fma(ar, ar, fma(ai, ai, fma(-(be + be), ar, sq)));
+                    const double ri = recip(be * D);
+                    tr = (be - ar) * ri;
+                    ti = -ai * ri;
+                    tau = zint{__double2ll_rn(scale2(tr, 60)), __double2ll_rn(scale2(ti, 60))};
+                    c2 = __double2ll_rn(scale2(D * ri * ri, 58));  // |tau|^2 = D / (beta D)^2
+                }
+                sh.tau = tau;
+                sh.c2 = c2;
+                if (b == 0) {
+                    p.o.tau[j] = cmk(tr, ti);
+                    p.o.ei[j] = sh.beta;
+                    p.o.esh[j] = shf + em + c;
+                }
+                if (b == l0 % C) p.o.V[(size_t)j * n + l0] = sh.v1;
+            }
+            __syncwarp();
+        } else {
+            // column -> v's limbs for the products (the first entry still alpha);
+            // v itself is kept for the back-transformation
+            int vm = -s0;
+            for (int l = l0 + tid; l < n; l += HM) {
+                const int d = ee[l] - em;
+                const zint x = xr[l];
+                vm = max(vm, max(bits64(x.x), bits64(x.y)) + shf - 2 * d - 56);
+                vD[l] = limbs29(zsft(x, shf - 2 * d));
+                if (l > l0 && l % C == b) p.o.V[(size_t)j * n + l] = zsft(x, shf - d);
+            }
+            vm = __reduce_max_sync(0xffffffffu, vm);
+            if (lane == 0) atomicMax(&sh.vm[j % 3], vm);
+            bar_named(1, HM);
+            // ---- A. rows: pending update, product with v ------------------------
+            zint P{0, 0}, Aj{0, 0};
+            ll Dg = 0;
+            int k = 0;
+            int i = b + C * warp;
+            if (i <= j) i += (j - i + 8 * C) / (8 * C) * (8 * C);  // first own row above j
+            const int i0 = i;
+            // lane k keeps the warp's k-th row's result (at most 32 rows a warp)
+            const bool moved = sh.shift[j % 3] != 0;
+            for (; i < n; i += 8 * C, ++k) {
+                zint* a = A + (size_t)row(i) * n;
+                Dot s{0, 0, 0, 0, 0, 0};
+                zint first{0, 0};
+                ll dg = 0;
+                if (pend) {
+                    const int4 wi = wU[i], vi = vU[i];
+                    const int di = de[i];
+                    for (int l = l0 + lane; l < n; l += 32) {
+                        zint x = a[l];
+                        if (moved) x = zsft(x, di + de[l]);
+                        update(x, wi, vi, wU[l], vU[l]);
+                        a[l] = x;
+                        if (l == l0) first = x;
+                        if (l == i) dg = x.x;
+                        dot_add(s, x, vD[l]);
+                    }
+                } else {
+                    for (int l = l0 + lane; l < n; l += 32) {
+                        const zint x = a[l];
+                        if (l == l0) first = x;
+                        if (l == i) dg = x.x;
+                        dot_add(s, x, vD[l]);
+                    }
+                }
+                const zint t = dot_value(s);
+                const ll px = warp_sum64(t.x), py = warp_sum64(t.y);
+                const ll fx = __shfl_sync(0xffffffffu, first.x, 0), fy = __shfl_sync(0xffffffffu, first.y, 0);
+                dg = __shfl_sync(0xffffffffu, dg, (i - l0) & 31);
+                if (lane == k) {
+                    P = zint{px, py};
+                    Aj = zint{fx, fy};
+                    Dg = dg;
+                }
+            }
+            bar_named(2, HT);  // beta and the first entry of v
+            const int io = i0 + 8 * C * lane;
+            ll q = 0;
+            if (lane < k) {
+                P = minus_real(P, Aj, sh.beta, s0);
+                q = re_dot(io == l0 ? zsft(sh.v1, -s0) : value29(vD[io]), P);
+                if (GRID) {
+                    mp[buf * n + io] = P;
+                    ma[buf * n + io] = Aj;
+                    md[buf * n + io] = Dg;
+                    mq[buf * n + io] = q;
+                }
+            }
+            if (!GRID) {
+                // every warp sends its share of q, rows or not: a block that has
+                // everybody's share knows that nobody reads the buffer it will
+                // write two steps on
+                ll qs = 0;
+                for (int r = 0; r < k; ++r) {
+                    const zint pr{__shfl_sync(0xffffffffu, P.x, r), __shfl_sync(0xffffffffu, P.y, r)};
+                    const zint ar{__shfl_sync(0xffffffffu, Aj.x, r), __shfl_sync(0xffffffffu, Aj.y, r)};
+                    const ll dr = __shfl_sync(0xffffffffu, Dg, r);
+                    qs += __shfl_sync(0xffffffffu, q, r);
+                    if (lane < C) {
+                        const int ir = buf * n + i0 + 8 * C * r;
+                        const uint32_t mb = map_shared(&sh.mbar[buf], lane);
+                        st_async(map_shared(mp + ir, lane), pr, mb);
+                        st_async(map_shared(ma + ir, lane), ar, mb);
+                        st_async(map_shared(md + ir, lane), dr, mb);
+                    }
+                }
+                if (lane < C)
+                    st_async(map_shared(&sh.qt[buf][8 * b + warp], lane), qs, map_shared(&sh.mbar[buf], lane));
+            }
+        }
+        if (GRID) {
+            arrivals += (unsigned)C;
+            if (!grid_sync(p.bar, p.err, arrivals)) return;
+        } else if (warp < 8) {
+            if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) sh.abort = 1;
+        }
+        // ---- B. w, column j+1, its norm ----------------------------------------
+        const int off = buf * n;
+        ll q = 0;
+        if (warp < 8) {
+            if (GRID) {
+                for (int l = j + 1 + tid; l < n; l += HM) q += __ldcg(mq + off + l);
+                q = warp_sum64(q);
+                if (lane == 0) sh.q[warp] = q;
+            } else {  // every warp adds all shares itself
+                for (int t = lane; t < 8 * C; t += 32) q += sh.qt[buf][t];
+                q = warp_sum64(q);
+            }
+            if (tid < 8) sh.S[(j + 1) % 3][tid] = 0;
+        }
+        bar_named(3, HT);  // tau and c2
+        if (!GRID && sh.abort) {
+            if (tid == 0) atomicExch(p.err, 1);
+            break;
+        }
+        if (warp < 8) {
+            if (GRID) {
+                q = 0;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) q += sh.q[w];
+            }
+            // h = log2 sqrt(v^H A v): w and v scaled by its powers stay bounded
+            const int h = p.psd ? q_exponent(q, sh.vm[j % 3]) : 0;
+            const ll al2 = q_scaled(sh.c2, q, h);
+            const zint tau = sh.tau;
+            // float copies for the exponents' estimate
+            const float tx = (float)(tau.x >> 32) * 0x1p-28f, ty = (float)(tau.y >> 32) * 0x1p-28f;
+            const float fp = __int_as_float((127 - 61 - h) << 23), fv = __int_as_float((127 + shf + h - 56) << 23);
+            const float fa = (float)(al2 >> 32) * 0x1p-25f, ft = fabsf(tx) + fabsf(ty);
+            const int nb = (j + 1) % 3;
+            int emn = INT_MAX, any = 0;
+            for (int l = l0 + 1 + tid; l < n; l += HM) {
+                const zint pl = GRID ? ld_zint(mp + off + l) : mp[off + l];
+                const zint x = xr[l];
+                const int el = ee[l];
+                int en = el;
+                if (p.psd) {
+                    const float px = __ll2float_rn(pl.x) * fp, py = __ll2float_rn(pl.y) * fp;
+                    const float vx = __ll2float_rn(x.x) * fv, vy = __ll2float_rn(x.y) * fv;
+                    const float wx = tx * px - ty * py - fa * vx, wy = tx * py + ty * px - fa * vy;
+                    const float av = fabsf(vx) + fabsf(vy);
+                    const float a = __ll2float_rn(GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
+                    en = next_exponent(el, cap[l], a, 2.f * (wx * vx + wy * vy),
+                                       2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), vx * vx + vy * vy);
+                }
+                const int d = en - el;
+                const zint vt = zsft(x, shf + h + d);
+                wU[l] = limbs31(make_w(tau, zsft(pl, d - h), al2, vt));
+                vU[l] = limbs29(vt);
+                ee[l] = (signed char)en;
+                de[l] = (signed char)d;
+                emn = min(emn, en);
+                any |= d;
+            }
+            emn = __reduce_min_sync(0xffffffffu, emn);
+            any = __reduce_or_sync(0xffffffffu, (unsigned)any);
+            if (lane == 0) {
+                atomicMin(&sh.emin[nb], emn);
+                if (any) sh.shift[nb] = 1;
+            }
+            bar_named(1, HM);
+            emn = min(sh.emin[nb], 1 << 20);
+            if (l0 + 1 >= n) emn = em;
+            // the next column is that of row l0, whose exponent becomes cn: its w and v
+            const int cn = max(0, min(emn, (int)ee[l0]) - 6), d0 = cn - ee[l0];
+            const zint v0 = zsft(sh.v1, cn + h - em);
+            const int4 v1 = limbs29(v0);
+            const int4 w1 = limbs31(make_w(tau, zsft(GRID ? ld_zint(mp + off + l0) : mp[off + l0], d0 - h), al2, v0));
+            if (b == 0 && tid == 0) {
+                zint x = zsft(GRID ? ld_zint(ma + off + l0) : ma[off + l0], 2 * d0);
+                update(x, w1, v1, w1, v1);
+                p.o.di[l0] = x.x;
+                p.o.dsh[l0] = 2 * cn;
+            }
+            Norm2 S2{0, 0};
+            for (int l = l0 + 1 + tid; l < n; l += HM) {
+                zint x = zsft(GRID ? ld_zint(ma + off + l) : ma[off + l], de[l] + d0);
+                update(x, wU[l], vU[l], w1, v1);
+                emit(l, l0 + 1, x, ee[l], emn, S2);
+            }
+            add_norm(S2, nb);
+            if (tid == 0) {
+                sh.em = emn;
+                sh.c = cn;
+            }
+        }
+        if (tid == 0) {  // buffers of the step after next
+            sh.emin[(j + 2) % 3] = INT_MAX;
+            sh.vm[(j + 2) % 3] = INT_MIN;
+            sh.shift[(j + 2) % 3] = 0;
+        }
+        pend = true;
+    }
+    if (!GRID) cluster_sync();  // no block leaves while its shared memory is written
+}
+
+// d, e and the reflectors as FP64: column j of G becomes reflector j (zeros down
+// to the diagonal, the first entry explicit).
+__global__ void __launch_bounds__(256) hetrd_finish_kernel(TrdOut o, int n, cplx* __restrict__ G,
+                                                           double* __restrict__ d,
+                                                           double* __restrict__ e) {
+    const int f = *o.f;
+    const bool bad = f == INT_MIN;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n * n;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int j = (int)(t / n), i = (int)(t % n);
+        cplx g = cmk(0, 0);
+        if (i > j && !bad) {
+            const zint v = o.V[t];
+            g = cmk(__ll2double_rn(v.x) * 0x1p-56, __ll2double_rn(v.y) * 0x1p-56);
+        } else if (i == j) {
+            d[j] = bad ? nan : scalbn(__ll2double_rn(o.di[j]), f - 61 - o.dsh[j]);
+            if (j + 1 < n) e[j] = bad ? nan : scalbn(__ll2double_rn(o.ei[j]), f - 61 - o.esh[j]);
+            if (bad || j + 1 == n) o.tau[j] = cmk(0, 0);
+        }
+        G[t] = g;
+    }
+}
+
+size_t hetrd_smem(int64_t n, int64_t C) {
+    const size_t R = (size_t)((n + C - 1) / C);
+    return 16 * (8 * (size_t)n + R * n) + 19 * (size_t)n;
+}
+
+constexpr size_t HSMEM = 223 * 1024;  // dynamic shared memory a block can have beside ShCtl
+
+}  // namespace
+
+// G (n x n Hermitian, lower triangle read) -> T (d, e) and the reflectors: column
+// j of G is v_j (rows j+1.., zeros above), tau[j] its scalar.  psd: G is positive
+// semidefinite and keeps graded accuracy, its row perm[l] as row l of Q.  No host
+// synchronisation; a grid barrier that ran out leaves ctx->d_bar[2] nonzero.
+void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool psd, int* perm) {
+    // Blocks of the cluster: the row work of a step (n^2 / 3 entries on average at
+    // 180 clocks per 32) against the exchange with more blocks.
+    int64_t C = n <= 16 ? 1 : n <= 32 ? 4 : n <= 64 ? 8 : HC;
+    const bool grid = hetrd_smem(n, C) > HSMEM || ctx->trd_clusters == 0;
+    if (grid) C = ctx->sm_count;
+    auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t nn = r256(sizeof(zint) * (size_t)n * n), n8 = r256(sizeof(ll) * n),
+                 n4 = r256(sizeof(int) * n), nz = r256(sizeof(zint) * 2 * n);
+    const size_t nx = r256(sizeof(zint) * (size_t)n * C);
+    const size_t total = nn + 2 * n8 + 2 * n4 + 512 + (grid ? nn + nx + 2 * nz + 4 * n8 + r256(2 * 4 * C) : 0);
+    char* base = static_cast<char*>(ctx->s_trd.get(ctx, total));
+    auto take = [&](size_t b) {
+        char* q = base;
+        base += b;
+        return q;
+    };
+    TrdIn a{};
+    a.G = G;
+    a.n = (int)n;
+    a.psd = psd ? 1 : 0;
+    a.o.V = reinterpret_cast<zint*>(take(nn));
+    a.o.di = reinterpret_cast<ll*>(take(n8));
+    a.o.ei = reinterpret_cast<ll*>(take(n8));
+    a.o.esh = reinterpret_cast<int*>(take(n4));
+    a.o.dsh = reinterpret_cast<int*>(take(n4));
+    a.o.f = reinterpret_cast<int*>(take(256));
+    a.o.tau = tau;
+    a.o.perm = perm;
+    a.err = reinterpret_cast<int*>(ctx->d_bar + 2);
+    a.bar = ctx->d_bar;
+    if (grid) {
+        take(256);
+        a.A = reinterpret_cast<zint*>(take(nn));
+        a.mp = reinterpret_cast<zint*>(take(nz));
+        a.ma = reinterpret_cast<zint*>(take(nz));
+        a.md = reinterpret_cast<ll*>(take(2 * n8));
+        a.mq = reinterpret_cast<ll*>(take(2 * n8));
+        a.xr = reinterpret_cast<zint*>(take(nx));
+        a.part = reinterpret_cast<unsigned*>(take(r256(2 * 4 * C)));
+        const size_t smem = 51 * (size_t)n;
+        TN_REQUIRE(smem <= HSMEM, "hetrd: matrix order too large");
+        // the limit for the largest order, the same from every thread
+        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<true>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
+        void* args[] = {&a};
+        TN_CHECK_CUDA(cudaLaunchCooperativeKernel((void*)hetrd_fix_kernel<true>, dim3((unsigned)C),
+                                                  dim3(HT), args, smem, ctx->stream));
+    } else {
+        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<false>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
+        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<false>,
+                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)C;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)C);
+        cfg.blockDim = dim3(HT);
+        cfg.dynamicSmemBytes = hetrd_smem(n, C);
+        cfg.stream = ctx->stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if (ctx->trd_clusters < 0) {  // whether this GPU can hold the widest cluster at all
+            cudaLaunchConfig_t w = cfg;
+            cudaLaunchAttribute wat = at;
+            wat.val.clusterDim.x = HC;
+            w.gridDim = dim3(HC);
+            w.dynamicSmemBytes = HSMEM;
+            w.attrs = &wat;
+            int fit = 0;
+            TN_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&fit, hetrd_fix_kernel<false>, &w));
+            ctx->trd_clusters = fit;
+            if (fit == 0) return hetrd(ctx, G, n, d, e, tau, psd, perm);
+        }
+        TN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hetrd_fix_kernel<false>, a));
+    }
+    ctx->count();
+    const int64_t blocks = std::min<int64_t>((n * n + 255) / 256, (int64_t)ctx->sm_count * 8);
+    hetrd_finish_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(a.o, (int)n, G, d, e);
+    ctx->count();
+    TN_CHECK_CUDA(cudaGetLastError());
+}
+
+}  // namespace tn

@@ -84,7 +84,8 @@ void ctx_release(Ctx& c) {
     // scratch buffers release through the stream before it goes away
     Scratch* all[] = {&c.s_gram, &c.s_eigval, &c.s_work, &c.s_x, &c.s_y, &c.s_t1, &c.s_t2,
                       &c.s_dot, &c.s_coef, &c.s_mixa, &c.s_mixb, &c.s_mixc, &c.s_mixd, &c.s_mixe,
-                      &c.s_mixf, &c.s_eig, &c.s_splitk, &c.s_tcz};
+                      &c.s_mixf, &c.s_eig, &c.s_splitk, &c.s_tcz,
+                      &c.s_trd, &c.s_bt, &c.s_dc};
     for (Scratch* s : all) s->buf.reset();
     if (c.stream) cudaStreamSynchronize(c.stream);
     if (c.d_info) cudaFree(c.d_info);
@@ -131,7 +132,7 @@ void Ctx::prof_flush() {
 // ---- eigen-decomposition ---------------------------------------------------
 void heev_full(Ctx* ctx, cplx* G, int64_t n, double* dlam) {
     DBuf V(ctx, sizeof(cplx) * n * n);
-    eig_top(ctx, G, n, n, dlam, V.c());
+    eig_top(ctx, G, n, n, dlam, V.c(), true);
     take_top_eigvecs(ctx, V.c(), n, n, G);  // descending -> ascending columns
     int h = 0;
     TN_CHECK_CUDA(cudaMemcpyAsync(&h, ctx->d_bar + 2, sizeof(int), cudaMemcpyDeviceToHost,
@@ -165,7 +166,7 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
     double* dtotal = lam + want + sz;  // the trace gives the weight below the computed values
     gram_trace(ctx, G, g, dtotal);
     cplx* V = ctx->s_x.c(ctx, (size_t)g * want);  // top eigenvectors, descending
-    eig_top(ctx, G, g, want, lam, V);
+    eig_top(ctx, G, g, want, lam, V, true);
     // the eigensolver's barrier status is read back with the keep-rule result
     KeepResult kr = keep_rule(ctx, lam, want, want, cutoff, maxdim, mindim, dS, dtotal,
                               reinterpret_cast<const int*>(ctx->d_bar + 2));
