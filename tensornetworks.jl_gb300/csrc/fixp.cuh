@@ -96,20 +96,69 @@ TN_HD zint dot_value(const Dot& s) {  // unit 2^-61 F
                 (ll)((ull)s.my << 5) + ((s.cy + (s.ly >> 29) + (1ll << 23)) >> 24)};
 }
 
-// round(x / 2^s)
-TN_HD ll rshift(i128 x, int s) { return (ll)((x + ((i128)1 << (s - 1))) >> s); }
+// Limbs of 32 bits: v = hi 2^32 + lo with a signed low limb (|v| < 2^63 - 2^31).
+struct limb32 {
+    int h, l;
+};
+TN_HD limb32 split32(ll v) { return limb32{(int)((v + (1ll << 31)) >> 32), (int)v}; }
 
-// p - a b 2^-s for b real (unit 2^-56)
+// Running sum of products a b = m 2^64 + x 2^32 + l; the cross products of a call's
+// two terms stay below 2^63 for |a| < 2^61, |b| < 2^62.
+struct Prod {
+    ll m, x, l;
+};
+TN_HD Prod mul32(limb32 a, limb32 b) {
+    return Prod{mw(a.h, b.h, 0), mw(a.l, b.h, mw(a.h, b.l, 0)), mw(a.l, b.l, 0)};
+}
+TN_HD Prod mul32(limb32 a, limb32 b, Prod c) {
+    return Prod{mw(a.h, b.h, c.m), mw(a.l, b.h, mw(a.h, b.l, c.x)), (mw(a.l, b.l, 0) >> 1) + (c.l >> 1)};
+}
+// the sum of one product / 2^s, of two / 2^s; 32 < s < 64, rounded
+TN_HD ll prod1(const Prod& p, int s) {
+    return (ll)((ull)p.m << (64 - s)) + ((p.x + (p.l >> 32) + (1ll << (s - 33))) >> (s - 32));
+}
+TN_HD ll prod2(const Prod& p, int s) {
+    return (ll)((ull)p.m << (64 - s)) + ((p.x + (p.l >> 31) + (1ll << (s - 33))) >> (s - 32));
+}
+TN_HD limb32 neg(limb32 a) { return limb32{-a.h, -a.l}; }
+
+// x 2^s (s negative: rounded), componentwise; zero beyond |s| = 62 (upwards only a
+// zero gets there)
+struct Shift {
+    int l, r;
+    ll half;
+};
+TN_HD Shift shift_by(int s) {
+    Shift h;
+    h.l = s > 0 ? (s < 63 ? s : 63) : 0;
+    h.r = s < 0 ? (s > -63 ? -s : 63) : 0;
+    h.half = (1ll << h.r) >> 1 & 0x7fffffffffffffffll;
+    return h;
+}
+TN_HD ll sft(ll x, Shift h) { return (ll)(((ull)x << h.l) + (ull)h.half) >> h.r; }
+TN_HD ll sft(ll x, int s) { return sft(x, shift_by(s)); }
+TN_HD zint zsft(zint v, int s) {
+    const Shift h = shift_by(s);
+    return zint{sft(v.x, h), sft(v.y, h)};
+}
+
+// p - a b 2^-s for b real (unit 2^-56), s >= 0
 TN_HD zint minus_real(zint p, zint a, ll b, int s) {
-    return zint{p.x - rshift((i128)a.x * b, 56 + s), p.y - rshift((i128)a.y * b, 56 + s)};
+    const limb32 lb = split32(b);
+    const zint t{prod1(mul32(split32(a.x), lb), 56), prod1(mul32(split32(a.y), lb), 56)};
+    const zint u = zsft(t, -s);
+    return zint{p.x - u.x, p.y - u.y};
 }
 // Re(conj(v) p), unit 2^-60 F
-TN_HD ll re_dot(zint v, zint p) { return rshift((i128)v.x * p.x + (i128)v.y * p.y, 57); }
+TN_HD ll re_dot(zint v, zint p) {
+    return prod2(mul32(split32(v.x), split32(p.x), mul32(split32(v.y), split32(p.y))), 57);
+}
 
-// w = tau p - al v: tau in units of 2^-60, al 2^-57, p 2^-61 F, v 2^-56; w 2^-57 F
+// w = tau p - al v: tau in units of 2^-59, al 2^-57, p 2^-61 F, v 2^-56; w 2^-57 F
 TN_HD zint make_w(zint tau, zint p, ll al, zint v) {
-    return zint{rshift((i128)tau.x * p.x - (i128)tau.y * p.y, 64) - rshift((i128)al * v.x, 56),
-                rshift((i128)tau.x * p.y + (i128)tau.y * p.x, 64) - rshift((i128)al * v.y, 56)};
+    const limb32 tx = split32(tau.x), ty = split32(tau.y), px = split32(p.x), py = split32(p.y), la = split32(al);
+    return zint{prod2(mul32(tx, px, mul32(neg(ty), py)), 63) - prod1(mul32(split32(v.x), la), 56),
+                prod2(mul32(tx, py, mul32(ty, px)), 63) - prod1(mul32(split32(v.y), la), 56)};
 }
 
 TN_HD u128 abs2(zint x) {
@@ -126,15 +175,8 @@ TN_HD int bits128(u128 s) {
 #endif
 }
 
-// x 2^s (s negative: rounded), componentwise; zero beyond |s| = 62 (upwards only a
-// zero gets there)
-TN_HD ll sft(ll x, int s) {
-    return s > 62 || s < -62 ? 0 : s >= 0 ? (ll)((ull)x << s) : ((x + (1ll << (-s - 1))) >> -s);
-}
-TN_HD zint zsft(zint v, int s) { return zint{sft(v.x, s), sft(v.y, s)}; }
-
-// Sum of |x_l|^2 2^(56 - 2 d_l), exact: 192 bits, summed across threads as eight
-// 24-bit limbs.
+// Sum of |x_l|^2 2^(56 - 2 d_l), exact: 192 bits, summed across up to 1024 threads as
+// nine 22-bit limbs.
 struct Norm2 {
     u128 lo;
     ull hi;
@@ -146,11 +188,12 @@ TN_HD void norm_add(Norm2& s, zint x, int d) {
     s.hi += (sl ? (ull)(a >> (128 - sl)) : 0) + (t < s.lo ? 1 : 0);
     s.lo = t;
 }
+constexpr int NORM_LIMBS = 9;
 TN_HD unsigned norm_limb(const Norm2& s, int k) {
-    const unsigned m = 0xffffff;
-    if (k < 5) return (unsigned)(s.lo >> (24 * k)) & m;
-    if (k == 5) return ((unsigned)(s.lo >> 120) | (unsigned)(s.hi << 8)) & m;
-    return (unsigned)(s.hi >> (24 * k - 128)) & m;
+    const unsigned m = 0x3fffff;
+    if (k < 5) return (unsigned)(s.lo >> (22 * k)) & m;
+    if (k == 5) return ((unsigned)(s.lo >> 110) | (unsigned)(s.hi << 18)) & m;
+    return (unsigned)(s.hi >> (22 * k - 128)) & m;
 }
 // From the summed limbs (32 bits each): the sum as top 2^(bl - 64), bl = 0 for zero.
 struct NormTop {
@@ -158,22 +201,22 @@ struct NormTop {
     ull top;
 };
 TN_HD NormTop norm_top(const unsigned* l) {
-    u128 L = 0, H = 0;
+    u128 L = 0, H = l[8];
 #pragma unroll
     for (int k = 3; k >= 0; --k) {
-        L = (L << 24) + l[k];
-        H = (H << 24) + l[k + 4];
+        L = (L << 22) + l[k];
+        H = (H << 22) + l[k + 4];
     }
-    H += L >> 96;
-    L &= (((u128)1) << 96) - 1;
+    H += L >> 88;
+    L &= (((u128)1) << 88) - 1;
     NormTop r{0, 0};
     const int h = bits128(H);
     if (h >= 64) {
-        r.bl = 96 + h;
+        r.bl = 88 + h;
         r.top = (ull)(H >> (h - 64));
     } else if (h > 0) {
-        r.bl = 96 + h;
-        r.top = (ull)((H << (64 - h)) | (L >> (32 + h)));
+        r.bl = 88 + h;
+        r.top = (ull)((H << (64 - h)) | (L >> (24 + h)));
     } else {
         const int b = bits128(L);
         r.bl = b;
@@ -181,6 +224,11 @@ TN_HD NormTop norm_top(const unsigned* l) {
     }
     return r;
 }
+// The sum's bit length from limbs k and k - 1 alone: 22 k + that of this, k the
+// highest for which it is nonzero (one short where a carry from further below
+// reaches a power of two)
+TN_HD unsigned norm_carry(unsigned l, unsigned below) { return l + (below >> 22); }
+
 // Shift that takes the column to a norm in [1/2, 1) in the unit 2^-56.  The
 // reflector is H = I - tau v v^H with v = column - beta e_1, H^H (column) =
 // beta e_1, beta real of the sign opposite to the first entry's real part (LAPACK
@@ -228,10 +276,7 @@ TN_HD int q_exponent(ll q, int vm) {
     return h < lo ? lo : h;
 }
 // al = |tau|^2 / 2 q 2^(-2 h), unit 2^-57, from |tau|^2 / 2 in units of 2^-59
-TN_HD ll q_scaled(ll c2, ll q, int h) {
-    const int s = 62 + 2 * h;
-    return s > 0 ? rshift((i128)c2 * q, s) : (ll)((i128)c2 * q << -s);
-}
+TN_HD ll q_scaled(ll c2, ll q, int h) { return prod1(mul32(split32(c2), split32(sft(q, -2 * h))), 62); }
 
 }  // namespace fixp
 }  // namespace tn

@@ -41,29 +41,36 @@ __device__ __forceinline__ double recip(double x) {
     return fma(r, fma(-x, r, 1.0), r);
 }
 
-// Barrier of all blocks of a cooperative launch on a counter that only grows;
-// bounded by the global timer, false (in every thread of the block) when the
-// wait ran out here or in another block.
+// Barrier of all blocks of a cooperative launch on a counter that only grows, by one
+// thread of each block; the wait is bounded by the global timer, false when it ran
+// out here or in another block (looked at every 32 polls: a look is a second trip
+// to L2).
+__device__ __forceinline__ void grid_arrive(unsigned* count) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(unsigned* count, int* err, unsigned target) {
+    uint64_t t0 = 0;
+    for (int polls = 1;; ++polls) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        if (v >= target) return true;
+        if (polls % 32) continue;
+        if (*(volatile int*)err) return false;
+        const uint64_t t = hclock();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > HWAIT_NS) {
+            atomicExch(err, 1);
+            return false;
+        }
+    }
+}
+// the same for all threads of the block
 __device__ __forceinline__ bool grid_sync(unsigned* count, int* err, unsigned target) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ok = 1;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-        if (v < target) {
-            const uint64_t t0 = hclock();
-            do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-                if (*(volatile int*)err) ok = 0;
-                else if (hclock() - t0 > HWAIT_NS) {
-                    atomicExch(err, 1);
-                    ok = 0;
-                }
-            } while (ok && v < target);
-        }
-        s_ok = ok;
+        grid_arrive(count);
+        s_ok = grid_wait(count, err, target);
     }
     __syncthreads();
     return s_ok != 0;

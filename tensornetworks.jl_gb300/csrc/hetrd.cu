@@ -2,18 +2,29 @@
 // G = Q T Q^H, in fixed point (fixp.cuh): step 1 of the eigensolver (eig.cu).
 //
 // One thread-block cluster holds the whole matrix in its shared memories up to
-// order 405 (sixteen blocks), one cooperative grid in global memory above.  Row
-// i belongs to block i mod C.  Step j:
+// order 288; above, the blocks of a cooperative grid do, and from about order 1100
+// the rows stay in global memory (L2).  Row i belongs to block i mod C.  Step j:
 //   A. a warp per row applies the pending rank-2 update of step j-1 to the
-//      row and sums its product with v, in one pass, while a ninth warp forms
+//      row and sums its product with v, in one pass, while a further warp forms
 //      the reflector's scalars in FP64 (its only FP64 work: about thirty
 //      instructions of 64 clocks); the row's product, its entry of column j+1
 //      and its share of v^H A v go to every block;
 //   B. after one barrier (cluster: 0.2 us, grid: 1.2 us) every block forms w,
 //      column j+1 with this step's update and its exact squared norm itself.
-// The FP64 version spent 8.7 us per step at order 256: a 1.9 us grid barrier,
-// five block sums of ten dependent 64-clock additions each and a serial
+// The FP64 version spent 8.7 us per step at order 256, 11 at 512: a 1.9 us grid
+// barrier, five block sums of ten dependent 64-clock additions each and a serial
 // square root and two divisions (2,000 clocks).
+//
+// Up to order 200 a step is a chain of dependent integer instructions (7,700
+// clocks at order 64: limbs of v 720, rows 2,050 with their sums, exchange 1,760,
+// w 1,850, column and norm 1,380); rows take over above (order 256: 6,800 of
+// 16,000 clocks) and their traffic through L2 at order 2048 (41,000 of 62,000).
+// A thread per entry (16 row warps in the larger forms), rows two entries deep with
+// the next two loaded ahead, the products of w by 32-bit limbs, the new exponent of
+// row j+1 from the last step's smallest exponent (so that w needs one pass) and
+// work that nobody waits for behind the exchange took order 64 from 308 to 257 us,
+// 128 from 699 to 576, 256 from 2,069 to 1,873, 512 from 6,574 to 4,437, 2048 from
+// 98 to 61 ms.
 //
 // Reflector j is kept as V[j n + i] (i > j; integers of unit 2^-56 with the
 // first entry explicit) and tau[j]: H_j = I - tau_j v_j v_j^H.
@@ -31,9 +42,12 @@ namespace {
 using namespace fixp;
 using namespace griddev;
 
-constexpr int HT = 288;       // threads: eight row warps and the scalar warp
-constexpr int HM = 256;       // threads of the row warps
-constexpr int HC = 16;        // blocks of a full cluster
+constexpr int HC = 16;   // blocks of a full cluster
+constexpr int HPAD = 64;  // zeros after the vectors: rows run in steps of 64 entries
+
+// A cluster with its rows in shared memory, a grid likewise, a grid with its rows in
+// global memory.
+enum Form { CLUSTER, GRID_SHARED, GRID_GLOBAL };
 
 struct TrdOut {
     zint* V;      // n x n, column j: reflector j
@@ -52,8 +66,9 @@ struct TrdIn {
     zint* A;          // grid form: n x n rows in global memory
     zint* mp;         // grid form: mailbox, two buffers of n entries each
     zint* ma;
-    ll *md, *mq;
-    zint* xr;         // grid form: a block's copy of the column
+    ll* md;
+    ull* mq;          // grid form: v^H A v, triple buffered by step
+    zint* xr;         // rows in global memory: a block's copy of the column
     unsigned* part;   // grid form: per-block scale partials
     unsigned* bar;    // grid form: arrival counter (zero at launch)
     int* err;
@@ -102,18 +117,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     }
 }
 
+// sum modulo 2^64 by three 22-bit limbs (three REDUX; ten shuffles take 144 clocks)
 __device__ __forceinline__ ll warp_sum64(ll v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x3fffffu);
+    const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 22) & 0x3fffffu);
+    const unsigned c = __reduce_add_sync(0xffffffffu, (unsigned)((ull)v >> 44));
+    return (ll)((ull)a + ((ull)b << 22) + ((ull)c << 44));
 }
 
 struct ShCtl {
-    ll q[8];             // grid form: partial v^H A v of the warps
-    ll qt[2][8 * HC];    // cluster form: every warp's share, from every block
+    ull q;               // grid form: the block's share of v^H A v
+    ll qt[2][16 * HC];   // cluster form: every warp's share, from every block
     uint64_t mbar[2];    // cluster form: a step's exchange has arrived
     int abort;
-    unsigned S[3][8];    // squared norm, 24-bit limbs, triple buffered by step
+    unsigned S[3][NORM_LIMBS];  // squared norm, limbs, triple buffered by step
     int vm[3];           // largest entry of v 2^-e, log2, likewise
     int emin[3];         // smallest exponent of the rows left, likewise
     int shift[3];        // whether any exponent changed, likewise
@@ -140,40 +157,46 @@ __device__ __forceinline__ ll to_fix(double x, int s) {
     return b < 0 ? -r : r;
 }
 
-template <bool GRID>
-__global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
+template <int FORM, int RW>
+__global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
+    constexpr bool GRID = FORM != CLUSTER;
+    constexpr int HM = 32 * RW, HT = HM + 32;  // threads of the row warps; the scalar warp
     extern __shared__ __align__(16) unsigned char hsm[];
     __shared__ ShCtl sh;
     const int n = p.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int C = GRID ? (int)gridDim.x : (int)cluster_size();
     const int b = GRID ? (int)blockIdx.x : (int)cluster_rank();
     const int R = (n + C - 1) / C;
-    // shared memory: the column, v's limbs for products, v's and w's for the pending
-    // update, exponents and their pending change; in the cluster form the mailbox
-    // and the rows
+    // shared memory: v's limbs for products, v's and w's for the pending update,
+    // exponents, their pending change and their bound; the column and the rows
+    // unless they are in global memory; in the cluster form the mailbox
     int4* vD = reinterpret_cast<int4*>(hsm);
-    int4* vU = vD + n;
-    int4* wU = vU + n;
-    zint* mp = GRID ? p.mp : reinterpret_cast<zint*>(wU + n);
+    int4* vU = vD + n + HPAD;
+    int4* wU = vU + n + HPAD;
+    zint* xs = reinterpret_cast<zint*>(wU + n + HPAD);
+    zint* xr = FORM == GRID_GLOBAL ? p.xr + (size_t)b * n : xs;
+    zint* A = FORM == GRID_GLOBAL ? p.A : xs + n;  // row i at A + row(i) n
+    zint* mp = GRID ? p.mp : xs + n + (size_t)R * n;
     zint* ma = GRID ? p.ma : mp + 2 * n;
-    zint* xr = GRID ? p.xr + (size_t)b * n : ma + 2 * n;
-    zint* A = GRID ? p.A : xr + n;  // row i at A + row(i) n
-    ll* md = GRID ? p.md : reinterpret_cast<ll*>(A + (size_t)R * n);
-    signed char* ee = GRID ? reinterpret_cast<signed char*>(wU + n) : reinterpret_cast<signed char*>(md + 2 * n);
+    ll* md = GRID ? p.md : reinterpret_cast<ll*>(ma + 2 * n);
+    signed char* ee = FORM == GRID_GLOBAL   ? reinterpret_cast<signed char*>(xs)
+                      : FORM == GRID_SHARED ? reinterpret_cast<signed char*>(A + (size_t)R * n)
+                                            : reinterpret_cast<signed char*>(md + 2 * n);
     signed char* de = ee + n;
     signed char* cap = de + n;  // largest exponent a row may get
-    ll* mq = p.mq;
-    auto row = [&](int i) { return GRID ? i : i / C; };
+    auto row = [&](int i) { return FORM == GRID_GLOBAL ? i : i / C; };
     unsigned arrivals = 0;
 
     // ---- scale: a power of two above the Frobenius norm -------------------------
-    if (tid < 24) (&sh.S[0][0])[tid] = 0;
+    if (tid < 3 * NORM_LIMBS) (&sh.S[0][0])[tid] = 0;
     if (tid == 0) {
         sh.abort = 0;
+        sh.q = 0;
         for (int k = 0; k < 3; ++k) {
             sh.emin[k] = INT_MAX;
             sh.vm[k] = INT_MIN;
             sh.shift[k] = 0;
+            if (GRID && b == 0) p.mq[k] = 0;
         }
         if (!GRID) {  // the cluster barriers below come before the first exchange
             for (int k = 0; k < 2; ++k)
@@ -183,7 +206,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         }
     }
     unsigned hmax = 0;
-    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+    for (int i = b + C * warp; i < n && warp < RW; i += RW * C)
         for (int l = lane; l <= i; l += 32) {
             const cplx v = p.G[i + (size_t)n * l];
             const double im = l == i ? 0.0 : v.y;
@@ -192,10 +215,10 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         }
     hmax = __reduce_max_sync(0xffffffffu, hmax);
     __shared__ unsigned s_max;
-    __shared__ float s_sum[8];
+    __shared__ float s_sum[RW];
     if (tid == 0) s_max = 0;
     __syncthreads();
-    if (lane == 0 && warp < 8) atomicMax(&s_max, hmax);
+    if (lane == 0 && warp < RW) atomicMax(&s_max, hmax);
     __syncthreads();
     auto share = [&](unsigned v, int slot) -> bool {  // this block's partial to all blocks
         if (GRID) {
@@ -221,7 +244,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
     const int emax = max((int)(hmax >> 20), 1) - 1022;  // |entries| < 2^emax
     const double dn = scalbn(1.0, -max(emax, -1000));
     float sum = 0.f;
-    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+    for (int i = b + C * warp; i < n && warp < RW; i += RW * C)
         for (int l = lane; l <= i; l += 32) {
             const cplx v = p.G[i + (size_t)n * l];
             const float x = (float)(v.x * dn), y = l == i ? 0.f : (float)(v.y * dn);
@@ -229,10 +252,10 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0 && warp < 8) s_sum[warp] = sum;
+    if (lane == 0 && warp < RW) s_sum[warp] = sum;
     __syncthreads();
     sum = 0.f;
-    for (int w = 0; w < 8; ++w) sum += s_sum[w];
+    for (int w = 0; w < RW; ++w) sum += s_sum[w];
     if (!share(__float_as_uint(sum), 1)) return;
     sum = 0.f;
     for (int i = 0; i < C; ++i) sum += __uint_as_float(shared_part(1, i));
@@ -267,6 +290,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         const int64_t pl = perm[l];
         const int e0 = p.psd ? next_exponent(0, EXP_MAX, (float)scalbn(p.G[pl + n * pl].x, -f), 0.f, 0.f, 0.f) : 0;
         ee[l] = (signed char)e0;
+        de[l] = 0;
         cap[l] = (signed char)min(EXP_MAX, e0 + EXP_GAIN);
         em = min(em, e0);
     }
@@ -286,7 +310,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         if (pl == pi) v.y = 0.0;
         return v;
     };
-    for (int i = b + C * warp; i < n && warp < 8; i += 8 * C)
+    for (int i = b + C * warp; i < n && warp < RW; i += RW * C)
         for (int l = lane; l < n; l += 32) {
             const cplx v = entry(i, l);
             const int s = 61 - f + ee[i] + ee[l];
@@ -299,16 +323,16 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         if (l == l1) sh.alpha = x;
         norm_add(S, x, el - emn);
     };
-    auto add_norm = [&](const Norm2& S, int buf) {  // exact: 24-bit limbs through warp adds
+    auto add_norm = [&](const Norm2& S, int buf) {  // exact: limbs through warp adds
         unsigned mine = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < NORM_LIMBS; ++k) {
             const unsigned t = __reduce_add_sync(0xffffffffu, norm_limb(S, k));
             if (lane == k) mine = t;
         }
-        if (lane < 8 && mine) atomicAdd(&sh.S[buf][lane], mine);
+        if (lane < NORM_LIMBS && mine) atomicAdd(&sh.S[buf][lane], mine);
     };
-    if (warp < 8) {  // column 0
+    if (warp < RW) {  // column 0
         Norm2 S{0, 0};
         for (int l = tid; l < n; l += HM) {
             const cplx v = entry(l, 0);
@@ -324,25 +348,34 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
         }
         add_norm(S, 0);
     }
-    __syncthreads();  // perm gives way to w
-    bool pend = false;
+    __syncthreads();
+    for (int l = tid; l < 3 * (n + HPAD); l += HT) vD[l] = make_int4(0, 0, 0, 0);  // vU and wU too
     for (int j = 0; j + 1 < n; ++j) {
         __syncthreads();  // squared norm of the column, its entries and alpha
-        const NormTop S = norm_top(sh.S[j % 3]);
-        const int shf = S.bl ? norm_shift(S.bl) : 0;
+        // its bit length, by lanes
+        const unsigned nl = lane < NORM_LIMBS ? sh.S[j % 3][lane] : 0;
+        unsigned below = __shfl_up_sync(0xffffffffu, nl, 1);
+        if (lane == 0) below = 0;
+        const unsigned nc = norm_carry(nl, below);
+        const unsigned some = __ballot_sync(0xffffffffu, nc != 0);
+        const int kt = 31 - __clz(some | 1);
+        const int bl = 22 * kt + 32 - __clz(__shfl_sync(0xffffffffu, nc, kt));  // zero: no column
+        const int shf = bl ? norm_shift(bl) : 0;
         em = sh.em;
         c = sh.c;
         const int l0 = j + 1, s0 = ee[l0] - em;  // first row left
-        const int buf = j & 1;
-        if (warp == 8) {
+        const int cn = max(0, em - 6);  // its new exponent: its diagonal is at most the trace, n 2^(-2 em)
+        const int buf = j & 1, nb = (j + 1) % 3;
+        if (warp == RW) {
             // beta and v's first entry for the row warps, then tau and c2 while
             // the rows' results travel
             double ar = 0.0, ai = 0.0, be = 0.0, sq = 0.0;
             if (lane == 0) {
                 ll beta = 0;
                 zint al{0, 0};
-                if (S.bl) {
+                if (bl) {
                     // squared norm in v's unit: S 2^(2 shf - 112 - 56), in [1/4, 1)
+                    const NormTop S = norm_top(sh.S[j % 3]);
                     sq = scale2(__ull2double_rn(S.top), S.bl + 2 * shf - 232);
                     al = zsft(sh.alpha, shf - s0);
                     be = sq * rsqrt(sq);
@@ -354,7 +387,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                 if (!GRID)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                      (uint32_t)__cvta_generic_to_shared(&sh.mbar[buf])),
-                                 "r"(40 * (n - j - 1) + 64 * C)
+                                 "r"(40 * (n - j - 1) + 8 * RW * C)
                                  : "memory");
                 ar = scale2(__ll2double_rn(al.x), -56);
                 ai = scale2(__ll2double_rn(al.y), -56);
@@ -365,13 +398,13 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                 zint tau{0, 0};
                 ll c2 = 0;
                 double tr = 0.0, ti = 0.0;
-                if (S.bl) {
+                if (bl) {
                     // |beta - alpha|^2 = s + |alpha|^2 + 2 |beta alpha_r| (no cancellation)
                     const double D = fma(ar, ar, fma(ai, ai, fma(-(be + be), ar, sq)));
                     const double ri = recip(be * D);
                     tr = (be - ar) * ri;
                     ti = -ai * ri;
-                    tau = zint{__double2ll_rn(scale2(tr, 60)), __double2ll_rn(scale2(ti, 60))};
+                    tau = zint{__double2ll_rn(scale2(tr, 59)), __double2ll_rn(scale2(ti, 59))};
                     c2 = __double2ll_rn(scale2(D * ri * ri, 58));  // |tau|^2 = D / (beta D)^2
                 }
                 sh.tau = tau;
@@ -385,52 +418,41 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
             }
             __syncwarp();
         } else {
-            // column -> v's limbs for the products (the first entry still alpha);
-            // v itself is kept for the back-transformation
-            int vm = -s0;
-            for (int l = l0 + tid; l < n; l += HM) {
-                const int d = ee[l] - em;
-                const zint x = xr[l];
-                vm = max(vm, max(bits64(x.x), bits64(x.y)) + shf - 2 * d - 56);
-                vD[l] = limbs29(zsft(x, shf - 2 * d));
-                if (l > l0 && l % C == b) p.o.V[(size_t)j * n + l] = zsft(x, shf - d);
-            }
-            vm = __reduce_max_sync(0xffffffffu, vm);
-            if (lane == 0) atomicMax(&sh.vm[j % 3], vm);
+            // column -> v's limbs for the products (the first entry still alpha)
+            for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em)));
             bar_named(1, HM);
             // ---- A. rows: pending update, product with v ------------------------
             zint P{0, 0}, Aj{0, 0};
             ll Dg = 0;
             int k = 0;
             int i = b + C * warp;
-            if (i <= j) i += (j - i + 8 * C) / (8 * C) * (8 * C);  // first own row above j
+            if (i <= j) i += (j - i + RW * C) / (RW * C) * (RW * C);  // first own row above j
             const int i0 = i;
             // lane k keeps the warp's k-th row's result (at most 32 rows a warp)
             const bool moved = sh.shift[j % 3] != 0;
-            for (; i < n; i += 8 * C, ++k) {
+            for (; i < n; i += RW * C, ++k) {
                 zint* a = A + (size_t)row(i) * n;
                 Dot s{0, 0, 0, 0, 0, 0};
                 zint first{0, 0};
                 ll dg = 0;
-                if (pend) {
-                    const int4 wi = wU[i], vi = vU[i];
-                    const int di = de[i];
-                    for (int l = l0 + lane; l < n; l += 32) {
-                        zint x = a[l];
-                        if (moved) x = zsft(x, di + de[l]);
-                        update(x, wi, vi, wU[l], vU[l]);
-                        a[l] = x;
-                        if (l == l0) first = x;
-                        if (l == i) dg = x.x;
-                        dot_add(s, x, vD[l]);
-                    }
-                } else {
-                    for (int l = l0 + lane; l < n; l += 32) {
-                        const zint x = a[l];
-                        if (l == l0) first = x;
-                        if (l == i) dg = x.x;
-                        dot_add(s, x, vD[l]);
-                    }
+                const int4 wi = wU[i], vi = vU[i];
+                const int di = de[i];
+                auto one = [&](zint x, int l) {  // entries from n on count zero
+                    if (moved) x = zsft(x, di + de[min(l, n - 1)]);
+                    update(x, wi, vi, wU[l], vU[l]);
+                    if (l < n) a[l] = x;
+                    if (l == l0) first = x;
+                    if (l == i) dg = x.x;
+                    dot_add(s, x, vD[l]);
+                };
+                int l = l0 + lane;
+                zint x0 = a[min(l, n - 1)], x1 = a[min(l + 32, n - 1)];
+                for (; l < n; l += 64) {
+                    const zint y0 = a[min(l + 64, n - 1)], y1 = a[min(l + 96, n - 1)];
+                    one(x0, l);
+                    one(x1, l + 32);
+                    x0 = y0;
+                    x1 = y1;
                 }
                 const zint t = dot_value(s);
                 const ll px = warp_sum64(t.x), py = warp_sum64(t.y);
@@ -443,7 +465,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                 }
             }
             bar_named(2, HT);  // beta and the first entry of v
-            const int io = i0 + 8 * C * lane;
+            const int io = i0 + RW * C * lane;
             ll q = 0;
             if (lane < k) {
                 P = minus_real(P, Aj, sh.beta, s0);
@@ -452,10 +474,21 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                     mp[buf * n + io] = P;
                     ma[buf * n + io] = Aj;
                     md[buf * n + io] = Dg;
-                    mq[buf * n + io] = q;
                 }
             }
-            if (!GRID) {
+            if (GRID) {
+                if (k) {
+                    q = warp_sum64(q);
+                    if (lane == 0) atomicAdd(&sh.q, (ull)q);
+                }
+                bar_named(1, HM);
+                arrivals += (unsigned)C;
+                if (tid == 0) {
+                    atomicAdd(p.mq + j % 3, sh.q);
+                    sh.q = 0;
+                    grid_arrive(p.bar);
+                }
+            } else {
                 // every warp sends its share of q, rows or not: a block that has
                 // everybody's share knows that nobody reads the buffer it will
                 // write two steps on
@@ -466,7 +499,7 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                     const ll dr = __shfl_sync(0xffffffffu, Dg, r);
                     qs += __shfl_sync(0xffffffffu, q, r);
                     if (lane < C) {
-                        const int ir = buf * n + i0 + 8 * C * r;
+                        const int ir = buf * n + i0 + RW * C * r;
                         const uint32_t mb = map_shared(&sh.mbar[buf], lane);
                         st_async(map_shared(mp + ir, lane), pr, mb);
                         st_async(map_shared(ma + ir, lane), ar, mb);
@@ -474,51 +507,57 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                     }
                 }
                 if (lane < C)
-                    st_async(map_shared(&sh.qt[buf][8 * b + warp], lane), qs, map_shared(&sh.mbar[buf], lane));
+                    st_async(map_shared(&sh.qt[buf][RW * b + warp], lane), qs, map_shared(&sh.mbar[buf], lane));
             }
-        }
-        if (GRID) {
-            arrivals += (unsigned)C;
-            if (!grid_sync(p.bar, p.err, arrivals)) return;
-        } else if (warp < 8) {
-            if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) sh.abort = 1;
-        }
-        // ---- B. w, column j+1, its norm ----------------------------------------
-        const int off = buf * n;
-        ll q = 0;
-        if (warp < 8) {
+            // while the results travel: v for the back-transformation, the largest
+            // entry of v 2^-e
+            int vm = -s0;
+            for (int l = l0 + tid; l < n; l += HM) {
+                const int d = ee[l] - em;
+                const zint x = xr[l];
+                if (l > l0 && l % C == b) p.o.V[(size_t)j * n + l] = zsft(x, shf - d);
+                vm = max(vm, max(bits64(x.x), bits64(x.y)) + shf - 2 * d - 56);
+            }
+            vm = __reduce_max_sync(0xffffffffu, vm);
+            if (lane == 0) atomicMax(&sh.vm[j % 3], vm);
+            if (tid < NORM_LIMBS) sh.S[nb][tid] = 0;
             if (GRID) {
-                for (int l = j + 1 + tid; l < n; l += HM) q += __ldcg(mq + off + l);
-                q = warp_sum64(q);
-                if (lane == 0) sh.q[warp] = q;
-            } else {  // every warp adds all shares itself
-                for (int t = lane; t < 8 * C; t += 32) q += sh.qt[buf][t];
-                q = warp_sum64(q);
+                if (tid == 0) {
+                    if (!grid_wait(p.bar, p.err, arrivals)) sh.abort = 1;
+                    if (b == 0) p.mq[(j + 2) % 3] = 0;  // every block has read step j - 1's
+                }
+            } else if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) {
+                sh.abort = 1;
             }
-            if (tid < 8) sh.S[(j + 1) % 3][tid] = 0;
         }
-        bar_named(3, HT);  // tau and c2
-        if (!GRID && sh.abort) {
+        bar_named(3, HT);  // the exchange; tau and c2
+        if (sh.abort) {
             if (tid == 0) atomicExch(p.err, 1);
             break;
         }
-        if (warp < 8) {
+        // ---- B. w, column j+1, its norm ----------------------------------------
+        if (warp < RW) {
+            const int off = buf * n;
+            ll q = 0;
             if (GRID) {
-                q = 0;
+                q = (ll)__ldcg(p.mq + j % 3);
+            } else {  // every warp adds all shares itself
 #pragma unroll
-                for (int w = 0; w < 8; ++w) q += sh.q[w];
+                for (int t = 0; t < RW * HC; t += 32)
+                    if (t + lane < RW * C) q += sh.qt[buf][t + lane];
+                q = warp_sum64(q);
             }
             // h = log2 sqrt(v^H A v): w and v scaled by its powers stay bounded
             const int h = p.psd ? q_exponent(q, sh.vm[j % 3]) : 0;
             const ll al2 = q_scaled(sh.c2, q, h);
             const zint tau = sh.tau;
             // float copies for the exponents' estimate
-            const float tx = (float)(tau.x >> 32) * 0x1p-28f, ty = (float)(tau.y >> 32) * 0x1p-28f;
+            const float tx = (float)(int)(tau.x >> 32) * 0x1p-27f, ty = (float)(int)(tau.y >> 32) * 0x1p-27f;
             const float fp = __int_as_float((127 - 61 - h) << 23), fv = __int_as_float((127 + shf + h - 56) << 23);
-            const float fa = (float)(al2 >> 32) * 0x1p-25f, ft = fabsf(tx) + fabsf(ty);
-            const int nb = (j + 1) % 3;
+            const float fa = (float)(int)(al2 >> 32) * 0x1p-25f, ft = fabsf(tx) + fabsf(ty);
             int emn = INT_MAX, any = 0;
-            for (int l = l0 + 1 + tid; l < n; l += HM) {
+            for (int l = l0 + tid; l < n; l += HM) {
+                const bool top = l == l0;
                 const zint pl = GRID ? ld_zint(mp + off + l) : mp[off + l];
                 const zint x = xr[l];
                 const int el = ee[l];
@@ -531,15 +570,18 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                     const float a = __ll2float_rn(GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
                     en = next_exponent(el, cap[l], a, 2.f * (wx * vx + wy * vy),
                                        2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), vx * vx + vy * vy);
+                    if (top) en = cn;  // its row becomes column j+1
                 }
                 const int d = en - el;
-                const zint vt = zsft(x, shf + h + d);
+                const zint vt = zsft(top ? sh.v1 : x, top ? cn + h - em : shf + h + d);
                 wU[l] = limbs31(make_w(tau, zsft(pl, d - h), al2, vt));
                 vU[l] = limbs29(vt);
                 ee[l] = (signed char)en;
                 de[l] = (signed char)d;
-                emn = min(emn, en);
-                any |= d;
+                if (!top) {
+                    emn = min(emn, en);
+                    any |= d;
+                }
             }
             emn = __reduce_min_sync(0xffffffffu, emn);
             any = __reduce_or_sync(0xffffffffu, (unsigned)any);
@@ -548,37 +590,30 @@ __global__ void __launch_bounds__(HT) hetrd_fix_kernel(TrdIn p) {
                 if (any) sh.shift[nb] = 1;
             }
             bar_named(1, HM);
-            emn = min(sh.emin[nb], 1 << 20);
-            if (l0 + 1 >= n) emn = em;
-            // the next column is that of row l0, whose exponent becomes cn: its w and v
-            const int cn = max(0, min(emn, (int)ee[l0]) - 6), d0 = cn - ee[l0];
-            const zint v0 = zsft(sh.v1, cn + h - em);
-            const int4 v1 = limbs29(v0);
-            const int4 w1 = limbs31(make_w(tau, zsft(GRID ? ld_zint(mp + off + l0) : mp[off + l0], d0 - h), al2, v0));
-            if (b == 0 && tid == 0) {
-                zint x = zsft(GRID ? ld_zint(ma + off + l0) : ma[off + l0], 2 * d0);
-                update(x, w1, v1, w1, v1);
-                p.o.di[l0] = x.x;
-                p.o.dsh[l0] = 2 * cn;
-            }
+            emn = l0 + 1 < n ? sh.emin[nb] : em;
+            const int4 w1 = wU[l0], v1 = vU[l0];
+            const int d0 = de[l0];
             Norm2 S2{0, 0};
-            for (int l = l0 + 1 + tid; l < n; l += HM) {
+            for (int l = l0 + tid; l < n; l += HM) {
                 zint x = zsft(GRID ? ld_zint(ma + off + l) : ma[off + l], de[l] + d0);
                 update(x, wU[l], vU[l], w1, v1);
-                emit(l, l0 + 1, x, ee[l], emn, S2);
+                if (l > l0) {
+                    emit(l, l0 + 1, x, ee[l], emn, S2);
+                } else if (b == 0) {
+                    p.o.di[l0] = x.x;
+                    p.o.dsh[l0] = 2 * cn;
+                }
             }
-            add_norm(S2, nb);
+            if (l0 + 32 * warp < n) add_norm(S2, nb);
             if (tid == 0) {
                 sh.em = emn;
                 sh.c = cn;
+                // buffers of the step after next
+                sh.emin[(j + 2) % 3] = INT_MAX;
+                sh.vm[(j + 2) % 3] = INT_MIN;
+                sh.shift[(j + 2) % 3] = 0;
             }
         }
-        if (tid == 0) {  // buffers of the step after next
-            sh.emin[(j + 2) % 3] = INT_MAX;
-            sh.vm[(j + 2) % 3] = INT_MIN;
-            sh.shift[(j + 2) % 3] = 0;
-        }
-        pend = true;
     }
     if (!GRID) cluster_sync();  // no block leaves while its shared memory is written
 }
@@ -607,12 +642,59 @@ __global__ void __launch_bounds__(256) hetrd_finish_kernel(TrdOut o, int n, cplx
     }
 }
 
-size_t hetrd_smem(int64_t n, int64_t C) {
+size_t hetrd_smem(Form form, int64_t n, int64_t C) {
     const size_t R = (size_t)((n + C - 1) / C);
-    return 16 * (8 * (size_t)n + R * n) + 19 * (size_t)n;
+    return 48 * (size_t)(n + HPAD) + 3 * (size_t)n + (form == GRID_GLOBAL ? 0 : 16 * (R + 1) * n) +
+           (form == CLUSTER ? 80 * (size_t)n : 0);
 }
 
-constexpr size_t HSMEM = 223 * 1024;  // dynamic shared memory a block can have beside ShCtl
+constexpr size_t HSMEM = 220 * 1024;  // dynamic shared memory a block can have beside ShCtl
+
+template <int FORM, int RW>
+void launch(Ctx* ctx, const TrdIn& a, int64_t C, size_t smem) {
+    auto k = hetrd_fix_kernel<FORM, RW>;
+    // the limit for the largest order, the same from every thread
+    TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
+    TN_REQUIRE(smem <= HSMEM, "hetrd: matrix order too large");
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at;
+    cfg.gridDim = dim3((unsigned)C);
+    cfg.blockDim = dim3(32 * RW + 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (FORM == CLUSTER) {
+        TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)C;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    TN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+}
+
+// whether this GPU can hold the widest cluster at all
+int clusters_fit() {
+    auto k = hetrd_fix_kernel<CLUSTER, 16>;
+    TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
+    TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = HC;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(HC);
+    cfg.blockDim = dim3(32 * 16 + 32);
+    cfg.dynamicSmemBytes = HSMEM;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    TN_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&fit, k, &cfg));
+    return fit;
+}
 
 }  // namespace
 
@@ -621,16 +703,22 @@ constexpr size_t HSMEM = 223 * 1024;  // dynamic shared memory a block can have 
 // semidefinite and keeps graded accuracy, its row perm[l] as row l of Q.  No host
 // synchronisation; a grid barrier that ran out leaves ctx->d_bar[2] nonzero.
 void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool psd, int* perm) {
+    if (ctx->trd_clusters < 0) ctx->trd_clusters = clusters_fit();
     // Blocks of the cluster: the row work of a step (n^2 / 3 entries on average at
-    // 180 clocks per 32) against the exchange with more blocks.
+    // 180 clocks per 32) against the exchange with more blocks.  The grid's barrier
+    // and vectors through L2 cost 4 us a step more, its rows next to nothing: order
+    // 300 takes 2,589 us in a cluster and 2,308 on the grid, order 256 1,873 in a
+    // cluster, order 400 4,915 against 3,214.
     int64_t C = n <= 16 ? 1 : n <= 32 ? 4 : n <= 64 ? 8 : HC;
-    const bool grid = hetrd_smem(n, C) > HSMEM || ctx->trd_clusters == 0;
+    const bool grid = n > 288 || ctx->trd_clusters == 0;
     if (grid) C = ctx->sm_count;
+    const bool rows_global = grid && hetrd_smem(GRID_SHARED, n, C) > HSMEM;
     auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t nn = r256(sizeof(zint) * (size_t)n * n), n8 = r256(sizeof(ll) * n),
                  n4 = r256(sizeof(int) * n), nz = r256(sizeof(zint) * 2 * n);
     const size_t nx = r256(sizeof(zint) * (size_t)n * C);
-    const size_t total = nn + 2 * n8 + 2 * n4 + 512 + (grid ? nn + nx + 2 * nz + 4 * n8 + r256(2 * 4 * C) : 0);
+    const size_t total = nn + 2 * n8 + 2 * n4 + 512 + (rows_global ? nn + nx : 0) +
+                         (grid ? 256 + 2 * nz + 2 * n8 + r256(2 * 4 * C) : 0);
     char* base = static_cast<char*>(ctx->s_trd.get(ctx, total));
     auto take = [&](size_t b) {
         char* q = base;
@@ -652,51 +740,22 @@ void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool p
     a.err = reinterpret_cast<int*>(ctx->d_bar + 2);
     a.bar = ctx->d_bar;
     if (grid) {
-        take(256);
-        a.A = reinterpret_cast<zint*>(take(nn));
+        a.mq = reinterpret_cast<ull*>(take(256));
         a.mp = reinterpret_cast<zint*>(take(nz));
         a.ma = reinterpret_cast<zint*>(take(nz));
         a.md = reinterpret_cast<ll*>(take(2 * n8));
-        a.mq = reinterpret_cast<ll*>(take(2 * n8));
-        a.xr = reinterpret_cast<zint*>(take(nx));
         a.part = reinterpret_cast<unsigned*>(take(r256(2 * 4 * C)));
-        const size_t smem = 51 * (size_t)n;
-        TN_REQUIRE(smem <= HSMEM, "hetrd: matrix order too large");
-        // the limit for the largest order, the same from every thread
-        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
-        void* args[] = {&a};
-        TN_CHECK_CUDA(cudaLaunchCooperativeKernel((void*)hetrd_fix_kernel<true>, dim3((unsigned)C),
-                                                  dim3(HT), args, smem, ctx->stream));
+    }
+    if (rows_global) {
+        a.A = reinterpret_cast<zint*>(take(nn));
+        a.xr = reinterpret_cast<zint*>(take(nx));
+        launch<GRID_GLOBAL, 16>(ctx, a, C, hetrd_smem(GRID_GLOBAL, n, C));
+    } else if (grid) {
+        launch<GRID_SHARED, 16>(ctx, a, C, hetrd_smem(GRID_SHARED, n, C));
+    } else if (n <= 8 * C) {  // a warp per row
+        launch<CLUSTER, 8>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
     } else {
-        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
-        TN_CHECK_CUDA(cudaFuncSetAttribute(hetrd_fix_kernel<false>,
-                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = (unsigned)C;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)C);
-        cfg.blockDim = dim3(HT);
-        cfg.dynamicSmemBytes = hetrd_smem(n, C);
-        cfg.stream = ctx->stream;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        if (ctx->trd_clusters < 0) {  // whether this GPU can hold the widest cluster at all
-            cudaLaunchConfig_t w = cfg;
-            cudaLaunchAttribute wat = at;
-            wat.val.clusterDim.x = HC;
-            w.gridDim = dim3(HC);
-            w.dynamicSmemBytes = HSMEM;
-            w.attrs = &wat;
-            int fit = 0;
-            TN_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&fit, hetrd_fix_kernel<false>, &w));
-            ctx->trd_clusters = fit;
-            if (fit == 0) return hetrd(ctx, G, n, d, e, tau, psd, perm);
-        }
-        TN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hetrd_fix_kernel<false>, a));
+        launch<CLUSTER, 16>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
     }
     ctx->count();
     const int64_t blocks = std::min<int64_t>((n * n + 255) / 256, (int64_t)ctx->sm_count * 8);
