@@ -19,8 +19,16 @@
 // What it replaced is serial in the order: a Sturm count is n steps of four FP64
 // instructions of 64 clocks each, an inverse iteration six such sweeps, the QR
 // of the vectors n grid barriers; at order 256, 128 vectors: bisection 1,071 us,
-// inverse iteration 731, QR and its Q 1,114.  Here a level costs four barriers
-// and the whole 250 us at order 64, 350 at 128, 430 at 256.
+// inverse iteration 731, QR and its Q 1,114.  Here all of it takes 72 us at order
+// 32, 94 at 64, 152 at 128, 210 at 256.
+//
+// A level is a chain of FP64 instructions that cost the same for one lane as for
+// 32, so a warp finds several roots at once where merges are small (32 / K lanes),
+// blocks of eight rows are merged by one warp without barriers, the FP32 start of a
+// root is a search in up to 32 sections a round, and Newton stops when the next step
+// would change nothing (two evaluations a root).  A warp per root throughout, with
+// bisection and a confirming step, took 163 us at order 32, 207 at 64, 272 at 128
+// and 313 at 256.
 #include <climits>
 #include <cmath>
 
@@ -64,30 +72,33 @@ __device__ __forceinline__ ll okey(double x) {
 __device__ __forceinline__ double unkey(ll k) {
     return __longlong_as_double(k < 0 ? k ^ 0x7fffffffffffffffll : k);
 }
-// Monotone map to integers whose unit step is an ulp, or 2^-82 below 2^-30.
+// Monotone map to integers whose unit step is an ulp, or 2^-82 below 2^-30; in
+// integers, as FP64 conversions cost 64 clocks each.
 constexpr ll B30 = (1023ll - 30) << 52;
 __device__ __forceinline__ ll to_grid(double v) {
-    const double a = fabs(v);
-    const ll k = a < 0x1p-30 ? __double2ll_rn(a * 0x1p82) : (1ll << 52) + __double_as_longlong(a) - B30;
-    return v < 0.0 ? -k : k;
+    const ll bits = __double_as_longlong(v), a = bits & LLONG_MAX;
+    const int s = 993 - (int)(a >> 52);  // below 2^-30 the mantissa moves down by s
+    ll k;
+    if (s <= 0) k = (1ll << 52) + a - B30;
+    else if (s > 53) k = 0;
+    else k = (((a & ((1ll << 52) - 1)) | (1ll << 52)) + (1ll << (s - 1))) >> s;
+    return bits < 0 ? -k : k;
 }
 __device__ __forceinline__ double from_grid(ll k) {
     const ll a = k < 0 ? -k : k;
-    const double x = a < (1ll << 52) ? __ll2double_rn(a) * 0x1p-82 : __longlong_as_double(B30 + a - (1ll << 52));
-    return k < 0 ? -x : x;
+    ll bits;
+    if (a >= (1ll << 52)) {
+        bits = B30 + a - (1ll << 52);
+    } else if (a == 0) {
+        bits = 0;
+    } else {
+        const int s = __clzll(a) - 11;  // mantissa's leading bit to bit 52
+        bits = ((ll)(993 - s) << 52) + ((a << s) - (1ll << 52));
+    }
+    return __longlong_as_double(k < 0 ? bits | LLONG_MIN : bits);
 }
 __device__ __forceinline__ ll shfl_up64(ll v, int o) {
     return __shfl_up_sync(0xffffffffu, v, o);
-}
-__device__ __forceinline__ double wsum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ float wsumf(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
 }
 // 1 / x for any normal x: recip() on the mantissa, the exponent by integers
 __device__ __forceinline__ double rcp(double x) {
@@ -99,21 +110,270 @@ __device__ __forceinline__ double rcp(double x) {
     return __hiloint2double(__double2hiint(r) + (sh << 20), __double2loint(r));
 }
 
+// floor(log2 |x|) of a normal x; zero counts as 2^-1023
+__device__ __forceinline__ int expo(double x) { return ((__double2hiint(x) >> 20) & 0x7ff) - 1023; }
+
+// sums over aligned groups of g lanes
+__device__ __forceinline__ double gsum(double v, int g) {
+    for (int o = g >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ float gsumf(float v, int g) {
+    for (int o = g >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// FP32 reciprocal, good to an ulp (denormals count as zero)
+__device__ __forceinline__ float rcpf(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+constexpr int BASE = 8;  // rows of a base block
+
+// base blocks are merged in shared memory by one warp, the rest through L2
+template <bool LOC, class T>
+__device__ __forceinline__ T ld(const T* p) {
+    return LOC ? *p : __ldcg(p);
+}
+
+// A merge: K poles ds (ascending, distinct), z, 1 / rho.  The warp finds 32 / g roots,
+// g lanes and K0 entries of pf to a root; this lane's is root j.  EPL elements a
+// lane in registers (K0 <= EPL g), or 0: any number, read again for every sum.
+// Out: origin pole o and offset of the root from it.
+template <int EPL, bool LOC>
+__device__ __forceinline__ void find_root(const double* ds, const double* zz, int K, int K0, int g, int j,
+                                          double rinv, float2* pf, int& o_out, double& mu_out) {
+    const int lane = threadIdx.x & 31, gl = lane & (g - 1);
+    const float rf = (float)rinv;
+    const double dj = ld<LOC>(ds + j);
+    double dr[EPL ? EPL : 1], zr[EPL ? EPL : 1];  // poles, z^2
+    if (EPL) {
+#pragma unroll
+        for (int t = 0; t < EPL; ++t) {
+            const int i = gl + g * t;
+            dr[t] = i < K ? ld<LOC>(ds + i) : 8.0;  // z = 0 there
+            zr[t] = i < K ? ld<LOC>(zz + i) : 0.0;
+            if (g * t < K0) zr[t] *= zr[t];
+        }
+    }
+    auto each = [&](auto f) {  // f(i, pole, z^2)
+        if (EPL) {
+#pragma unroll
+            for (int t = 0; t < EPL; ++t)
+                if (g * t < K0) f(gl + g * t, dr[t], zr[t]);
+        } else {
+            for (int i = gl; i < K0; i += g) {
+                const double z = i < K ? ld<LOC>(zz + i) : 0.0;
+                f(i, i < K ? ld<LOC>(ds + i) : 8.0, z * z);
+            }
+        }
+    };
+    // the sum of the terms at org + x in FP64, its derivative and the terms' moduli
+    double f, fp;
+    float fa;
+    auto eval = [&](double org, double x) {
+        double fl = 0.0, fr = 0.0;  // poles up to j, above j
+        fp = 0.0;
+        each([&](int i, double d, double z2) {
+            const double r = rcp((d - org) - x);
+            const double t = z2 * r;
+            if (i <= j) fl += t;
+            else fr += t;
+            fp = fma(t, r, fp);
+        });
+        f = fl + fr;
+        fa = (float)(fr - fl);
+        for (int s = g >> 1; s > 0; s >>= 1) {
+            f += __shfl_xor_sync(0xffffffffu, f, s);
+            fp += __shfl_xor_sync(0xffffffffu, fp, s);
+            fa += __shfl_xor_sync(0xffffffffu, fa, s);
+        }
+        f += rinv;
+        fa += rf;
+    };
+    auto fill = [&](double org) {
+        __syncwarp();
+        each([&](int i, double d, double z2) {  // entries from K on count zero
+            pf[i] = make_float2((float)(d - org), (float)z2);
+        });
+        __syncwarp();
+    };
+    if (LOC)
+        for (int i = K0 + gl; i < BASE; i += g) pf[i] = make_float2(8.f, 0.f);
+    fill(dj);
+    // the root lies within half of its origin; where FP32 rounding (a term is good
+    // to 2^-20, a sum of K / g + 5 likewise) could have the sign at the middle
+    // wrong, it is taken in FP64
+    double half;
+    float sz = 0.f, s = 0.f, sa = 0.f;
+    const bool lastpole = j + 1 >= K;
+    half = lastpole ? 0.0 : 0.5 * (ld<LOC>(ds + j + 1) - dj);
+    {
+        const float hf = (float)half;
+#pragma unroll 4
+        for (int i = gl; i < K0; i += g) {
+            const float2 q = pf[i];
+            const float t = __fdividef(q.y, q.x - hf);
+            sz += q.y;
+            s += t;
+            sa += fabsf(t);
+        }
+    }
+    sz = gsumf(sz, g);
+    s = gsumf(s, g) + rf;
+    sa = gsumf(sa, g) + rf;
+    bool beyond = !lastpole && s < 0.f;
+    const bool unsure = !lastpole && !(fabsf(s) > (float)(K / g + 16) * 0x1p-22f * sa);
+    if (__any_sync(0xffffffffu, unsure)) {
+        eval(dj, half);
+        if (unsure) beyond = __double2hiint(f) < 0;
+    }
+    if (lastpole) half = (double)(sz * 1.0001f) * rcp(rinv);
+    const int o = beyond ? j + 1 : j;
+    const double sg = beyond ? -1.0 : 1.0;
+    const double dorg = beyond ? ld<LOC>(ds + o) : dj;
+    if (__any_sync(0xffffffffu, beyond)) fill(dorg);
+    // FP32: the bits of |offset| to 2^-17 in sections; a base block's groups of four
+    // lanes take four points a lane, larger merges one, by sp lanes where there are
+    // many poles
+    constexpr int PPL = LOC ? 4 : 1;
+    const int lsp = K0 <= 32 ? 0 : K0 <= 64 ? 1 : K0 <= 128 ? 2 : K0 <= 256 ? 3 : 4, sp = 1 << lsp;
+    const int ls = LOC ? 4 : 31 - __clz(g) - lsp;  // log2 of the sections
+    const int pl = gl & (sp - 1), q0 = (gl >> lsp) * PPL;
+    unsigned bl = 0x00800000u, bh = max(__float_as_uint((float)half * 1.001f), bl);
+    const unsigned gmask = (g == 32 ? 0xffffffffu : (1u << g) - 1u) << (lane & ~(g - 1));
+    for (int it = 0; it < 24; ++it) {
+        const bool more = bh > bl + 64u;
+        if (!__any_sync(0xffffffffu, more)) break;
+        const unsigned step = (bh - bl) >> ls;
+        float x[PPL], v[PPL];
+#pragma unroll
+        for (int r = 0; r < PPL; ++r) {
+            x[r] = (float)sg * __uint_as_float(bl + step * (unsigned)(q0 + r));
+            v[r] = rf;
+        }
+        if (LOC) {
+#pragma unroll
+            for (int i = 0; i < BASE; ++i) {
+                const float2 q = pf[i];  // entries from K0 on have z = 0
+#pragma unroll
+                for (int r = 0; r < PPL; ++r) v[r] += q.y * rcpf(q.x - x[r]);
+            }
+        } else {
+            float w = 0.f;
+            v[0] = 0.f;
+#pragma unroll 4
+            for (int i = pl; i < K0; i += 2 * sp) {  // K0 / sp is even
+                const float2 q = pf[i], q2 = pf[i + sp];
+                v[0] += q.y * rcpf(q.x - x[0]);
+                w += q2.y * rcpf(q2.x - x[0]);
+            }
+            v[0] += w;
+            for (int t = sp >> 1; t > 0; t >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], t);
+            v[0] += rf;
+        }
+        unsigned c = 0;  // points below the root, bl first
+#pragma unroll
+        for (int r = 0; r < PPL; ++r)
+            c += (unsigned)__popc(__ballot_sync(0xffffffffu, q0 + r == 0 || (v[r] < 0.f) == (sg > 0.0)) & gmask);
+        c >>= lsp;
+        if (more) {
+            if (c < (1u << ls)) bh = bl + step * c;
+            bl += step * (c - 1);
+        }
+    }
+    // FP64: Newton on x f(x), which has no pole at the origin, inside the bracket
+    // that the signs give.  Steps are compared by their exponents relative to m.
+    double m = fmin((double)__uint_as_float(bl + (bh - bl) / 2), half), ml = 0.0, mh = half * 1.001;
+    int before = -20;
+    bool done = false;
+    for (int it = 0; it < 48; ++it) {
+        const double x = sg * m;
+        eval(dorg, x);
+        if (!done) {
+            if ((__double2hiint(f) < 0) == (sg > 0.0)) ml = m;
+            else mh = m;
+            const double mn = fma(-m * f, rcp(fma(x, fp, f)), m);
+            const int em = expo(m), st = expo(mn - m) - em;
+            const bool noise = expo(f) <= ilogbf(fa) - 51;  // rounding of the sum
+            const ll im = __double_as_longlong(mn);
+            if ((im > __double_as_longlong(ml) && im < __double_as_longlong(mh) && st <= -3) || st <= -21) {
+                m = mn;
+                // converged, or the next step would be (its error is the cube of
+                // this over the square of the last), or as near as the sum allows
+                done = st <= -51 || (before <= -8 && 3 * (st + 1) - 2 * before <= -56) ||
+                       (st >= before - 2 && (noise || st <= -37));
+                before = st;
+            } else if (noise) {  // the sign says nothing
+                done = true;
+            } else {  // halve the bracket's exponent
+                const ll a = __double_as_longlong(fmax(ml, m * 0x1p-16));
+                m = __longlong_as_double((a + __double_as_longlong(mh)) / 2);
+                before = 0;
+            }
+        }
+        if (__all_sync(0xffffffffu, done)) break;
+    }
+    o_out = o;
+    mu_out = sg * m;
+}
+
+// z_i from the roots (Loewner's formula), g lanes to an i
+template <bool LOC>
+__device__ __forceinline__ double new_z(const double* ds, const double* mu, const int* org, const double* z, int K,
+                                        int g, int i) {
+    const int gl = threadIdx.x & (g - 1);
+    const double di = ld<LOC>(ds + i);
+    double pr = 1.0;
+    for (int j = gl; j < K; j += g) {
+        const int oj = min(max(ld<LOC>(org + j), 0), K - 1);
+        const double t = (ld<LOC>(ds + oj) - di) + ld<LOC>(mu + j);  // root j - pole i
+        pr *= j == i ? t : t * rcp(ld<LOC>(ds + j) - di);
+    }
+    for (int s = g >> 1; s > 0; s >>= 1) pr *= __shfl_xor_sync(0xffffffffu, pr, s);
+    return copysign(sqrt(fabs(pr)), ld<LOC>(z + i));
+}
+
+// Coefficients of an eigenvector in the merge's unsorted basis, to u; its norm's inverse.
+template <bool LOC>
+__device__ __forceinline__ double coefficients(const double* ds, const double* zh, const int* idx, double dorg,
+                                               double x, int K, int g, double* u) {
+    const int gl = threadIdx.x & (g - 1);
+    double nrm = 0.0;
+    for (int i = gl; i < K; i += g) {
+        const double v = ld<LOC>(zh + i) * rcp((ld<LOC>(ds + i) - dorg) - x);
+        nrm = fma(v, v, nrm);
+        u[min(max(ld<LOC>(idx + i), 0), K - 1)] = v;
+    }
+    return rsqrt(gsum(nrm, g));
+}
+
+// a warp's shared memory while it merges a base block
+struct BaseMem {
+    double D[BASE], ds[BASE], z[BASE], zh[BASE], mu[BASE], Q[2][BASE * BASE];
+    ll key[BASE], srt[BASE];
+    int org[BASE], idx[BASE];
+    double u[BASE][BASE];
+    float2 pf[BASE][BASE];
+};
+
 template <bool GRID>
 __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ ll s_scan[DW];
     __shared__ unsigned s_max;
     const int n = p.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nt = (int)blockDim.x, nw = nt / 32;
     const int C = (int)gridDim.x, b = (int)blockIdx.x;  // a cluster launch is one cluster
-    const int W = C * DW, wid = b * DW + warp;
+    const int W = C * nw, wid = b + C * warp;
     unsigned arrivals = 0;
     auto sync = [&]() -> bool {
         if (GRID) {
             arrivals += (unsigned)C;
             return grid_sync(p.bar, p.err, arrivals);
         }
-        __threadfence();
         cluster_sync();
         return true;
     };
@@ -122,7 +382,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
     __syncthreads();
     {
         unsigned m = 0;
-        for (int i = tid; i < n; i += DT) {
+        for (int i = tid; i < n; i += nt) {
             m = max(m, (unsigned)__double2hiint(p.d[i]) & 0x7fffffffu);
             if (i + 1 < n) m = max(m, (unsigned)__double2hiint(p.e[i]) & 0x7fffffffu);
         }
@@ -133,17 +393,109 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
     const int ex = min(max((int)(s_max >> 20) - 1022, -900), 900);
     const double down = scalbn(1.0, -ex), up = s_max ? scalbn(1.0, ex) : 0.0;
     const double rho_min = 0x1p-58;
-    // 1 x 1 blocks
-    for (int i = b * DT + tid; i < n; i += C * DT) {
-        double x = p.d[i] * down;
-        if (i > 0) x -= fmax(fabs(p.e[i - 1] * down), rho_min);
-        if (i + 1 < n) x -= fmax(fabs(p.e[i] * down), rho_min);
-        p.D[i] = x;
-        p.Qa[i + (size_t)n * i] = 1.0;
+    double *Q = p.Qa, *Qn = p.Qb;
+    // ---- base blocks: a warp each, levels 2, 4 and 8 in its shared memory ------------
+    for (int B = wid; B * BASE < n; B += W) {
+        BaseMem& s = *reinterpret_cast<BaseMem*>(dsm + (size_t)warp * sizeof(BaseMem));
+        const int r0 = B * BASE, N = min(BASE, n - r0), i = lane & (BASE - 1);
+        __syncwarp();
+        if (lane < N) {
+            double x = p.d[r0 + i] * down;
+            if (r0 + i > 0) x -= fmax(fabs(p.e[r0 + i - 1] * down), rho_min);
+            if (r0 + i + 1 < n) x -= fmax(fabs(p.e[r0 + i] * down), rho_min);
+            s.D[i] = x;
+        }
+        for (int t = lane; t < BASE * BASE; t += 32) s.Q[0][t] = t % BASE == t / BASE ? 1.0 : 0.0;
+        int cur = 0;
+        for (int h = 1; h < N; h *= 2) {
+            const int K0 = 2 * h;
+            __syncwarp();
+            const double *q = s.Q[cur];
+            double* qn = s.Q[cur ^ 1];
+            {  // poles: lanes 0..7
+                const int lo = i / K0 * K0, mid = lo + h, hi = min(lo + K0, N);
+                const bool on = lane < N && mid < N;
+                if (lane < N) s.key[i] = okey(s.D[i]);
+                __syncwarp();
+                int rk = i - lo;
+                if (on) {
+                    const ll k = s.key[i];
+                    rk = 0;
+                    for (int t = lo; t < hi; ++t) rk += s.key[t] < k || (s.key[t] == k && t < i);
+                    double z = i < mid ? q[(mid - 1) + BASE * i] : copysign(1.0, p.e[r0 + mid - 1]) * q[mid + BASE * i];
+                    if (expo(z) < -56) z = copysign(0x1p-56, z);
+                    s.srt[lo + rk] = k;
+                    s.z[lo + rk] = z;
+                    s.idx[lo + rk] = i - lo;
+                }
+                __syncwarp();
+                if (on) {  // i as a place in the order
+                    const double v = unkey(s.srt[i]);
+                    const int r = i - lo;
+                    ll run = LLONG_MIN / 2;
+                    for (int t = 0; t < r; ++t) run = max(run, to_grid(unkey(s.srt[lo + t])) - t);
+                    s.ds[i] = to_grid(v) < run + r ? from_grid(run + r) : v;
+                }
+                __syncwarp();
+            }
+            // roots: groups of four lanes
+            const int g = 4, jj = min(lane / g, N - 1);
+            {
+                const int lo = jj / K0 * K0, mid = lo + h;
+                const bool on = lane / g < N && mid < N;
+                // lanes without a root follow the first
+                const int lo1 = on ? lo : 0, j = on ? jj - lo : 0, K = min(lo1 + K0, N) - lo1;
+                const double rinv = rcp(fmax(fabs(p.e[r0 + lo1 + h - 1] * down), rho_min));
+                int o;
+                double mu;
+                find_root<2, true>(s.ds + lo1, s.z + lo1, K, K0, g, j, rinv, s.pf[lane / g], o, mu);
+                __syncwarp();
+                if (on && (lane & (g - 1)) == 0) {
+                    double lam = s.ds[lo + o] + mu;
+                    lam = fmax(lam, s.ds[jj]);
+                    if (j + 1 < K) lam = fmin(lam, s.ds[jj + 1]);
+                    s.org[jj] = o;
+                    s.mu[jj] = mu;
+                    s.D[jj] = lam;
+                }
+                __syncwarp();
+                const double zh = new_z<true>(s.ds + lo1, s.mu + lo1, s.org + lo1, s.z + lo1, K, g, j);
+                if (on && (lane & (g - 1)) == 0) s.zh[jj] = zh;
+                __syncwarp();
+                double* u = s.u[lane / g];
+                const int jr = on ? jj : 0;
+                const double inv = coefficients<true>(s.ds + lo1, s.zh + lo1, s.idx + lo1, s.ds[lo1 + s.org[jr]],
+                                                      s.mu[jr], K, g, u);
+                __syncwarp();
+                if (lane / g < N)
+                    for (int r = lane & (g - 1); r < K0 && lo + r < N; r += g) {
+                        const int row = lo + r;
+                        double v = 0.0;
+                        if (on) {
+                            const int i0 = row < mid ? 0 : h, i1 = row < mid ? h : K;
+                            for (int t = i0; t < i1; ++t) v = fma(q[row + BASE * (lo + t)], u[t], v);
+                            v *= inv;
+                        } else {
+                            v = q[row + BASE * jj];
+                        }
+                        qn[row + BASE * jj] = v;
+                    }
+            }
+            cur ^= 1;
+        }
+        __syncwarp();
+        if (lane < N) p.D[r0 + i] = s.D[i];
+        if (n > BASE) {
+            for (int t = lane; t < N * N; t += 32)
+                Q[r0 + t % N + (size_t)n * (r0 + t / N)] = s.Q[cur][t % N + BASE * (t / N)];
+        } else {
+            for (int t = lane; t < N * p.want; t += 32)
+                p.Z[t % N + N * (t / N)] = s.Q[cur][t % N + BASE * (N - 1 - t / N)];
+            if (lane < p.want) p.lam_asc[lane] = s.D[N - p.want + lane] * up;
+        }
     }
     if (!sync()) return;
-    double *Q = p.Qa, *Qn = p.Qb;
-    for (int h = 1; h < n; h *= 2) {
+    for (int h = BASE; h < n; h *= 2) {
         const int K0 = 2 * h, nm = (n + K0 - 1) / K0;
         const bool last = K0 >= n;
         // ---- poles of every merge: one block each -----------------------------
@@ -153,9 +505,11 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
             ll* key = reinterpret_cast<ll*>(dsm);
             ll* srt = key + K;
             const double ev = p.e[mid - 1];
-            for (int i = tid; i < K; i += DT) key[i] = okey(__ldcg(p.D + lo + i));
+            for (int i = tid; i < K; i += nt) key[i] = okey(__ldcg(p.D + lo + i));
             __syncthreads();
-            for (int i = tid; i < K; i += DT) {
+            for (int i = tid; i < K; i += nt) {
+                double z = i < h ? __ldcg(Q + (mid - 1) + (size_t)n * (lo + i))
+                                 : copysign(1.0, ev) * __ldcg(Q + mid + (size_t)n * (lo + i));
                 const ll k = key[i];
                 const int base = i < h ? h : 0;  // the other block; ties: first block first
                 int l = 0, r = i < h ? K - h : h;
@@ -167,9 +521,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
                 }
                 const int rk = min((i < h ? i : i - h) + l, K - 1);
                 srt[rk] = k;
-                double z = i < h ? __ldcg(Q + (mid - 1) + (size_t)n * (lo + i))
-                                 : copysign(1.0, ev) * __ldcg(Q + mid + (size_t)n * (lo + i));
-                if (!(fabs(z) >= 0x1p-56)) z = copysign(0x1p-56, z);
+                if (expo(z) < -56) z = copysign(0x1p-56, z);
                 p.z[lo + rk] = z;
                 p.idx[lo + rk] = i;
             }
@@ -177,7 +529,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
             // distinct: on a grid of ulps, 2^-82 below 2^-30, pole r at least one
             // step above pole r-1 (a prefix maximum); poles that are distinct
             // already stay
-            const int per = (K + DT - 1) / DT, r0 = min(tid * per, K), r1 = min(r0 + per, K);
+            const int per = (K + nt - 1) / nt, r0 = min(tid * per, K), r1 = min(r0 + per, K);
             ll mx = LLONG_MIN / 2;
             for (int r = r0; r < r1; ++r) mx = max(mx, to_grid(unkey(srt[r])) - r);
             ll inc = mx;
@@ -201,144 +553,42 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
             __syncthreads();
         }
         if (!sync()) return;
-        // ---- roots: a warp each ------------------------------------------------
+        // groups of g lanes, gw of them to a warp; unit u of the level at lane's group
+        const int g = min(K0, 32), gw = 32 / g, gl = lane & (g - 1), sub = lane / g;
+        // ---- roots ----------------------------------------------------------------
         if (warp < p.warps2) {
-            for (int g = b + C * warp; g < n; g += C * p.warps2) {
-                const int lo = g / K0 * K0, mid = lo + h, hi = min(lo + K0, n), K = hi - lo, j = g - lo;
-                if (mid >= n) continue;
-                float2* pf = reinterpret_cast<float2*>(dsm) + (size_t)warp * K0;
-                const double* ds = p.ds + lo;
-                const double* zz = p.z + lo;
+            for (int u0 = wid * gw; u0 < n; u0 += C * p.warps2 * gw) {
+                const int r = u0 + sub;
+                // an unpaired block or none: lanes follow the level's first root
+                const bool on = r < n && r / K0 * K0 + h < n;
+                if (!__any_sync(0xffffffffu, on)) continue;
+                const int G = on ? r : 0, lo = G / K0 * K0, mid = lo + h, K = min(lo + K0, n) - lo, j = G - lo;
+                float2* pf = reinterpret_cast<float2*>(dsm) + (size_t)warp * max(K0, 32) + sub * K0;
                 const double rinv = rcp(fmax(fabs(p.e[mid - 1] * down), rho_min));
-                const float rf = (float)rinv;
-                const double dj = __ldcg(ds + j);
-                __syncwarp();
-                float sz = 0.f;
-                for (int i = lane; i < K; i += 32) {
-                    const float zf = (float)__ldcg(zz + i);
-                    pf[i] = make_float2((float)(__ldcg(ds + i) - dj), zf * zf);
-                    sz += zf * zf;
+                int o;
+                double mu;
+                if (K0 <= 128) find_root<4, false>(p.ds + lo, p.z + lo, K, K0, g, j, rinv, pf, o, mu);
+                else find_root<0, false>(p.ds + lo, p.z + lo, K, K0, g, j, rinv, pf, o, mu);
+                if (on && gl == 0) {
+                    double lam = __ldcg(p.ds + lo + o) + mu;
+                    lam = fmax(lam, __ldcg(p.ds + G));
+                    if (j + 1 < K) lam = fmin(lam, __ldcg(p.ds + G + 1));
+                    p.org[G] = o;
+                    p.mu[G] = mu;
+                    p.D[G] = lam;
                 }
                 __syncwarp();
-                auto evalf = [&](float x) {
-                    float s = 0.f;
-                    for (int i = lane; i < K; i += 32) s += __fdividef(pf[i].y, pf[i].x - x);
-                    return wsumf(s) + rf;
-                };
-                // sum of the terms at x = sg m in FP64, its derivative and the terms' moduli
-                double f, fp;
-                float fa;
-                auto eval = [&](double org, double x) {
-                    double fl = 0.0, fr = 0.0;  // poles up to j, above j
-                    fp = 0.0;
-                    for (int i = lane; i < K; i += 32) {
-                        const double r = rcp((__ldcg(ds + i) - org) - x), zi = __ldcg(zz + i);
-                        const double t = zi * zi * r;
-                        if (i <= j) fl += t;
-                        else fr += t;
-                        fp = fma(t, r, fp);
-                    }
-                    f = fl + fr;
-                    fa = wsumf((float)(fr - fl)) + rf;
-#pragma unroll
-                    for (int s = 16; s > 0; s >>= 1) {
-                        f += __shfl_xor_sync(0xffffffffu, f, s);
-                        fp += __shfl_xor_sync(0xffffffffu, fp, s);
-                    }
-                    f += rinv;
-                };
-                int o = j;
-                // the root lies within half of its origin; where FP32 rounding (a
-                // term is good to 2^-20, a sum of K / 32 + 5 likewise) could have
-                // the sign at the middle wrong, it is taken in FP64
-                double half;
-                if (j + 1 < K) {
-                    half = 0.5 * (__ldcg(ds + j + 1) - dj);
-                    float s = 0.f, sa = 0.f;
-                    for (int i = lane; i < K; i += 32) {
-                        const float t = __fdividef(pf[i].y, pf[i].x - (float)half);
-                        s += t;
-                        sa += fabsf(t);
-                    }
-                    s = wsumf(s) + rf;
-                    sa = wsumf(sa) + rf;
-                    bool beyond = s < 0.f;
-                    if (!(fabsf(s) > (float)(K / 32 + 16) * 0x1p-22f * sa)) {
-                        eval(dj, half);
-                        beyond = f < 0.0;
-                    }
-                    if (beyond) {
-                        o = j + 1;
-                        const double d1 = __ldcg(ds + o);
-                        __syncwarp();
-                        for (int i = lane; i < K; i += 32) pf[i].x = (float)(__ldcg(ds + i) - d1);
-                        __syncwarp();
-                    }
-                } else {
-                    half = (double)(wsumf(sz) * 1.0001f) / rinv;
-                }
-                const double sg = o == j ? 1.0 : -1.0;
-                const double dorg = o == j ? dj : __ldcg(ds + o);
-                // FP32: bisection on the bits of |offset| to 2^-15
-                unsigned bl = 0x00800000u, bh = __float_as_uint((float)half * 1.001f);
-                for (int it = 0; it < 23 && bh > bl + 64u; ++it) {
-                    const unsigned bm = bl + (bh - bl) / 2;
-                    const float f = evalf((float)sg * __uint_as_float(bm));
-                    if ((f < 0.f) == (sg > 0.0)) bl = bm;
-                    else bh = bm;
-                }
-                // FP64: Newton on x f(x), which has no pole at the origin, inside
-                // the bracket that the signs give
-                double m = (double)__uint_as_float(bl + (bh - bl) / 2), ml = 0.0, mh = half * 1.001;
-                m = fmin(m, half);
-                double before = 1e300;
-                for (int it = 0; it < 48; ++it) {
-                    const double x = sg * m;
-                    eval(dorg, x);
-                    if ((f < 0.0) == (sg > 0.0)) ml = m;
-                    else mh = m;
-                    const double den = fma(x, fp, f);
-                    const double mn = m - m * f * rcp(den);
-                    const double st = fabs(mn - m);
-                    const bool noise = fabs(f) <= (double)(fa * 0x1p-50f);  // rounding of the sum
-                    if ((mn > ml && mn < mh && st <= 0.3 * m) || st <= 0x1p-20 * m) {
-                        m = mn;
-                        // converged, or as near as rounding of the sum allows
-                        if (st <= 0x1p-50 * m || (st >= 0.25 * before && (noise || st <= 0x1p-36 * m))) break;
-                        before = st;
-                    } else if (noise) {  // the sign says nothing
-                        break;
-                    } else {  // halve the bracket's exponent
-                        const ll a = __double_as_longlong(fmax(ml, m * 0x1p-16));
-                        m = __longlong_as_double((a + __double_as_longlong(mh)) / 2);
-                        before = 1e300;
-                    }
-                }
-                if (lane == 0) {
-                    double lam = fma(sg, m, dorg);
-                    if (lam < dj) lam = dj;
-                    if (j + 1 < K) lam = fmin(lam, __ldcg(ds + j + 1));
-                    p.org[g] = o;
-                    p.mu[g] = sg * m;
-                    p.D[g] = lam;
-                }
             }
         }
         if (!sync()) return;
         // ---- z from the roots ---------------------------------------------------
-        for (int g = wid; g < n; g += W) {
-            const int lo = g / K0 * K0, mid = lo + h, hi = min(lo + K0, n), K = hi - lo, i = g - lo;
-            if (mid >= n) continue;
-            const double di = __ldcg(p.ds + g);
-            double pr = 1.0;
-            for (int j = lane; j < K; j += 32) {
-                const int oj = min(max(__ldcg(p.org + lo + j), 0), K - 1);
-                const double t = (__ldcg(p.ds + lo + oj) - di) + __ldcg(p.mu + lo + j);  // root j - pole i
-                pr *= j == i ? t : t * rcp(__ldcg(p.ds + lo + j) - di);
-            }
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) pr *= __shfl_xor_sync(0xffffffffu, pr, s);
-            if (lane == 0) p.zh[g] = copysign(sqrt(fabs(pr)), __ldcg(p.z + g));
+        for (int u0 = wid * gw; u0 < n; u0 += W * gw) {
+            const int r = u0 + sub;
+            const bool on = r < n && r / K0 * K0 + h < n;
+            if (!__any_sync(0xffffffffu, on)) continue;
+            const int G = on ? r : 0, lo = G / K0 * K0, K = min(lo + K0, n) - lo;
+            const double zh = new_z<false>(p.ds + lo, p.mu + lo, p.org + lo, p.z + lo, K, g, G - lo);
+            if (on && gl == 0) p.zh[G] = zh;
         }
         if (!sync()) return;
         // ---- eigenvectors: Q blockdiag times the rank-one problem's ---------------
@@ -347,30 +597,28 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
         const int g0 = last ? n - p.want : 0, cols = n - g0;
         int wpc = 1;
         while (wpc < 16 && 2 * wpc * cols <= C * p.warps2 && 32 * wpc < K0) wpc *= 2;
-        for (int unit = b + C * warp; unit < cols * wpc && warp < p.warps2; unit += C * p.warps2) {
-            const int g = g0 + unit / wpc, part = unit % wpc;
-            const int lo = g / K0 * K0, mid = lo + h, hi = min(lo + K0, n), K = hi - lo;
-            double* out = last ? p.Z + (size_t)n * (n - 1 - g) : Qn + (size_t)n * g;
-            if (last && part == 0 && lane == 0) p.lam_asc[g - g0] = __ldcg(p.D + g) * up;
-            if (mid >= n) {  // unpaired
-                for (int r = lo + 32 * part + lane; r < hi; r += 32 * wpc)
-                    out[r] = __ldcg(Q + r + (size_t)n * g);
+        for (int u0 = wid * gw; u0 < cols * wpc && warp < p.warps2; u0 += C * p.warps2 * gw) {
+            const int unit = u0 + sub;
+            const bool have = unit < cols * wpc;
+            const int c = g0 + (have ? unit : 0) / wpc, part = (have ? unit : 0) % wpc;
+            const int lo = c / K0 * K0, mid = lo + h, hi = min(lo + K0, n);
+            const bool on = mid < n;
+            double* out = last ? p.Z + (size_t)n * (n - 1 - c) : Qn + (size_t)n * c;
+            if (have && last && part == 0 && gl == 0) p.lam_asc[c - g0] = __ldcg(p.D + c) * up;
+            double* u = reinterpret_cast<double*>(dsm) + (size_t)warp * max(K0, 32) + sub * K0;
+            // lanes without a merged column form the first column's coefficients
+            const int cc = on ? c : 0, lc = on ? lo : 0, K = min(lc + K0, n) - lc;
+            const int og = min(max(__ldcg(p.org + cc), 0), K - 1);
+            __syncwarp();
+            const double inv = coefficients<false>(p.ds + lc, p.zh + lc, p.idx + lc, __ldcg(p.ds + lc + og),
+                                                   __ldcg(p.mu + cc), K, g, u);
+            __syncwarp();
+            if (!have) continue;
+            if (!on) {  // unpaired
+                for (int r = lo + g * part + gl; r < hi; r += g * wpc) out[r] = __ldcg(Q + r + (size_t)n * c);
                 continue;
             }
-            double* u = reinterpret_cast<double*>(dsm) + (size_t)warp * K0;
-            const int og = min(max(__ldcg(p.org + g), 0), K - 1);
-            const double dorg = __ldcg(p.ds + lo + og), x = __ldcg(p.mu + g);
-            double nrm = 0.0;
-            __syncwarp();
-            for (int i = lane; i < K; i += 32) {
-                const double v = __ldcg(p.zh + lo + i) * rcp((__ldcg(p.ds + lo + i) - dorg) - x);
-                nrm = fma(v, v, nrm);
-                u[min(max(__ldcg(p.idx + lo + i), 0), K - 1)] = v;
-            }
-            nrm = wsum(nrm);
-            const double inv = rsqrt(nrm);
-            __syncwarp();
-            for (int r = lo + 32 * part + lane; r < hi; r += 32 * wpc) {
+            for (int r = lo + g * part + gl; r < hi; r += g * wpc) {
                 const bool top = r < mid;
                 const int i0 = top ? 0 : h, i1 = top ? h : K;
                 const double* q = Q + r + (size_t)n * lo;
@@ -439,12 +687,13 @@ void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t 
     while (K0 < n) K0 *= 2;
     // a warp's copy of the poles is 8 bytes an entry, so are its coefficients;
     // the block that sorts a merge needs 16 bytes an entry
-    a.warps2 = (int)std::min<int64_t>(DW, (int64_t)(DSMEM / (8 * K0)));
+    const bool grid = n > 128 || ctx->trd_clusters == 0;
+    const int nw = !grid && n <= 64 ? 4 : DW;  // warps of a block
+    a.warps2 = (int)std::min<int64_t>(nw, (int64_t)(DSMEM / (8 * K0)));
     TN_REQUIRE(a.warps2 >= 2, "tridiag_top: order too large");
-    const size_t dyn = (size_t)8 * K0 * a.warps2;
+    const size_t dyn = std::max<size_t>((size_t)8 * std::max<int64_t>(K0, 32) * a.warps2, sizeof(BaseMem) * nw);
     // One cluster (barrier 0.2 us against 1.2) while its sixteen SMs hold the
     // FP64 work of a level, the whole grid above.
-    const bool grid = n > 128 || ctx->trd_clusters == 0;
     if (grid) {
         TN_CHECK_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), ctx->stream));
         TN_CHECK_CUDA(cudaFuncSetAttribute(dc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -453,8 +702,8 @@ void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t 
         TN_CHECK_CUDA(cudaLaunchCooperativeKernel((void*)dc_kernel<true>, dim3((unsigned)ctx->sm_count),
                                                   dim3(DT), args, dyn, ctx->stream));
     } else {
-        // blocks: a warp per root
-        const int C = n <= 8 ? 1 : n <= 16 ? 2 : n <= 32 ? 4 : n <= 64 ? 8 : DC_CLUSTER;
+        // blocks: a warp per root at the last level, up to order 64 one on each scheduler
+        const int C = n <= 8 ? 1 : n <= 16 ? 2 : n <= 32 ? 8 : DC_CLUSTER;
         TN_CHECK_CUDA(cudaFuncSetAttribute(dc_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at;
@@ -462,7 +711,7 @@ void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t 
         at.val.clusterDim.x = (unsigned)C;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.gridDim = dim3((unsigned)C);
-        cfg.blockDim = dim3(DT);
+        cfg.blockDim = dim3(32 * nw);
         cfg.dynamicSmemBytes = dyn;
         cfg.stream = ctx->stream;
         cfg.attrs = &at;

@@ -12,8 +12,8 @@
 //
 // GB300 issues FP64 at two FMAs per clock per SM and each FP64 instruction of a
 // warp takes 64 clocks, so serial recurrences and reductions cost most; steps 1
-// and 2 say how each avoids them.  Order 64 with 32 vectors takes 0.58 ms, 128 with
-// 64 1.09, 256 with 128 2.64 (reduction 2.07), 512 with 256 7.7 (6.6).
+// and 2 say how each avoids them.  Order 64 with 32 vectors takes 0.41 ms, 128 with
+// 64 0.85, 256 with 128 2.3 (reduction 1.9), 512 with 256 5.3 (4.4).
 #include <cmath>
 
 #include "common.cuh"
