@@ -72,9 +72,11 @@ struct Ctx {
     Scratch s_gram, s_eigval, s_work, s_x, s_y, s_t1, s_t2, s_dot, s_coef, s_mixa, s_mixb, s_mixc,
         s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz, s_trd, s_bt, s_dc;
     int* d_info = nullptr;
-    // grid-barrier words of the eigensolver's cooperative kernels: arrival
-    // count, generation, and an error word set when a bounded wait ran out
+    // words of kernels whose blocks wait or count: 0 arrivals and 2 error of the
+    // eigensolver's barriers (a bounded wait ran out), 3 blocks done of a dot
+    // product, 4 arrivals, 5 exits and 6 error of a Lanczos step
     unsigned* d_bar = nullptr;
+    uint64_t lanczos_calls = 0;
     int trd_clusters = -1;  // 16-block clusters the GPU holds at once (-1: not asked yet)
     int* d_err = nullptr;  // set by device code when a bounded wait runs out
     // mixed precision on: environment updates and truncation projections run
@@ -189,6 +191,7 @@ void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int
 // out[j] = <v_j, w> for K vectors; result left in device memory dout (K cplx).
 void multi_dot(Ctx* ctx, const cplx* const* dV, int K, const cplx* w, int64_t n, cplx* dout);
 // w += sum_j coef[j] * v_j, coef on the device (K cplx); sign applied to coefs.
+double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, cplx* comp);
 void multi_axpy(Ctx* ctx, cplx* w, const cplx* const* dV, const cplx* dcoef, int K, int64_t n,
                 double sign);
 void zscale(Ctx* ctx, cplx* x, int64_t n, cplx a);

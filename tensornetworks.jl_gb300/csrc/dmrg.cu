@@ -101,7 +101,7 @@ static LanczosOut lanczos_lowest(Ctx* ctx, int64_t n, const cplx* x0, const MatV
 
     std::vector<double> H((size_t)(kd + 1) * (kd + 1), 0.0);
     auto h = [&](int i, int j) -> double& { return H[(size_t)i * (kd + 1) + j]; };
-    cplx* dcoef = ctx->s_coef.c(ctx, 4 * (kd + 2) + (size_t)(kd + 1) * (kd + 1));
+    cplx* dcoef = ctx->s_coef.c(ctx, (size_t)(kd + 1) * (kd + 1));
     int K = 0, numiter = 1;
     int64_t numops = 0;
     std::vector<double> D, U;
@@ -115,30 +115,19 @@ static LanczosOut lanczos_lowest(Ctx* ctx, int64_t n, const cplx* x0, const MatV
         ++numops;
         ptr.clear();
         for (int j = 0; j <= K; ++j) ptr.push_back(V[j].c());
-        // classical Gram-Schmidt, twice (full reorthogonalisation in FP64)
-        multi_dot(ctx, ptr.data(), K + 1, W.c(), n, dcoef);
-        multi_axpy(ctx, W.c(), ptr.data(), dcoef, K + 1, n, -1.0);
-        multi_dot(ctx, ptr.data(), K + 1, W.c(), n, dcoef + (kd + 2));
-        multi_axpy(ctx, W.c(), ptr.data(), dcoef + (kd + 2), K + 1, n, -1.0);
-        double* hp = ctx->pinned(4 * (kd + 2));
-        TN_CHECK_CUDA(cudaMemcpyAsync(hp, dcoef, sizeof(cplx) * 2 * (kd + 2),
-                                      cudaMemcpyDeviceToHost, ctx->stream));
-        ctx->sync();
-        for (int j = 0; j <= K; ++j) {
-            const double v = hp[2 * j] + hp[2 * (kd + 2 + j)];
-            h(j, K) = v;
-            h(K, j) = v;
-        }
+        // classical Gram-Schmidt, twice (full reorthogonalisation in FP64); W
+        // comes back normalised
+        cplx comp[49];
+        beta = lanczos_orth(ctx, ptr.data(), K + 1, W.c(), n, comp);
+        for (int j = 0; j <= K; ++j) h(j, K) = h(K, j) = comp[j].x;
         if (first && K >= 1) {  // <x0|H v_K> = <H x0|v_K>: rho for K = 1, else 0
             h(0, K) = K == 1 ? resid0 : 0.0;
             h(K, 0) = h(0, K);
         }
         ++K;
-        beta = std::sqrt(znorm2(ctx, W.c(), n));
         if (K == 1) resid0 = beta;
         const bool invariant = beta <= tol || K >= n;
         if (K < kd && !invariant) {
-            zscale(ctx, W.c(), n, cmk(1.0 / beta, 0.0));
             V[K] = std::move(W);
             W = DBuf(ctx, sizeof(cplx) * n);
             continue;
@@ -161,7 +150,7 @@ static LanczosOut lanczos_lowest(Ctx* ctx, int64_t n, const cplx* x0, const MatV
                 hc[2 * ((size_t)j * K + i)] = U[(size_t)i * K + j];
                 hc[2 * ((size_t)j * K + i) + 1] = 0.0;
             }
-        cplx* dU = dcoef + 2 * (kd + 2);
+        cplx* dU = dcoef;
         TN_CHECK_CUDA(cudaMemcpyAsync(dU, hc, sizeof(cplx) * K * keep, cudaMemcpyHostToDevice,
                                       ctx->stream));
         ptr.clear();
@@ -175,7 +164,6 @@ static LanczosOut lanczos_lowest(Ctx* ctx, int64_t n, const cplx* x0, const MatV
         ctx->sync();
         for (int j = 0; j < keep; ++j) V[j] = std::move(Y[j]);
         for (int j = keep; j <= kd; ++j) V[j].reset();
-        zscale(ctx, W.c(), n, cmk(1.0 / beta, 0.0));
         V[keep] = std::move(W);
         W = DBuf(ctx, sizeof(cplx) * n);
         std::fill(H.begin(), H.end(), 0.0);
@@ -193,7 +181,7 @@ static LanczosOut lanczos_lowest(Ctx* ctx, int64_t n, const cplx* x0, const MatV
         hc[2 * i] = U[(size_t)i * K + 0];
         hc[2 * i + 1] = 0.0;
     }
-    cplx* dU = dcoef + 2 * (kd + 2);
+    cplx* dU = dcoef;
     TN_CHECK_CUDA(cudaMemcpyAsync(dU, hc, sizeof(cplx) * K, cudaMemcpyHostToDevice, ctx->stream));
     ptr.clear();
     for (int i = 0; i < K; ++i) ptr.push_back(V[i].c());

@@ -8,6 +8,7 @@
 // thread keeps the DFMA pipe busy while shared-memory traffic stays far below
 // its bandwidth.
 #include "common.cuh"
+#include "grid_dev.cuh"
 
 namespace tn {
 
@@ -244,34 +245,110 @@ void zgemm_dispatch_b(Ctx* ctx, Op opb, dim3 grid, int64_t m, int64_t n, int64_t
 }
 
 // -------------------------------------------------------------------------
-__global__ void small_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
-                                   const cplx* __restrict__ M, int nI, int nJ, int64_t na,
-                                   int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o,
-                                   int64_t ldc_o, int accumulate) {
+// out[a, J, c] = sum_I in[a, I, c] M[I, J].  Two-site MPO tensors are mostly zero (28
+// of 144 entries for the transverse-field Ising chain, 52 of 400 for XXZ), and FP64
+// is what bounds this kernel, so every block lists the nonzero entries of M's
+// columns, real ones, imaginary ones (two multiply-adds either) and the rest (four),
+// and a thread multiplies those; a column of the input with an infinity or NaN takes
+// all entries, as 0 times it is NaN.  parts threads share a column's J.
+// Against all entries of four J at a time by one thread: bond dimension 64, 12 x 12:
+// 41.0 -> 8.2 us; 20 x 20: 104.5 -> 13.4, at 256 204 -> 30.7 (10.7 of them FP64).
+__global__ void __launch_bounds__(128) small_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
+                                                          const cplx* __restrict__ M, int nI, int nJ, int64_t na,
+                                                          int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o,
+                                                          int64_t ldc_o, int accumulate, int parts) {
     extern __shared__ cplx sM[];
+    unsigned short* li = reinterpret_cast<unsigned short*>(sM + nI * nJ);  // nonzero I of column J
+    unsigned short* cnt = li + nI * nJ;  // 3 to a column: where each kind ends
+    const int lane = threadIdx.x & 31;
     for (int t = threadIdx.x; t < nI * nJ; t += blockDim.x) sM[t] = M[t];
     __syncthreads();
-    const int64_t total = na * nc;
+    for (int J = threadIdx.x >> 5; J < nJ; J += blockDim.x >> 5) {
+        int c = 0;
+        for (int kind = 0; kind < 3; ++kind) {
+            for (int I0 = 0; I0 < nI; I0 += 32) {
+                const int I = I0 + lane;
+                bool on = false;
+                if (I < nI) {
+                    const cplx v = sM[I + nI * J];
+                    on = kind == (v.y == 0.0 ? (v.x == 0.0 ? 3 : 0) : v.x == 0.0 ? 1 : 2);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, on);
+                if (on) li[nI * J + c + __popc(m & ((1u << lane) - 1u))] = (unsigned short)I;
+                c += __popc(m);
+            }
+            if (lane == 0) cnt[3 * J + kind] = (unsigned short)c;
+        }
+    }
+    __syncthreads();
+    const int64_t total = na * nc * parts;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = idx % na, c = idx / na;
+        const int64_t a = idx % na, c = idx / na % nc;
+        const int part = (int)(idx / (na * nc));
         const cplx* x = in + a + ldc_i * c;
         cplx* y = out + a + ldc_o * c;
-        for (int J0 = 0; J0 < nJ; J0 += 4) {
-            cplx s[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-            for (int I = 0; I < nI; ++I) {
-                const cplx v = x[lda_i * I];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (J0 + j < nJ) s[j] = cfma(v, sM[I + nI * (J0 + j)], s[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (J0 + j >= nJ) break;
-                cplx* dst = y + lda_o * (J0 + j);
-                *dst = accumulate ? cadd(*dst, s[j]) : s[j];
-            }
+        bool bad = false;
+        for (int I = 0; I < nI; ++I) {
+            const cplx v = x[lda_i * I];
+            bad |= (__double2hiint(v.x) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(v.y) & 0x7ff00000) == 0x7ff00000;
         }
+        for (int J = part; J < nJ; J += parts) {
+            cplx s = cmk(0, 0);
+            if (bad) {
+                for (int I = 0; I < nI; ++I) s = cfma(x[lda_i * I], sM[I + nI * J], s);
+            } else {
+                const unsigned short* l = li + nI * J;
+                const cplx* m = sM + nI * J;
+                const int n0 = cnt[3 * J], n1 = cnt[3 * J + 1], n2 = cnt[3 * J + 2];
+#pragma unroll 4
+                for (int t = 0; t < n0; ++t) {
+                    const cplx v = x[lda_i * l[t]];
+                    const double r = m[l[t]].x;
+                    s = cmk(fma(v.x, r, s.x), fma(v.y, r, s.y));
+                }
+#pragma unroll 2
+                for (int t = n0; t < n1; ++t) {
+                    const cplx v = x[lda_i * l[t]];
+                    const double r = m[l[t]].y;
+                    s = cmk(fma(-v.y, r, s.x), fma(v.x, r, s.y));
+                }
+#pragma unroll 2
+                for (int t = n1; t < n2; ++t) s = cfma(x[lda_i * l[t]], m[l[t]], s);
+            }
+            cplx* dst = y + lda_o * J;
+            *dst = accumulate ? cadd(*dst, s) : s;
+        }
+    }
+}
+
+// The same for nI <= 4 (gates and operators on one or two spin-1/2 legs), a thread per
+// output and all loads at once: what takes the time there is one load's latency, and
+// lists of nonzeros would be two more (2 x 2: 5.2 us with them, 4.1 without;
+// 4 x 4 at bond dimension 32: 6.2 and 4.1).
+__global__ void __launch_bounds__(128) dense_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
+                                                          const cplx* __restrict__ M, int nI, int nJ, int64_t na,
+                                                          int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o,
+                                                          int64_t ldc_o, int accumulate) {
+    const int64_t total = na * nc * nJ;
+    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t a = idx % na, c = idx / na / nJ;
+        const int J = (int)(idx / na % nJ);
+        const cplx* x = in + a + ldc_i * c;
+        cplx v[4], m[4];
+#pragma unroll
+        for (int I = 0; I < 4; ++I)
+            if (I < nI) {
+                v[I] = x[lda_i * I];
+                m[I] = M[I + nI * J];
+            }
+        cplx s = cmk(0, 0);
+#pragma unroll
+        for (int I = 0; I < 4; ++I)
+            if (I < nI) s = cfma(v[I], m[I], s);
+        cplx* dst = out + a + ldc_o * c + lda_o * J;
+        *dst = accumulate ? cadd(*dst, s) : s;
     }
 }
 
@@ -290,10 +367,42 @@ __device__ inline cplx warp_sum(cplx v) {
     return v;
 }
 
-// partial[blk*K + j] = sum over this block's slice of conj(v_j[i]) * w[i]
+// Sum of all blocks' partials of K outputs by the block that comes last, one warp per
+// output in fixed order (a launch of its own for that took 3.3 us).  red: the
+// block's partials, in shared memory; count is zero before and after.
+__device__ inline void last_block_sum(const cplx* red, int K, cplx* __restrict__ partial, cplx* __restrict__ out,
+                                      unsigned* __restrict__ count) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (gridDim.x == 1) {
+        if (t < K) out[t] = red[t];
+        return;
+    }
+    __shared__ bool s_last;
+    if (t < K) {
+        partial[blockIdx.x * K + t] = red[t];
+        __threadfence();
+    }
+    __syncthreads();
+    if (t == 0) s_last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int j = warp; j < K; j += blockDim.x >> 5) {
+        cplx s = cmk(0, 0);
+        for (int b = lane; b < (int)gridDim.x; b += 32) {
+            const double2 v = __ldcg(reinterpret_cast<const double2*>(partial) + b * K + j);
+            s = cadd(s, cmk(v.x, v.y));
+        }
+        s = warp_sum(s);
+        if (lane == 0) out[j] = s;
+    }
+}
+
+// out[j] = sum of conj(v_j[i]) * w[i]
 template <int K>
 __global__ void __launch_bounds__(256) multi_dot_kernel(PtrPack V, const cplx* __restrict__ w,
-                                                        int64_t n, cplx* __restrict__ partial) {
+                                                        int64_t n, cplx* __restrict__ partial,
+                                                        cplx* __restrict__ out, unsigned* __restrict__ count) {
     cplx acc[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) acc[j] = cmk(0, 0);
@@ -311,16 +420,19 @@ __global__ void __launch_bounds__(256) multi_dot_kernel(PtrPack V, const cplx* _
         if (lane == 0) red[warp][j] = s;
     }
     __syncthreads();
+    __shared__ cplx sum[K];
     if (threadIdx.x < K) {
         cplx s = cmk(0, 0);
         for (int wp = 0; wp < (int)(blockDim.x >> 5); ++wp) s = cadd(s, red[wp][threadIdx.x]);
-        partial[blockIdx.x * K + threadIdx.x] = s;
+        sum[threadIdx.x] = s;
     }
+    last_block_sum(sum, K, partial, out, count);
 }
 
 __global__ void __launch_bounds__(256) bilinear_dot_kernel(const cplx* __restrict__ x,
                                                            const cplx* __restrict__ y, int64_t n,
-                                                           cplx* __restrict__ partial) {
+                                                           cplx* __restrict__ partial, cplx* __restrict__ out,
+                                                           unsigned* __restrict__ count) {
     cplx acc = cmk(0, 0);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -330,21 +442,13 @@ __global__ void __launch_bounds__(256) bilinear_dot_kernel(const cplx* __restric
     acc = warp_sum(acc);
     if (lane == 0) red[warp] = acc;
     __syncthreads();
+    __shared__ cplx sum;
     if (threadIdx.x == 0) {
         cplx s = cmk(0, 0);
         for (int wp = 0; wp < (int)(blockDim.x >> 5); ++wp) s = cadd(s, red[wp]);
-        partial[blockIdx.x] = s;
+        sum = s;
     }
-}
-
-__global__ void reduce_partials_kernel(const cplx* __restrict__ partial, int nblk, int K,
-                                       cplx* __restrict__ out) {
-    // one warp per output, fixed order -> deterministic
-    const int j = blockIdx.x;
-    cplx s = cmk(0, 0);
-    for (int b = threadIdx.x; b < nblk; b += 32) s = cadd(s, partial[b * K + j]);
-    s = warp_sum(s);
-    if (threadIdx.x == 0) out[j] = s;
+    last_block_sum(&sum, 1, partial, out, count);
 }
 
 template <int K>
@@ -359,6 +463,153 @@ __global__ void multi_axpy_kernel(cplx* __restrict__ w, PtrPack V, const cplx* _
 #pragma unroll
         for (int j = 0; j < K; ++j) acc = cfma(c[j], V.p[j][i], acc);
         w[i] = acc;
+    }
+}
+
+// ---- one Lanczos step's orthogonalisation ------------------------------------
+// w <- w minus its components along v_0 .. v_{K-1}, twice (classical Gram-Schmidt);
+// w <- w / |w|.  coef: the K components of either pass, |w|^2 and a mark that the
+// kernel ran to its end.  One cooperative grid in place of nine launches and a host
+// round trip: a thread keeps to its entries of w, so only the K + K + 1 sums cross
+// blocks, in fixed order, at a barrier each (1.2 us).  On average over a DMRG run at
+// bond dimension 64 (vectors up to 16,384, K up to 8): 47 us of kernels and nine
+// gaps -> 17.6 us.  FP64 bounds long vectors (16 K instructions an entry), as before.
+constexpr int LMAX = 49, LG = 8;
+struct LanczosArgs {
+    const cplx* v[LMAX];
+    cplx *w, *partial, *coef;  // partial: gridDim.x x (2 K + 1)
+    int64_t n;
+    int K;
+    double mark;
+    unsigned *bar, *exits;  // zero at launch and after
+    int* err;
+};
+
+// Sums over a warp of LG complex values: halves change lanes, so that 16 additions
+// do for 16 sums (64 clocks each; five a sum otherwise).  Lane 2 r gets value r of
+// (re_0, im_0, re_1, ...).
+__device__ __forceinline__ double warp_sums(const cplx* acc) {
+    const int lane = threadIdx.x & 31;
+    double v[2 * LG];
+#pragma unroll
+    for (int j = 0; j < LG; ++j) {
+        v[2 * j] = acc[j].x;
+        v[2 * j + 1] = acc[j].y;
+    }
+#pragma unroll
+    for (int h = LG, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const double give = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+__global__ void __launch_bounds__(512) lanczos_orth_kernel(LanczosArgs p) {
+    __shared__ double red[16][2 * LG];
+    __shared__ cplx c[LMAX];
+    const int nw = blockDim.x >> 5, t = threadIdx.x, lane = t & 31, warp = t >> 5, C = gridDim.x, K = p.K;
+    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + t, di = (int64_t)C * blockDim.x;
+    unsigned arrivals = 0;
+    // this block's sum of nv values a thread to slot s of the partials
+    auto put = [&](const cplx* acc, int nv, int s) {
+        const double v = warp_sums(acc);
+        if (!(lane & 1)) red[warp][lane >> 1] = v;
+        __syncthreads();
+        if (t < 2 * nv) {
+            double u = red[0][t];
+            for (int k = 1; k < nw; ++k) u += red[k][t];
+            reinterpret_cast<double*>(p.partial)[2 * ((int64_t)blockIdx.x * (2 * LMAX + 1) + s) + t] = u;
+        }
+        __syncthreads();
+    };
+    // all blocks' partials of slots s .. s + nv - 1, to c and (block 0) to coef
+    auto gather = [&](int nv, int s) -> bool {
+        arrivals += (unsigned)C;
+        if (C > 1 && !griddev::grid_sync(p.bar, p.err, arrivals)) return false;
+        for (int j = warp; j < nv; j += nw) {
+            cplx v = cmk(0, 0);
+            for (int b = lane; b < C; b += 32) {
+                const double2 x = __ldcg(reinterpret_cast<const double2*>(p.partial) + (int64_t)b * (2 * LMAX + 1) + s + j);
+                v = cadd(v, cmk(x.x, x.y));
+            }
+            v = warp_sum(v);
+            if (lane == 0) {
+                c[j] = v;
+                if (blockIdx.x == 0) p.coef[s + j] = v;
+            }
+        }
+        __syncthreads();
+        return true;
+    };
+    // subtract the components c and, in the same pass, take the products for the next
+    // sums with the vectors of group j0 (the last group holds the finished entries)
+    for (int j0 = 0; j0 < K; j0 += LG) {
+        const int kk = min(LG, K - j0);
+        cplx acc[LG];
+#pragma unroll
+        for (int j = 0; j < LG; ++j) acc[j] = cmk(0, 0);
+        for (int64_t i = i0; i < p.n; i += di) {
+            const cplx w = p.w[i];
+#pragma unroll
+            for (int j = 0; j < LG; ++j)
+                if (j < kk) acc[j] = cfma(cconj(p.v[j0 + j][i]), w, acc[j]);
+        }
+        put(acc, kk, j0);
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        if (!gather(K, pass * LMAX)) return;
+        for (int j0 = 0; j0 < K; j0 += LG) {
+            const int kk = min(LG, K - j0);
+            const bool last = j0 + LG >= K;
+            cplx acc[LG];
+#pragma unroll
+            for (int j = 0; j < LG; ++j) acc[j] = cmk(0, 0);
+            for (int64_t i = i0; i < p.n; i += di) {
+                cplx w = p.w[i], v[LG];
+#pragma unroll
+                for (int j = 0; j < LG; ++j)
+                    if (j < kk) {
+                        v[j] = p.v[j0 + j][i];
+                        w = cfma(cmk(-c[j0 + j].x, -c[j0 + j].y), v[j], w);
+                    }
+                p.w[i] = w;
+                if (pass == 1) {
+                    if (last) acc[0].x = fma(w.x, w.x, fma(w.y, w.y, acc[0].x));
+                } else if (K <= LG) {
+#pragma unroll
+                    for (int j = 0; j < LG; ++j)
+                        if (j < kk) acc[j] = cfma(cconj(v[j]), w, acc[j]);
+                }
+            }
+            if (pass == 0 && K <= LG) put(acc, kk, LMAX);
+            if (pass == 1 && last) put(acc, 1, 2 * LMAX);
+        }
+        if (pass == 0 && K > LG)  // components of the finished w
+            for (int j0 = 0; j0 < K; j0 += LG) {
+                const int kk = min(LG, K - j0);
+                cplx acc[LG];
+#pragma unroll
+                for (int j = 0; j < LG; ++j) acc[j] = cmk(0, 0);
+                for (int64_t i = i0; i < p.n; i += di) {
+                    const cplx w = p.w[i];
+#pragma unroll
+                    for (int j = 0; j < LG; ++j)
+                        if (j < kk) acc[j] = cfma(cconj(p.v[j0 + j][i]), w, acc[j]);
+                }
+                put(acc, kk, LMAX + j0);
+            }
+    }
+    if (!gather(1, 2 * LMAX)) return;
+    const double b2 = c[0].x, s = b2 > 0.0 ? 1.0 / sqrt(b2) : 0.0;
+    for (int64_t i = i0; i < p.n; i += di) p.w[i] = cmk(p.w[i].x * s, p.w[i].y * s);
+    if (t == 0) {
+        if (blockIdx.x == 0) p.coef[2 * LMAX + 1] = cmk(p.mark, 0.0);
+        // everybody has passed the last barrier once the last block is here
+        if (atomicInc(p.exits, C - 1) == (unsigned)C - 1) *p.bar = 0;
     }
 }
 
@@ -584,6 +835,11 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
 // the per-output kernel takes 37 us; at 128^3 = 2.1 M it is 27 us against 23).
 constexpr double ZTC_MIN = 2.5e6;
 
+// Threads of a kernel of one block that scans n values: no more warps than there are
+// values for, as every FP64 instruction of every warp holds its scheduler for 64
+// clocks (the keep rule of 32 values takes 6.7 us with one warp, 13 with 32).
+inline unsigned one_block(int64_t n) { return (unsigned)std::min<int64_t>(1024, (n + 31) / 32 * 32); }
+
 inline int grid_for(Ctx* ctx, int64_t n, int threads = 256) {
     int64_t g = (n + threads - 1) / threads;
     const int64_t cap = (int64_t)ctx->sm_count * 8;
@@ -670,16 +926,26 @@ void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int
                  bool accumulate) {
     if (na <= 0 || nc <= 0) return;
     TN_REQUIRE(nI * nJ <= 4096, "small_apply: operator too large");
-    const size_t smem = sizeof(cplx) * nI * nJ;
-    // the whole operator is staged in shared memory: up to 64 KiB, above the
+    ProfScope ps(ctx, 3, 8.0 * na * nc * nI * nJ, 16.0 * na * nc * (nI + nJ));
+    if (nI <= 4) {
+        dense_apply_kernel<<<grid_for(ctx, na * nc * nJ, 128), 128, 0, ctx->stream>>>(
+            in, out, M, nI, nJ, na, nc, lda_i, ldc_i, lda_o, ldc_o, accumulate ? 1 : 0);
+        ctx->count();
+        TN_CHECK_CUDA(cudaGetLastError());
+        return;
+    }
+    const size_t smem = (sizeof(cplx) + 2) * nI * nJ + 6 * nJ;
+    // the whole operator is staged in shared memory: up to 96 KiB, above the
     // 48 KiB a launch gets without opting in
     if (smem > 48 * 1024)
-        TN_CHECK_CUDA(cudaFuncSetAttribute(small_apply_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(sizeof(cplx) * 4096)));
-    ProfScope ps(ctx, 3, 8.0 * na * nc * nI * nJ, 16.0 * na * nc * (nI + nJ));
-    small_apply_kernel<<<grid_for(ctx, na * nc), 256, smem, ctx->stream>>>(
-        in, out, M, nI, nJ, na, nc, lda_i, ldc_i, lda_o, ldc_o, accumulate ? 1 : 0);
+        TN_CHECK_CUDA(cudaFuncSetAttribute(small_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           18 * 4096 + 6 * 4096));
+    // threads to a column until two warps are on every scheduler
+    int parts = 1;
+    while (parts < nJ && na * nc * parts < (int64_t)ctx->sm_count * 256) parts *= 2;
+    parts = std::min(parts, nJ);
+    small_apply_kernel<<<grid_for(ctx, na * nc * parts, 128), 128, smem, ctx->stream>>>(
+        in, out, M, nI, nJ, na, nc, lda_i, ldc_i, lda_o, ldc_o, accumulate ? 1 : 0, parts);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
 }
@@ -693,12 +959,10 @@ void multi_dot(Ctx* ctx, const cplx* const* hV, int K, const cplx* w, int64_t n,
         PtrPack P{};
         for (int j = 0; j < kk; ++j) P.p[j] = hV[j0 + j];
         switch (kk) {
-#define TN_MD(KK) case KK: multi_dot_kernel<KK><<<nblk, 256, 0, ctx->stream>>>(P, w, n, partial); break;
+#define TN_MD(KK) case KK: multi_dot_kernel<KK><<<nblk, 256, 0, ctx->stream>>>(P, w, n, partial, dout + j0, ctx->d_bar + 3); break;
             TN_MD(1) TN_MD(2) TN_MD(3) TN_MD(4) TN_MD(5) TN_MD(6) TN_MD(7) TN_MD(8)
 #undef TN_MD
         }
-        ctx->count();
-        reduce_partials_kernel<<<kk, 32, 0, ctx->stream>>>(partial, nblk, kk, dout + j0);
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
@@ -707,9 +971,7 @@ void multi_dot(Ctx* ctx, const cplx* const* hV, int K, const cplx* w, int64_t n,
 void bilinear_dot(Ctx* ctx, const cplx* x, const cplx* y, int64_t n, cplx* dout) {
     const int nblk = grid_for(ctx, n);
     cplx* partial = ctx->s_dot.c(ctx, (size_t)nblk * MAXV);
-    bilinear_dot_kernel<<<nblk, 256, 0, ctx->stream>>>(x, y, n, partial);
-    ctx->count();
-    reduce_partials_kernel<<<1, 32, 0, ctx->stream>>>(partial, nblk, 1, dout);
+    bilinear_dot_kernel<<<nblk, 256, 0, ctx->stream>>>(x, y, n, partial, dout, ctx->d_bar + 3);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
 }
@@ -730,6 +992,43 @@ void multi_axpy(Ctx* ctx, cplx* w, const cplx* const* hV, const cplx* dcoef, int
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
+}
+
+// The components of both passes (c1[j] + c2[j] to comp[j]) and |w| of the result, w
+// divided by it; one host synchronisation.
+double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, cplx* comp) {
+    TN_REQUIRE(K >= 1 && K <= LMAX, "lanczos_orth: too many vectors");
+    ProfScope ps(ctx, 6, 32.0 * n * K, 16.0 * n * (3 * K + 5));
+    LanczosArgs a{};
+    for (int j = 0; j < K; ++j) a.v[j] = hV[j];
+    // one warp on every scheduler keeps the FP64 units busy and has the fewest sums;
+    // vectors beyond L2 want more loads in flight
+    const int threads = n <= (1 << 20) ? 128 : 512;
+    const int C = (int)std::min<int64_t>(ctx->sm_count, (n + threads - 1) / threads);
+    // coefficients and mark, then the partials
+    a.coef = ctx->s_dot.c(ctx, (size_t)(2 * LMAX + 2) + (size_t)C * (2 * LMAX + 1));
+    a.partial = a.coef + 2 * LMAX + 2;
+    a.w = w;
+    a.n = n;
+    a.K = K;
+    a.mark = (double)++ctx->lanczos_calls;
+    a.bar = ctx->d_bar + 4;
+    a.exits = ctx->d_bar + 5;
+    a.err = reinterpret_cast<int*>(ctx->d_bar + 6);
+    void* args[] = {&a};
+    TN_CHECK_CUDA(cudaLaunchCooperativeKernel((void*)lanczos_orth_kernel, dim3((unsigned)C), dim3(threads), args, 0,
+                                              ctx->stream));
+    ctx->count();
+    double* h = ctx->pinned(2 * (2 * LMAX + 2));
+    TN_CHECK_CUDA(cudaMemcpyAsync(h, a.coef, sizeof(cplx) * (2 * LMAX + 2), cudaMemcpyDeviceToHost, ctx->stream));
+    ctx->sync();
+    if (h[2 * (2 * LMAX + 1)] != a.mark) {
+        TN_CHECK_CUDA(cudaMemsetAsync(ctx->d_bar + 4, 0, 3 * sizeof(unsigned), ctx->stream));
+        throw Error(TN_ERR_TIMEOUT, "Lanczos: a bounded grid barrier ran out");
+    }
+    for (int j = 0; j < K; ++j)
+        comp[j] = cmk(h[2 * j] + h[2 * (LMAX + j)], h[2 * j + 1] + h[2 * (LMAX + j) + 1]);
+    return std::sqrt(h[4 * LMAX]);
 }
 
 void zaxpy(Ctx* ctx, cplx* y, const cplx* x, int64_t n, cplx a) {
@@ -786,7 +1085,7 @@ void take_top_eigvecs(Ctx* ctx, const cplx* G, int64_t n, int64_t k, cplx* dst, 
 }
 
 void gram_trace(Ctx* ctx, const cplx* G, int64_t n, double* dout) {
-    gram_trace_kernel<<<1, 1024, 0, ctx->stream>>>(G, n, dout);
+    gram_trace_kernel<<<1, one_block(n), 0, ctx->stream>>>(G, n, dout);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
 }
@@ -833,7 +1132,7 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
                      const int* dinfo) {
     TN_REQUIRE(sz <= n, "keep_rule: more singular values than eigenvalues");
     KeepDev* dres = static_cast<KeepDev*>(ctx->s_coef.get(ctx, 256));
-    keep_rule_kernel<<<1, 1024, 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, dtotal,
+    keep_rule_kernel<<<1, one_block(sz), 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, dtotal,
                                                   dinfo, ctx->d_err, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());

@@ -71,8 +71,8 @@ void ctx_init(Ctx& c, int device) {
     uint64_t thr = UINT64_MAX;  // keep freed blocks cached in the pool
     TN_CHECK_CUDA(cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &thr));
     TN_CHECK_CUDA(cudaMalloc(&c.d_info, sizeof(int)));
-    TN_CHECK_CUDA(cudaMalloc(&c.d_bar, 4 * sizeof(unsigned)));
-    TN_CHECK_CUDA(cudaMemset(c.d_bar, 0, 4 * sizeof(unsigned)));
+    TN_CHECK_CUDA(cudaMalloc(&c.d_bar, 8 * sizeof(unsigned)));
+    TN_CHECK_CUDA(cudaMemset(c.d_bar, 0, 8 * sizeof(unsigned)));
     TN_CHECK_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
     TN_CHECK_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
     TN_CHECK_CUDA(cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device));
