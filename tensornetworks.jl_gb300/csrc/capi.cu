@@ -420,22 +420,19 @@ int32_t tn_inner_terms(tn_ctx* h, const tn_mps* bra, const tn_mps* ket, int32_t 
     Ctx* ctx = &h->c;
     const int d = ket->d;
     std::vector<Term> terms(nterms);
-    std::vector<DBuf> mats;
-    size_t off = 0;
+    size_t nops = 0;
     for (int t = 0; t < nterms; ++t) {
         terms[t].first = term_first[t];
         terms[t].len = term_len[t];
         TN_REQUIRE(term_len[t] >= 1, "term length must be positive");
         terms[t].coeff = cmk(coeffs[2 * t], coeffs[2 * t + 1]);
-        for (int j = 0; j < term_len[t]; ++j) {
-            mats.emplace_back();
-            upload_op_matrix(ctx, term_ops + off, d, mats.back());
-            off += 2 * (size_t)d * d;
-        }
+        nops += term_len[t];
     }
+    DBuf mats;
+    const std::vector<const cplx*> ops = upload_op_matrices(ctx, term_ops, nops, d, mats);
     size_t mi = 0;
     for (int t = 0; t < nterms; ++t)
-        for (int j = 0; j < term_len[t]; ++j) terms[t].dops.push_back(mats[mi++].c());
+        for (int j = 0; j < term_len[t]; ++j) terms[t].dops.push_back(ops[mi++]);
     std::vector<cplx> v = inner_terms(ctx, bra, ket, terms);
     for (int t = 0; t < nterms; ++t) {
         out[2 * t] = v[t].x;

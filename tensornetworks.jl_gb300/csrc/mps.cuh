@@ -113,6 +113,8 @@ double tebd_grad(const tn_mps* psi0, const std::vector<const tn_gates*>& gls,
 
 // small_apply matrix of a d x d operator acting on the physical leg
 void upload_op_matrix(Ctx* ctx, const double* op_interleaved, int d, DBuf& out);
+// n operators at once, to out; their places there
+std::vector<const cplx*> upload_op_matrices(Ctx* ctx, const double* ops, size_t n, int d, DBuf& out);
 void apply_site_op(tn_mps* psi, int site, const cplx* M);
 
 }  // namespace tn
