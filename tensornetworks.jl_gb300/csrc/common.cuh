@@ -205,8 +205,6 @@ double znorm2(Ctx* ctx, const cplx* x, int64_t n);  // ||x||^2, synchronous
 // ncols = n, a full ascending eigenvector matrix)
 void take_top_eigvecs(Ctx* ctx, const cplx* G, int64_t n, int64_t k, cplx* dst,
                       int64_t ncols = -1);
-// *dout = sum of the real diagonal of the n x n matrix G (device)
-void gram_trace(Ctx* ctx, const cplx* G, int64_t n, double* dout);
 // scale columns: X[:, j] *= s[j] (s real, device)
 // dst (c x r) = src(r x c)^H, tiled through shared memory for coalescing
 void conj_transpose(Ctx* ctx, const cplx* src, int64_t r, int64_t c, cplx* dst);
@@ -219,15 +217,14 @@ void scale_rows(Ctx* ctx, cplx* X, int64_t k, int64_t n, const double* s, int in
 // Keep rule of tensors.jl:200-215 on ascending eigenvalues lam[0..n) of a Gram
 // matrix whose top sz values are the squared singular values.  Writes
 // (k, total, discarded) to host.  Also writes kept singular values (descending)
-// into dS when non-null.  With dtotal (device, the Gram trace) the n values
-// are only the top of the spectrum: the weight below them is the trace minus
-// their sum.
+// into dS when non-null.  With the g x g Gram matrix G the n values are only the
+// top of its spectrum: the weight below them is the trace minus their sum.
 struct KeepResult { int64_t k; double total; double discarded; };
 // dinfo (device, optional): an eigensolver status read back in the same
 // synchronisation with the tensor-core wait status; nonzero raises
 // TN_ERR_TIMEOUT.
 KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double cutoff,
-                     int64_t maxdim, int64_t mindim, double* dS, const double* dtotal = nullptr,
+                     int64_t maxdim, int64_t mindim, double* dS, const cplx* G = nullptr, int64_t g = 0,
                      const int* dinfo = nullptr);
 
 // ---- linear algebra (linalg.cu) ----------------------------------------
@@ -239,15 +236,15 @@ struct SplitResult { int64_t k; double discarded; double total; };
 SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, double cutoff,
                         int64_t maxdim, int64_t mindim, bool left_iso, DBuf& X, DBuf& Y,
                         std::vector<double>* S);
-// Top `want` eigenpairs of the Hermitian n x n matrix G (lower triangle read,
-// G destroyed), hand-written FP64 kernels (eig.cu): lam_asc[want-1-g] is the
+// Top `want` eigenpairs of the Hermitian n x n matrix G (lower triangle read;
+// hand-written kernels, eig.cu): lam_asc[want-1-g] is the
 // g-th largest eigenvalue and X[:, g] (n x want) its eigenvector.  No host
 // synchronisation; a timed-out grid barrier leaves ctx->d_bar[2] nonzero.
 // psd: G is positive semidefinite (a Gram matrix).
-void eig_top(Ctx* ctx, cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X, bool psd);
+void eig_top(Ctx* ctx, const cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X, bool psd);
 // Householder tridiagonalisation (hetrd.cu): T in (d, e), reflector j in column j
-// of G (rows j+1.., explicit first entry, zeros above), H_j = I - tau_j v_j v_j^H.
-void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool psd, int* perm);
+// of V (rows j+1.., explicit first entry), H_j = I - tau_j v_j v_j^H.
+void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, cplx* V, bool psd, int* perm);
 // Top `want` eigenpairs of the real symmetric tridiagonal (d, e) (dc.cu): lam_asc
 // ascending, Z (n x want) in descending order.
 void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t want,

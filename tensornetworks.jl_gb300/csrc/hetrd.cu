@@ -26,8 +26,9 @@
 // 128 from 699 to 576, 256 from 2,069 to 1,873, 512 from 6,574 to 4,437, 2048 from
 // 98 to 61 ms.
 //
-// Reflector j is kept as V[j n + i] (i > j; integers of unit 2^-56 with the
-// first entry explicit) and tau[j]: H_j = I - tau_j v_j v_j^H.
+// Reflector j is kept as V[j n + i] (i > j, the first entry explicit) and tau[j]:
+// H_j = I - tau_j v_j v_j^H.  Results become FP64 while the exchange travels, or by
+// the scalar warp while it waits: a launch of their own took 4.7 us.
 #include <climits>
 #include <cmath>
 
@@ -50,13 +51,10 @@ constexpr int HPAD = 64;  // zeros after the vectors: rows run in steps of 64 en
 enum Form { CLUSTER, GRID_SHARED, GRID_GLOBAL };
 
 struct TrdOut {
-    zint* V;      // n x n, column j: reflector j
-    cplx* tau;    // n
-    ll* di;       // n: diagonal, unit 2^(f - 61 - dsh)
-    ll* ei;       // n: off-diagonal, unit 2^(f - 61 - esh)
-    int *dsh, *esh;  // n
-    int* f;       // exponent of the scale, or INT_MIN: the matrix is not finite
-    int* perm;    // n: row of G that became row l, when psd
+    cplx* V;         // n x n, column j: reflector j
+    cplx* tau;       // n
+    double *d, *e;   // n: the tridiagonal
+    int* perm;       // n: row of G that became row l, when psd
 };
 
 struct TrdIn {
@@ -137,6 +135,8 @@ struct ShCtl {
     int em, c;           // smallest exponent of the rows left, the column's exponent
     zint alpha;          // first entry of the column before the shift
     ll beta;
+    ll dint;  // diagonal entry just formed, in units of 2^(f - 61 - dexp)
+    int dexp;
     zint v1, tau;
     ll c2;
     unsigned part[2 * HC];  // scale partials of the cluster's blocks
@@ -156,6 +156,9 @@ __device__ __forceinline__ ll to_fix(double x, int s) {
     const ll r = sft(m, ex - 1075 + s);
     return b < 0 ? -r : r;
 }
+
+// x 2^-56 as FP64, |x| < 2^62
+__device__ __forceinline__ double unit56(ll x) { return scale2(__ll2double_rn(x), -56); }
 
 template <int FORM, int RW>
 __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
@@ -237,7 +240,15 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
     hmax = 0;
     for (int i = 0; i < C; ++i) hmax = max(hmax, shared_part(0, i));
     if (hmax >= 0x7ff00000u) {  // an infinity or NaN: no block goes on
-        if (b == 0 && tid == 0) *p.o.f = INT_MIN;
+        if (b == 0) {
+            const double nan = __longlong_as_double(0x7ff8000000000000ll);
+            for (int i = tid; i < n; i += HT) {
+                p.o.d[i] = p.o.e[i] = nan;
+                p.o.tau[i] = cmk(0, 0);
+                if (p.psd) p.o.perm[i] = i;
+            }
+            for (int64_t i = tid; i < (int64_t)n * n; i += HT) p.o.V[i] = cmk(0, 0);
+        }
         if (!GRID) cluster_sync();  // no block leaves while others read its memory
         return;
     }
@@ -263,7 +274,6 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
     int fe;
     frexpf(sum * 1.01f, &fe);
     const int f = max(emax, -1000) + (fe + 1) / 2;
-    if (b == 0 && tid == 0) *p.o.f = f;
 
     // ---- order, exponents, this block's rows as integers --------------------------
     // Rows of a graded matrix go by descending diagonal: eliminated in that order,
@@ -337,10 +347,8 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
         for (int l = tid; l < n; l += HM) {
             const cplx v = entry(l, 0);
             if (l == 0) {
-                if (b == 0) {
-                    p.o.di[0] = to_fix(v.x, 61 - f + 2 * c);
-                    p.o.dsh[0] = 2 * c;
-                }
+                sh.dint = to_fix(v.x, 61 - f + 2 * c);
+                sh.dexp = 2 * c;
                 continue;
             }
             const int s = 61 - f + ee[l] + c;
@@ -348,6 +356,8 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
         }
         add_norm(S, 0);
     }
+    // an integer of unit 2^(f - 61 - s) as FP64
+    auto unfix = [&](ll x, int s) { return scalbn(__ll2double_rn(x), f - 61 - s); };
     __syncthreads();
     for (int l = tid; l < 3 * (n + HPAD); l += HT) vD[l] = make_int4(0, 0, 0, 0);  // vU and wU too
     for (int j = 0; j + 1 < n; ++j) {
@@ -369,7 +379,9 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
         if (warp == RW) {
             // beta and v's first entry for the row warps, then tau and c2 while
             // the rows' results travel
-            double ar = 0.0, ai = 0.0, be = 0.0, sq = 0.0;
+            double ar = 0.0, ai = 0.0, be = 0.0, sq = 0.0, tr = 0.0, ti = 0.0;
+            const ll dint = sh.dint;
+            const int dexp = sh.dexp;
             if (lane == 0) {
                 ll beta = 0;
                 zint al{0, 0};
@@ -397,7 +409,6 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             if (lane == 0) {
                 zint tau{0, 0};
                 ll c2 = 0;
-                double tr = 0.0, ti = 0.0;
                 if (bl) {
                     // |beta - alpha|^2 = s + |alpha|^2 + 2 |beta alpha_r| (no cancellation)
                     const double D = fma(ar, ar, fma(ai, ai, fma(-(be + be), ar, sq)));
@@ -409,14 +420,19 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
                 }
                 sh.tau = tau;
                 sh.c2 = c2;
-                if (b == 0) {
-                    p.o.tau[j] = cmk(tr, ti);
-                    p.o.ei[j] = sh.beta;
-                    p.o.esh[j] = shf + em + c;
-                }
-                if (b == l0 % C) p.o.V[(size_t)j * n + l0] = sh.v1;
             }
             __syncwarp();
+            bar_named(3, HT);  // the exchange; tau and c2
+            if (lane == 0) {
+                if (b == 0) {
+                    p.o.tau[j] = cmk(tr, ti);
+                    p.o.d[j] = unfix(dint, dexp);
+                    p.o.e[j] = unfix(sh.beta, shf + em + c);
+                }
+                if (b == l0 % C)
+                    p.o.V[(size_t)j * n + l0] = cmk(unit56(sh.v1.x), unit56(sh.v1.y));
+            }
+            if (sh.abort) break;
         } else {
             // column -> v's limbs for the products (the first entry still alpha)
             for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em)));
@@ -515,7 +531,10 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             for (int l = l0 + tid; l < n; l += HM) {
                 const int d = ee[l] - em;
                 const zint x = xr[l];
-                if (l > l0 && l % C == b) p.o.V[(size_t)j * n + l] = zsft(x, shf - d);
+                if (l > l0 && l % C == b) {
+                    const zint v = zsft(x, shf - d);
+                    p.o.V[(size_t)j * n + l] = cmk(unit56(v.x), unit56(v.y));
+                }
                 vm = max(vm, max(bits64(x.x), bits64(x.y)) + shf - 2 * d - 56);
             }
             vm = __reduce_max_sync(0xffffffffu, vm);
@@ -529,11 +548,11 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             } else if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) {
                 sh.abort = 1;
             }
-        }
-        bar_named(3, HT);  // the exchange; tau and c2
-        if (sh.abort) {
-            if (tid == 0) atomicExch(p.err, 1);
-            break;
+            bar_named(3, HT);  // the exchange; tau and c2
+            if (sh.abort) {
+                if (tid == 0) atomicExch(p.err, 1);
+                break;
+            }
         }
         // ---- B. w, column j+1, its norm ----------------------------------------
         if (warp < RW) {
@@ -599,9 +618,9 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
                 update(x, wU[l], vU[l], w1, v1);
                 if (l > l0) {
                     emit(l, l0 + 1, x, ee[l], emn, S2);
-                } else if (b == 0) {
-                    p.o.di[l0] = x.x;
-                    p.o.dsh[l0] = 2 * cn;
+                } else {
+                    sh.dint = x.x;
+                    sh.dexp = 2 * cn;
                 }
             }
             if (l0 + 32 * warp < n) add_norm(S2, nb);
@@ -615,31 +634,12 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             }
         }
     }
-    if (!GRID) cluster_sync();  // no block leaves while its shared memory is written
-}
-
-// d, e and the reflectors as FP64: column j of G becomes reflector j (zeros down
-// to the diagonal, the first entry explicit).
-__global__ void __launch_bounds__(256) hetrd_finish_kernel(TrdOut o, int n, cplx* __restrict__ G,
-                                                           double* __restrict__ d,
-                                                           double* __restrict__ e) {
-    const int f = *o.f;
-    const bool bad = f == INT_MIN;
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n * n;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int j = (int)(t / n), i = (int)(t % n);
-        cplx g = cmk(0, 0);
-        if (i > j && !bad) {
-            const zint v = o.V[t];
-            g = cmk(__ll2double_rn(v.x) * 0x1p-56, __ll2double_rn(v.y) * 0x1p-56);
-        } else if (i == j) {
-            d[j] = bad ? nan : scalbn(__ll2double_rn(o.di[j]), f - 61 - o.dsh[j]);
-            if (j + 1 < n) e[j] = bad ? nan : scalbn(__ll2double_rn(o.ei[j]), f - 61 - o.esh[j]);
-            if (bad || j + 1 == n) o.tau[j] = cmk(0, 0);
-        }
-        G[t] = g;
+    __syncthreads();
+    if (b == 0 && tid == 0) {
+        p.o.d[n - 1] = unfix(sh.dint, sh.dexp);
+        p.o.tau[n - 1] = cmk(0, 0);
     }
+    if (!GRID) cluster_sync();  // no block leaves while its shared memory is written
 }
 
 size_t hetrd_smem(Form form, int64_t n, int64_t C) {
@@ -699,10 +699,10 @@ int clusters_fit() {
 }  // namespace
 
 // G (n x n Hermitian, lower triangle read) -> T (d, e) and the reflectors: column
-// j of G is v_j (rows j+1.., zeros above), tau[j] its scalar.  psd: G is positive
-// semidefinite and keeps graded accuracy, its row perm[l] as row l of Q.  No host
-// synchronisation; a grid barrier that ran out leaves ctx->d_bar[2] nonzero.
-void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool psd, int* perm) {
+// j of V is v_j in rows j+1.. (rows above are not written), tau[j] its scalar.  psd: G
+// is positive semidefinite and keeps graded accuracy, its row perm[l] as row l of Q.
+// No host synchronisation; a grid barrier that ran out leaves ctx->d_bar[2] nonzero.
+void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, cplx* V, bool psd, int* perm) {
     if (ctx->trd_clusters < 0) ctx->trd_clusters = clusters_fit();
     // Blocks of the cluster: the row work of a step (n^2 / 3 entries on average at
     // 180 clocks per 32) against the exchange with more blocks.  The grid's barrier
@@ -715,11 +715,10 @@ void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool p
     const bool rows_global = grid && hetrd_smem(GRID_SHARED, n, C) > HSMEM;
     auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t nn = r256(sizeof(zint) * (size_t)n * n), n8 = r256(sizeof(ll) * n),
-                 n4 = r256(sizeof(int) * n), nz = r256(sizeof(zint) * 2 * n);
+                 nz = r256(sizeof(zint) * 2 * n);
     const size_t nx = r256(sizeof(zint) * (size_t)n * C);
-    const size_t total = nn + 2 * n8 + 2 * n4 + 512 + (rows_global ? nn + nx : 0) +
-                         (grid ? 256 + 2 * nz + 2 * n8 + r256(2 * 4 * C) : 0);
-    char* base = static_cast<char*>(ctx->s_trd.get(ctx, total));
+    const size_t total = (rows_global ? nn + nx : 0) + (grid ? 256 + 2 * nz + 2 * n8 + r256(2 * 4 * C) : 0);
+    char* base = total ? static_cast<char*>(ctx->s_trd.get(ctx, total)) : nullptr;
     auto take = [&](size_t b) {
         char* q = base;
         base += b;
@@ -729,12 +728,9 @@ void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool p
     a.G = G;
     a.n = (int)n;
     a.psd = psd ? 1 : 0;
-    a.o.V = reinterpret_cast<zint*>(take(nn));
-    a.o.di = reinterpret_cast<ll*>(take(n8));
-    a.o.ei = reinterpret_cast<ll*>(take(n8));
-    a.o.esh = reinterpret_cast<int*>(take(n4));
-    a.o.dsh = reinterpret_cast<int*>(take(n4));
-    a.o.f = reinterpret_cast<int*>(take(256));
+    a.o.V = V;
+    a.o.d = d;
+    a.o.e = e;
     a.o.tau = tau;
     a.o.perm = perm;
     a.err = reinterpret_cast<int*>(ctx->d_bar + 2);
@@ -757,9 +753,6 @@ void hetrd(Ctx* ctx, cplx* G, int64_t n, double* d, double* e, cplx* tau, bool p
     } else {
         launch<CLUSTER, 16>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
     }
-    ctx->count();
-    const int64_t blocks = std::min<int64_t>((n * n + 255) / 256, (int64_t)ctx->sm_count * 8);
-    hetrd_finish_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(a.o, (int)n, G, d, e);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
 }

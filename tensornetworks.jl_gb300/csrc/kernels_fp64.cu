@@ -648,23 +648,6 @@ __global__ void top_eigvecs_kernel(const cplx* __restrict__ G, int64_t n, int64_
     }
 }
 
-// *out = sum_i Re G[i, i] (one block)
-__global__ void __launch_bounds__(1024) gram_trace_kernel(const cplx* __restrict__ G, int64_t n,
-                                                          double* __restrict__ out) {
-    __shared__ double ws[32];
-    double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += G[i + n * i].x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-        *out = t;
-    }
-}
-
 __global__ void scale_cols_kernel(cplx* X, int64_t m, int64_t k, const double* s, int invert) {
     const int64_t total = m * k;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -747,7 +730,7 @@ __device__ inline double s2_at(const double* lam, int64_t n, int64_t i) {
 __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restrict__ lam, int64_t n,
                                                          int64_t sz, double cutoff, int64_t maxdim,
                                                          int64_t mindim, double* __restrict__ S_out,
-                                                         const double* __restrict__ dtotal,
+                                                         const cplx* __restrict__ G, int64_t g,
                                                          const int* __restrict__ dinfo,
                                                          const int* __restrict__ derr,
                                                          KeepDev* __restrict__ res) {
@@ -758,6 +741,15 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
     const int nw = T >> 5;
     const int64_t per = (sz + T - 1) / T;
     const int64_t lo = min((int64_t)t * per, sz), hi = min(lo + per, sz);
+    // the whole spectrum's weight: the trace of the Gram matrix
+    __shared__ double wtr[32];
+    if (G) {
+        double tr = 0.0;
+        for (int64_t i = t; i < g; i += T) tr += G[i + g * i].x;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) tr += __shfl_down_sync(0xffffffffu, tr, o);
+        if (lane == 0) wtr[warp] = tr;
+    }
     double local = 0.0;
     for (int64_t i = hi - 1; i >= lo; --i) local += s2_at(lam, n, i);
     // inclusive suffix scan over threads: incl(t) = sum_{t' >= t} local(t')
@@ -778,7 +770,9 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
         }
         // partial spectrum: the weight below the available values is the
         // trace minus their sum
-        const double rest = dtotal ? fmax(*dtotal - acc, 0.0) : 0.0;
+        double tr = 0.0;
+        for (int w = 0; G && w < nw; ++w) tr += wtr[w];
+        const double rest = G ? fmax(tr - acc, 0.0) : 0.0;
         s_rest = rest;
         s_total = acc + rest;
     }
@@ -1084,12 +1078,6 @@ void take_top_eigvecs(Ctx* ctx, const cplx* G, int64_t n, int64_t k, cplx* dst, 
     TN_CHECK_CUDA(cudaGetLastError());
 }
 
-void gram_trace(Ctx* ctx, const cplx* G, int64_t n, double* dout) {
-    gram_trace_kernel<<<1, one_block(n), 0, ctx->stream>>>(G, n, dout);
-    ctx->count();
-    TN_CHECK_CUDA(cudaGetLastError());
-}
-
 void conj_transpose(Ctx* ctx, const cplx* src, int64_t r, int64_t c, cplx* dst) {
     if (r <= 0 || c <= 0) return;
     TN_REQUIRE((c + 31) / 32 <= 65535, "conj_transpose: too many columns");
@@ -1128,11 +1116,11 @@ void scale_rows(Ctx* ctx, cplx* X, int64_t k, int64_t n, const double* s, int in
 }
 
 KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double cutoff,
-                     int64_t maxdim, int64_t mindim, double* dS, const double* dtotal,
+                     int64_t maxdim, int64_t mindim, double* dS, const cplx* G, int64_t g,
                      const int* dinfo) {
     TN_REQUIRE(sz <= n, "keep_rule: more singular values than eigenvalues");
     KeepDev* dres = static_cast<KeepDev*>(ctx->s_coef.get(ctx, 256));
-    keep_rule_kernel<<<1, one_block(sz), 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, dtotal,
+    keep_rule_kernel<<<1, one_block(sz), 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
                                                   dinfo, ctx->d_err, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());

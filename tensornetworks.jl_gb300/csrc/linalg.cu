@@ -161,14 +161,13 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
     // eigenpairs the keep rule can select: max(maxdim, mindim), at most sz
     const int64_t maxd = (maxdim <= 0 || maxdim > sz) ? sz : maxdim;
     const int64_t want = std::min(sz, std::max(maxd, mindim));
-    double* lam = ctx->s_eigval.d(ctx, (size_t)want + sz + 2);
+    double* lam = ctx->s_eigval.d(ctx, (size_t)want + sz);
     double* dS = lam + want;
-    double* dtotal = lam + want + sz;  // the trace gives the weight below the computed values
-    gram_trace(ctx, G, g, dtotal);
     cplx* V = ctx->s_x.c(ctx, (size_t)g * want);  // top eigenvectors, descending
     eig_top(ctx, G, g, want, lam, V, true);
-    // the eigensolver's barrier status is read back with the keep-rule result
-    KeepResult kr = keep_rule(ctx, lam, want, want, cutoff, maxdim, mindim, dS, dtotal,
+    // G's trace gives the weight below the computed values; the eigensolver's barrier
+    // status is read back with the keep-rule result
+    KeepResult kr = keep_rule(ctx, lam, want, want, cutoff, maxdim, mindim, dS, G, g,
                               reinterpret_cast<const int*>(ctx->d_bar + 2));
     const int64_t k = kr.k;
     TN_REQUIRE(k <= want, "trunc_split: keep rule selected more vectors than computed");

@@ -1,7 +1,7 @@
 """The Hermitian eigensolver at the edges of its forms: cluster sizes 1, 4, 8
-and 16 of the reduction (orders 16, 32, 64 and 405), the divide and conquer's
+and 16 of the reduction (orders 16, 32, 64 and 288), the divide and conquer's
 levels (powers of two) and its two forms (128), the panel widths of the
-back-transformation (64, 128).
+back-transformation (64, 128) and its form for small orders (32, 48).
 
 tn_eigh_top is checked on indefinite, rank-deficient, diagonal and zero-padded
 matrices: residual and orthogonality are within 64 n 2^-52, a backward error of
@@ -18,7 +18,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 EPS = 2.0 ** -52
-SIZES = [1, 2, 3, 5, 8, 9, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 192, 193, 256, 257, 405, 406]
+SIZES = [1, 2, 3, 5, 8, 9, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 127, 128, 129, 192, 193, 256, 257, 405, 406]
 
 
 def dp(a):
