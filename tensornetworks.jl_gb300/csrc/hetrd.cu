@@ -2,7 +2,7 @@
 // G = Q T Q^H, in fixed point (fixp.cuh): step 1 of the eigensolver (eig.cu).
 //
 // One thread-block cluster holds the whole matrix in its shared memories up to
-// order 288; above, the blocks of a cooperative grid do, and from about order 1100
+// order 208; above, the blocks of a cooperative grid do, and from about order 1100
 // the rows stay in global memory (L2).  Row i belongs to block i mod C.  Step j:
 //   A. a warp per row applies the pending rank-2 update of step j-1 to the
 //      row and sums its product with v, in one pass, while a further warp forms
@@ -15,16 +15,17 @@
 // barrier, five block sums of ten dependent 64-clock additions each and a serial
 // square root and two divisions (2,000 clocks).
 //
-// Up to order 200 a step is a chain of dependent integer instructions (7,700
-// clocks at order 64: limbs of v 720, rows 2,050 with their sums, exchange 1,760,
-// w 1,850, column and norm 1,380); rows take over above (order 256: 6,800 of
-// 16,000 clocks) and their traffic through L2 at order 2048 (41,000 of 62,000).
-// A thread per entry (16 row warps in the larger forms), rows two entries deep with
-// the next two loaded ahead, the products of w by 32-bit limbs, the new exponent of
-// row j+1 from the last step's smallest exponent (so that w needs one pass) and
-// work that nobody waits for behind the exchange took order 64 from 308 to 257 us,
-// 128 from 699 to 576, 256 from 2,069 to 1,873, 512 from 6,574 to 4,437, 2048 from
-// 98 to 61 ms.
+// In a cluster a step is a chain of dependent integer instructions (7,900 clocks at
+// order 64: limbs of v 780, rows 2,200 with their sums, exchange 1,550, w 1,900,
+// column and norm 1,150); the grid adds its barrier and vectors through L2, and at
+// order 2048 the rows' integer multiplications and their traffic through L2 take
+// 38,000 of 60,000 clocks.  Against the first version (8 row warps, one entry a lane
+// at a time, w in two passes): rows two entries deep with the next two loaded ahead,
+// 16 row warps and rows shared by warps in the grid forms, the products of w by
+// 32-bit limbs, the new exponent of row j+1 from the last step's smallest exponent
+// (so that w needs one pass) and work that nobody waits for behind the exchange took
+// order 64 from 308 to 245 us, 128 from 699 to 571, 256 from 2,069 to 1,646, 512
+// from 6,574 to 3,830, 1024 from 21.3 to 12.0 ms, 2048 from 98 to 58 ms.
 //
 // Reflector j is kept as V[j n + i] (i > j, the first entry explicit) and tau[j]:
 // H_j = I - tau_j v_j v_j^H.  Results become FP64 while the exchange travels, or by
@@ -44,6 +45,7 @@ using namespace fixp;
 using namespace griddev;
 
 constexpr int HC = 16;   // blocks of a full cluster
+constexpr int HROWS = 32;  // most rows of a block left in a step
 constexpr int HPAD = 64;  // zeros after the vectors: rows run in steps of 64 entries
 
 // A cluster with its rows in shared memory, a grid likewise, a grid with its rows in
@@ -125,7 +127,10 @@ __device__ __forceinline__ ll warp_sum64(ll v) {
 
 struct ShCtl {
     ull q;               // grid form: the block's share of v^H A v
-    ll qt[2][16 * HC];   // cluster form: every warp's share, from every block
+    zint sum[HROWS];     // products of row segments with v
+    zint first[HROWS];   // rows' entries of column j+1
+    ll diag[HROWS];
+    ll qt[2][8 * HC];    // cluster form: every warp's share, from every block
     uint64_t mbar[2];    // cluster form: a step's exchange has arrived
     int abort;
     unsigned S[3][NORM_LIMBS];  // squared norm, limbs, triple buffered by step
@@ -160,9 +165,13 @@ __device__ __forceinline__ ll to_fix(double x, int s) {
 // x 2^-56 as FP64, |x| < 2^62
 __device__ __forceinline__ double unit56(ll x) { return scale2(__ll2double_rn(x), -56); }
 
-template <int FORM, int RW>
-__global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
+// row warps of a block
+constexpr int row_warps(int form) { return form == CLUSTER ? 8 : 16; }
+
+template <int FORM>
+__global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(TrdIn p) {
     constexpr bool GRID = FORM != CLUSTER;
+    constexpr int RW = row_warps(FORM);
     constexpr int HM = 32 * RW, HT = HM + 32;  // threads of the row warps; the scalar warp
     extern __shared__ __align__(16) unsigned char hsm[];
     __shared__ ShCtl sh;
@@ -360,6 +369,16 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
     auto unfix = [&](ll x, int s) { return scalbn(__ll2double_rn(x), f - 61 - s); };
     __syncthreads();
     for (int l = tid; l < 3 * (n + HPAD); l += HT) vD[l] = make_int4(0, 0, 0, 0);  // vU and wU too
+    // block `lane`'s mailbox
+    uint32_t rmp = 0, rma = 0, rmd = 0, rqt = 0, rbar = 0;
+    if (!GRID && lane < C) {
+        rmp = map_shared(mp, lane);
+        rma = map_shared(ma, lane);
+        rmd = map_shared(md, lane);
+        rqt = map_shared(sh.qt, lane);
+        rbar = map_shared(sh.mbar, lane);
+    }
+    int i0 = b, nrows = b < n ? (n - 1 - b) / C + 1 : 0;  // the first own row above j, own rows left
     for (int j = 0; j + 1 < n; ++j) {
         __syncthreads();  // squared norm of the column, its entries and alpha
         // its bit length, by lanes
@@ -438,19 +457,12 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em)));
             bar_named(1, HM);
             // ---- A. rows: pending update, product with v ------------------------
-            zint P{0, 0}, Aj{0, 0};
-            ll Dg = 0;
-            int k = 0;
-            int i = b + C * warp;
-            if (i <= j) i += (j - i + RW * C) / (RW * C) * (RW * C);  // first own row above j
-            const int i0 = i;
-            // lane k keeps the warp's k-th row's result (at most 32 rows a warp)
             const bool moved = sh.shift[j % 3] != 0;
-            for (; i < n; i += RW * C, ++k) {
+            // row i from its entry l on, every dl-th 64 of them: its lane's share of
+            // the product; the entry of column j+1 and the diagonal one as they pass
+            auto row_part = [&](int i, int l, int dl, zint& first, ll& dg) -> zint {
                 zint* a = A + (size_t)row(i) * n;
                 Dot s{0, 0, 0, 0, 0, 0};
-                zint first{0, 0};
-                ll dg = 0;
                 const int4 wi = wU[i], vi = vU[i];
                 const int di = de[i];
                 auto one = [&](zint x, int l) {  // entries from n on count zero
@@ -461,50 +473,44 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
                     if (l == i) dg = x.x;
                     dot_add(s, x, vD[l]);
                 };
-                int l = l0 + lane;
                 zint x0 = a[min(l, n - 1)], x1 = a[min(l + 32, n - 1)];
-                for (; l < n; l += 64) {
-                    const zint y0 = a[min(l + 64, n - 1)], y1 = a[min(l + 96, n - 1)];
+                for (; l - lane < n; l += dl) {
+                    const zint y0 = a[min(l + dl, n - 1)], y1 = a[min(l + dl + 32, n - 1)];
                     one(x0, l);
                     one(x1, l + 32);
                     x0 = y0;
                     x1 = y1;
                 }
-                const zint t = dot_value(s);
-                const ll px = warp_sum64(t.x), py = warp_sum64(t.y);
-                const ll fx = __shfl_sync(0xffffffffu, first.x, 0), fy = __shfl_sync(0xffffffffu, first.y, 0);
-                dg = __shfl_sync(0xffffffffu, dg, (i - l0) & 31);
-                if (lane == k) {
-                    P = zint{px, py};
-                    Aj = zint{fx, fy};
-                    Dg = dg;
+                return dot_value(s);
+            };
+            if (!GRID) {
+                // a warp to a row; lane k keeps and finishes the warp's k-th row
+                zint P{0, 0}, Aj{0, 0};
+                ll Dg = 0;
+                int k = 0;
+                int i = b + C * warp;
+                if (i <= j) i += (j - i + RW * C) / (RW * C) * (RW * C);  // first own row above j
+                const int w0 = i;
+                for (; i < n; i += RW * C, ++k) {
+                    zint first{0, 0};
+                    ll dg = 0;
+                    const zint t = row_part(i, l0 + lane, 64, first, dg);
+                    const ll px = warp_sum64(t.x), py = warp_sum64(t.y);
+                    const ll fx = __shfl_sync(0xffffffffu, first.x, 0), fy = __shfl_sync(0xffffffffu, first.y, 0);
+                    dg = __shfl_sync(0xffffffffu, dg, (i - l0) & 31);
+                    if (lane == k) {
+                        P = zint{px, py};
+                        Aj = zint{fx, fy};
+                        Dg = dg;
+                    }
                 }
-            }
-            bar_named(2, HT);  // beta and the first entry of v
-            const int io = i0 + RW * C * lane;
-            ll q = 0;
-            if (lane < k) {
-                P = minus_real(P, Aj, sh.beta, s0);
-                q = re_dot(io == l0 ? zsft(sh.v1, -s0) : value29(vD[io]), P);
-                if (GRID) {
-                    mp[buf * n + io] = P;
-                    ma[buf * n + io] = Aj;
-                    md[buf * n + io] = Dg;
+                bar_named(2, HT);  // beta and the first entry of v
+                const int io = w0 + RW * C * lane;
+                ll q = 0;
+                if (lane < k) {
+                    P = minus_real(P, Aj, sh.beta, s0);
+                    q = re_dot(io == l0 ? zsft(sh.v1, -s0) : value29(vD[io]), P);
                 }
-            }
-            if (GRID) {
-                if (k) {
-                    q = warp_sum64(q);
-                    if (lane == 0) atomicAdd(&sh.q, (ull)q);
-                }
-                bar_named(1, HM);
-                arrivals += (unsigned)C;
-                if (tid == 0) {
-                    atomicAdd(p.mq + j % 3, sh.q);
-                    sh.q = 0;
-                    grid_arrive(p.bar);
-                }
-            } else {
                 // every warp sends its share of q, rows or not: a block that has
                 // everybody's share knows that nobody reads the buffer it will
                 // write two steps on
@@ -515,15 +521,62 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
                     const ll dr = __shfl_sync(0xffffffffu, Dg, r);
                     qs += __shfl_sync(0xffffffffu, q, r);
                     if (lane < C) {
-                        const int ir = buf * n + i0 + RW * C * r;
-                        const uint32_t mb = map_shared(&sh.mbar[buf], lane);
-                        st_async(map_shared(mp + ir, lane), pr, mb);
-                        st_async(map_shared(ma + ir, lane), ar, mb);
-                        st_async(map_shared(md + ir, lane), dr, mb);
+                        const int ir = buf * n + w0 + RW * C * r;
+                        st_async(rmp + 16 * ir, pr, rbar + 8 * buf);
+                        st_async(rma + 16 * ir, ar, rbar + 8 * buf);
+                        st_async(rmd + 8 * ir, dr, rbar + 8 * buf);
                     }
                 }
-                if (lane < C)
-                    st_async(map_shared(&sh.qt[buf][RW * b + warp], lane), qs, map_shared(&sh.mbar[buf], lane));
+                if (lane < C) st_async(rqt + 8 * (8 * HC * buf + RW * b + warp), qs, rbar + 8 * buf);
+            } else {
+                // Local row r is matrix row i0 + C r; 2^ls warps share a row while there
+                // are more warps than rows (a warp alone on its scheduler takes 1,900
+                // clocks for 64 entries: order 512 4,427 us without sharing, 3,794 with)
+                if (i0 <= j) {
+                    i0 += C;
+                    --nrows;
+                }
+                int ls = 0;
+                if (nrows > 0) {
+                    ls = nrows > RW ? 0 : 31 - __clz(RW) - (nrows > 1 ? 32 - __clz(nrows - 1) : 0);
+                    ls = min(ls, 31 - __clz((n - l0 + 63) >> 6));
+                }
+                for (int r = warp >> ls; r < nrows; r += RW >> ls) {
+                    const int i = i0 + C * r, seg = warp & ((1 << ls) - 1);
+                    zint first{0, 0};
+                    ll dg = 0;
+                    const zint t = row_part(i, l0 + 64 * seg + lane, 64 << ls, first, dg);
+                    if (seg == 0 && lane == 0) sh.first[r] = first;
+                    if (((i - l0) >> 6 & ((1 << ls) - 1)) == seg && ((i - l0) & 31) == lane) sh.diag[r] = dg;
+                    const ll px = warp_sum64(t.x), py = warp_sum64(t.y);
+                    if (lane == 0) sh.sum[(r << ls) + seg] = zint{px, py};
+                }
+                bar_named(2, HT);  // the rows' sums; beta and the first entry of v
+                ll qs = 0;
+                for (int r = warp; r < nrows; r += RW) {  // a warp finishes a row
+                    const int i = i0 + C * r, ir = buf * n + i;
+                    zint P{0, 0};
+                    for (int t = 0; t < 1 << ls; ++t) {
+                        const zint u = sh.sum[(r << ls) + t];
+                        P = zint{P.x + u.x, P.y + u.y};
+                    }
+                    const zint Aj = sh.first[r];
+                    P = minus_real(P, Aj, sh.beta, s0);
+                    if (lane == 0) {
+                        mp[ir] = P;
+                        ma[ir] = Aj;
+                        md[ir] = sh.diag[r];
+                    }
+                    qs += re_dot(i == l0 ? zsft(sh.v1, -s0) : value29(vD[i]), P);
+                }
+                if (qs && lane == 0) atomicAdd(&sh.q, (ull)qs);
+                bar_named(1, HM);
+                arrivals += (unsigned)C;
+                if (tid == 0) {
+                    atomicAdd(p.mq + j % 3, sh.q);
+                    sh.q = 0;
+                    grid_arrive(p.bar);
+                }
             }
             // while the results travel: v for the back-transformation, the largest
             // entry of v 2^-e
@@ -557,6 +610,15 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
         // ---- B. w, column j+1, its norm ----------------------------------------
         if (warp < RW) {
             const int off = buf * n;
+            // the first entry's loads travel while h is found
+            zint pf{0, 0}, af{0, 0};
+            ll df = 0;
+            if (l0 + tid < n) {
+                const int o = off + l0 + tid;
+                pf = GRID ? ld_zint(mp + o) : mp[o];
+                af = GRID ? ld_zint(ma + o) : ma[o];
+                df = GRID ? __ldcg(md + o) : md[o];
+            }
             ll q = 0;
             if (GRID) {
                 q = (ll)__ldcg(p.mq + j % 3);
@@ -577,7 +639,7 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             int emn = INT_MAX, any = 0;
             for (int l = l0 + tid; l < n; l += HM) {
                 const bool top = l == l0;
-                const zint pl = GRID ? ld_zint(mp + off + l) : mp[off + l];
+                const zint pl = l == l0 + tid ? pf : GRID ? ld_zint(mp + off + l) : mp[off + l];
                 const zint x = xr[l];
                 const int el = ee[l];
                 int en = el;
@@ -586,7 +648,7 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
                     const float vx = __ll2float_rn(x.x) * fv, vy = __ll2float_rn(x.y) * fv;
                     const float wx = tx * px - ty * py - fa * vx, wy = tx * py + ty * px - fa * vy;
                     const float av = fabsf(vx) + fabsf(vy);
-                    const float a = __ll2float_rn(GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
+                    const float a = __ll2float_rn(l == l0 + tid ? df : GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
                     en = next_exponent(el, cap[l], a, 2.f * (wx * vx + wy * vy),
                                        2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), vx * vx + vy * vy);
                     if (top) en = cn;  // its row becomes column j+1
@@ -614,7 +676,7 @@ __global__ void __launch_bounds__(32 * RW + 32) hetrd_fix_kernel(TrdIn p) {
             const int d0 = de[l0];
             Norm2 S2{0, 0};
             for (int l = l0 + tid; l < n; l += HM) {
-                zint x = zsft(GRID ? ld_zint(ma + off + l) : ma[off + l], de[l] + d0);
+                zint x = zsft(l == l0 + tid ? af : GRID ? ld_zint(ma + off + l) : ma[off + l], de[l] + d0);
                 update(x, wU[l], vU[l], w1, v1);
                 if (l > l0) {
                     emit(l, l0 + 1, x, ee[l], emn, S2);
@@ -650,16 +712,16 @@ size_t hetrd_smem(Form form, int64_t n, int64_t C) {
 
 constexpr size_t HSMEM = 220 * 1024;  // dynamic shared memory a block can have beside ShCtl
 
-template <int FORM, int RW>
+template <int FORM>
 void launch(Ctx* ctx, const TrdIn& a, int64_t C, size_t smem) {
-    auto k = hetrd_fix_kernel<FORM, RW>;
+    auto k = hetrd_fix_kernel<FORM>;
     // the limit for the largest order, the same from every thread
     TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
-    TN_REQUIRE(smem <= HSMEM, "hetrd: matrix order too large");
+    TN_REQUIRE(smem <= HSMEM && (a.n + C - 1) / C <= HROWS, "hetrd: matrix order too large");
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at;
     cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(32 * RW + 32);
+    cfg.blockDim = dim3(32 * row_warps(FORM) + 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cfg.attrs = &at;
@@ -678,7 +740,7 @@ void launch(Ctx* ctx, const TrdIn& a, int64_t C, size_t smem) {
 
 // whether this GPU can hold the widest cluster at all
 int clusters_fit() {
-    auto k = hetrd_fix_kernel<CLUSTER, 16>;
+    auto k = hetrd_fix_kernel<CLUSTER>;
     TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HSMEM));
     TN_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
@@ -687,7 +749,7 @@ int clusters_fit() {
     at.val.clusterDim.x = HC;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3(HC);
-    cfg.blockDim = dim3(32 * 16 + 32);
+    cfg.blockDim = dim3(32 * row_warps(CLUSTER) + 32);
     cfg.dynamicSmemBytes = HSMEM;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
@@ -707,10 +769,10 @@ void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, 
     // Blocks of the cluster: the row work of a step (n^2 / 3 entries on average at
     // 180 clocks per 32) against the exchange with more blocks.  The grid's barrier
     // and vectors through L2 cost 4 us a step more, its rows next to nothing: order
-    // 300 takes 2,589 us in a cluster and 2,308 on the grid, order 256 1,873 in a
-    // cluster, order 400 4,915 against 3,214.
+    // 160 takes 837 us in a cluster and 1,069 on the grid, 200 1,179 and 1,329, 256
+    // 1,900 and 1,646.
     int64_t C = n <= 16 ? 1 : n <= 32 ? 4 : n <= 64 ? 8 : HC;
-    const bool grid = n > 288 || ctx->trd_clusters == 0;
+    const bool grid = n > 208 || ctx->trd_clusters == 0;
     if (grid) C = ctx->sm_count;
     const bool rows_global = grid && hetrd_smem(GRID_SHARED, n, C) > HSMEM;
     auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -745,13 +807,11 @@ void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, 
     if (rows_global) {
         a.A = reinterpret_cast<zint*>(take(nn));
         a.xr = reinterpret_cast<zint*>(take(nx));
-        launch<GRID_GLOBAL, 16>(ctx, a, C, hetrd_smem(GRID_GLOBAL, n, C));
+        launch<GRID_GLOBAL>(ctx, a, C, hetrd_smem(GRID_GLOBAL, n, C));
     } else if (grid) {
-        launch<GRID_SHARED, 16>(ctx, a, C, hetrd_smem(GRID_SHARED, n, C));
-    } else if (n <= 8 * C) {  // a warp per row
-        launch<CLUSTER, 8>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
+        launch<GRID_SHARED>(ctx, a, C, hetrd_smem(GRID_SHARED, n, C));
     } else {
-        launch<CLUSTER, 16>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
+        launch<CLUSTER>(ctx, a, C, hetrd_smem(CLUSTER, n, C));
     }
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());

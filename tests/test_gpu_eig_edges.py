@@ -1,5 +1,5 @@
 """The Hermitian eigensolver at the edges of its forms: cluster sizes 1, 4, 8
-and 16 of the reduction (orders 16, 32, 64 and 288), the divide and conquer's
+and 16 of the reduction (orders 16, 32, 64 and 208), the divide and conquer's
 levels (powers of two) and its two forms (128), the panel widths of the
 back-transformation (64, 128) and its form for small orders (32, 48).
 
@@ -18,7 +18,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 EPS = 2.0 ** -52
-SIZES = [1, 2, 3, 5, 8, 9, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 127, 128, 129, 192, 193, 256, 257, 405, 406]
+SIZES = [1, 2, 3, 5, 8, 9, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 127, 128, 129, 192, 193, 208, 209, 256, 257, 405, 406, 1100, 1200]
 
 
 def dp(a):
