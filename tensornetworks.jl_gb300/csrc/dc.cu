@@ -374,6 +374,8 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
             arrivals += (unsigned)C;
             return grid_sync(p.bar, p.err, arrivals);
         }
+        __threadfence();  // results go through L2
+        __syncwarp();
         cluster_sync();
         return true;
     };

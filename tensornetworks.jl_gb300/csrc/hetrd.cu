@@ -210,13 +210,15 @@ __global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(Tr
             sh.shift[k] = 0;
             if (GRID && b == 0) p.mq[k] = 0;
         }
-        if (!GRID) {  // the cluster barriers below come before the first exchange
+        if (!GRID) {  // seen by the others after the cluster barrier below
             for (int k = 0; k < 2; ++k)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
                     (uint32_t)__cvta_generic_to_shared(&sh.mbar[k])));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
+    // a block's shared memory takes others' stores from the time it runs, no earlier
+    if (!GRID) cluster_sync();
     unsigned hmax = 0;
     for (int i = b + C * warp; i < n && warp < RW; i += RW * C)
         for (int l = lane; l <= i; l += 32) {
@@ -455,6 +457,7 @@ __global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(Tr
         } else {
             // column -> v's limbs for the products (the first entry still alpha)
             for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em)));
+            __syncwarp();
             bar_named(1, HM);
             // ---- A. rows: pending update, product with v ------------------------
             const bool moved = sh.shift[j % 3] != 0;
@@ -570,6 +573,7 @@ __global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(Tr
                     qs += re_dot(i == l0 ? zsft(sh.v1, -s0) : value29(vD[i]), P);
                 }
                 if (qs && lane == 0) atomicAdd(&sh.q, (ull)qs);
+                __syncwarp();
                 bar_named(1, HM);
                 arrivals += (unsigned)C;
                 if (tid == 0) {
@@ -601,6 +605,7 @@ __global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(Tr
             } else if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) {
                 sh.abort = 1;
             }
+            __syncwarp();
             bar_named(3, HT);  // the exchange; tau and c2
             if (sh.abort) {
                 if (tid == 0) atomicExch(p.err, 1);
@@ -670,6 +675,7 @@ __global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(Tr
                 atomicMin(&sh.emin[nb], emn);
                 if (any) sh.shift[nb] = 1;
             }
+            __syncwarp();
             bar_named(1, HM);
             emn = l0 + 1 < n ? sh.emin[nb] : em;
             const int4 w1 = wU[l0], v1 = vU[l0];
