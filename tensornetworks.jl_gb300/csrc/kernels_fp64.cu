@@ -477,7 +477,7 @@ __global__ void multi_axpy_kernel(cplx* __restrict__ w, PtrPack V, const cplx* _
 constexpr int LMAX = 49, LG = 8;
 struct LanczosArgs {
     const cplx* v[LMAX];
-    cplx *w, *partial, *coef;  // partial: gridDim.x x (2 K + 1)
+    cplx *w, *partial, *coef;  // partial: gridDim.x x (2 LMAX + 1); coef: host memory
     int64_t n;
     int K;
     double mark;
@@ -737,6 +737,7 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
     __shared__ double wsum[32];
     __shared__ long long wcnt[32];
     __shared__ double s_total, s_rest;
+    __shared__ int64_t s_k;
     const int T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int nw = T >> 5;
     const int64_t per = (sz + T - 1) / T;
@@ -801,14 +802,11 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
             const int64_t idxs = c > 0 ? (int64_t)c : 1;
             maxd = min(maxd, idxs);
         }
-        const int64_t k = max(maxd, mind);
-        res->k = k;
-        res->total = total;
-        res->discarded = 0.0;
+        s_k = max(maxd, mind);
     }
     __syncthreads();
     // discarded weight = sum_{i >= k} s2 / total
-    const int64_t k = res->k;
+    const int64_t k = s_k;
     double disc = 0.0;
     for (int64_t i = max(lo, k); i < hi; ++i) disc += s2_at(lam, n, i);
 #pragma unroll
@@ -819,6 +817,8 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
     if (t == 0) {
         double d = rest;
         for (int w = 0; w < nw; ++w) d += wsum[w];
+        res->k = k;
+        res->total = total;
         res->discarded = total > 0 ? d / total : 0.0;
         res->err = (dinfo ? *dinfo : 0) | *derr;
     }
@@ -999,9 +999,10 @@ double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, 
     // vectors beyond L2 want more loads in flight
     const int threads = n <= (1 << 20) ? 128 : 512;
     const int C = (int)std::min<int64_t>(ctx->sm_count, (n + threads - 1) / threads);
-    // coefficients and mark, then the partials
-    a.coef = ctx->s_dot.c(ctx, (size_t)(2 * LMAX + 2) + (size_t)C * (2 * LMAX + 1));
-    a.partial = a.coef + 2 * LMAX + 2;
+    a.partial = ctx->s_dot.c(ctx, (size_t)C * (2 * LMAX + 1));
+    double* h = ctx->pinned(2 * (2 * LMAX + 2));
+    h[2 * (2 * LMAX + 1)] = 0.0;
+    a.coef = reinterpret_cast<cplx*>(h);
     a.w = w;
     a.n = n;
     a.K = K;
@@ -1013,8 +1014,6 @@ double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, 
     TN_CHECK_CUDA(cudaLaunchCooperativeKernel((void*)lanczos_orth_kernel, dim3((unsigned)C), dim3(threads), args, 0,
                                               ctx->stream));
     ctx->count();
-    double* h = ctx->pinned(2 * (2 * LMAX + 2));
-    TN_CHECK_CUDA(cudaMemcpyAsync(h, a.coef, sizeof(cplx) * (2 * LMAX + 2), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
     if (h[2 * (2 * LMAX + 1)] != a.mark) {
         TN_CHECK_CUDA(cudaMemsetAsync(ctx->d_bar + 4, 0, 3 * sizeof(unsigned), ctx->stream));
@@ -1060,11 +1059,9 @@ void zfill(Ctx* ctx, cplx* dst, int64_t n, cplx v) {
 }
 
 double znorm2(Ctx* ctx, const cplx* x, int64_t n) {
-    cplx* d = ctx->s_coef.c(ctx, 16);
     const cplx* V[1] = {x};
-    multi_dot(ctx, V, 1, x, n, d);
-    double* h = ctx->pinned(2);
-    TN_CHECK_CUDA(cudaMemcpyAsync(h, d, sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
+    double* h = ctx->pinned(2);  // the kernel writes there
+    multi_dot(ctx, V, 1, x, n, reinterpret_cast<cplx*>(h));
     ctx->sync();
     return h[0];
 }
@@ -1119,13 +1116,14 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
                      int64_t maxdim, int64_t mindim, double* dS, const cplx* G, int64_t g,
                      const int* dinfo) {
     TN_REQUIRE(sz <= n, "keep_rule: more singular values than eigenvalues");
-    KeepDev* dres = static_cast<KeepDev*>(ctx->s_coef.get(ctx, 256));
+    // the result goes to host memory (a copy of its own takes 5 us)
+    static_assert(sizeof(KeepDev) == 4 * sizeof(double), "four words");
+    double* h = ctx->pinned(4);
+    KeepDev* dres = reinterpret_cast<KeepDev*>(h);
     keep_rule_kernel<<<1, one_block(sz), 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
                                                   dinfo, ctx->d_err, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
-    double* h = ctx->pinned(4);
-    TN_CHECK_CUDA(cudaMemcpyAsync(h, dres, sizeof(KeepDev), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
     ctx->tc_pending = false;
     KeepDev r;

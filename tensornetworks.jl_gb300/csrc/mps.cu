@@ -393,11 +393,19 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
             most = std::max(most, ket->size(i));
         }
     }
-    DBuf dst(ctx, sizeof(StackTask) * st.size()), ddt(ctx, sizeof(DotTask) * terms.size());
-    TN_CHECK_CUDA(cudaMemcpyAsync(dst.p, st.data(), sizeof(StackTask) * st.size(), cudaMemcpyHostToDevice, ctx->stream));
+    // the kernels read their tasks from host memory and write the sums there
+    int64_t parts = 1;
+    for (int i = 1; i <= N; ++i)
+        parts = std::max(parts, std::min<int64_t>((bra->dr(i) * ket->dr(i) + 1023) / 1024, 16));
+    const size_t nsum = 2 * (size_t)parts * terms.size();  // first: its stores need 16 bytes' alignment
+    double* h = ctx->pinned(nsum + (sizeof(StackTask) * st.size() + sizeof(DotTask) * terms.size()) / sizeof(double));
+    const cplx* sums = reinterpret_cast<const cplx*>(h);
+    StackTask* hst = reinterpret_cast<StackTask*>(h + nsum);
+    DotTask* hdt = reinterpret_cast<DotTask*>(hst + st.size());
+    std::copy(st.begin(), st.end(), hst);
     for (size_t t = 0; t < st.size(); t += 65535) {
         const dim3 g((unsigned)std::min<int64_t>((most + 127) / 128, 64), (unsigned)std::min<size_t>(st.size() - t, 65535));
-        stack_ops_kernel<<<g, 128, 0, ctx->stream>>>(static_cast<const StackTask*>(dst.p) + t, d);
+        stack_ops_kernel<<<g, 128, 0, ctx->stream>>>(hst + t, d);
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
@@ -426,15 +434,13 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
               ZERO, L[i].c(), q * ca2, 0);
     }
     // sums; terms of three operators and more go on from their left block first
-    std::vector<DotTask> dt(terms.size());
     std::vector<DBuf> mid;
     DBuf B;
-    most = 1;
     for (size_t t = 0; t < terms.size(); ++t) {
         const Term& T = terms[t];
         const int s = T.first, e = s + T.len - 1;
         int64_t ta = bra->dr(s), tb = ket->dr(s);
-        DotTask& k = dt[t];
+        DotTask k;
         k.x = L[s].c() + li[t] * ta;
         k.ldx = nl(s) * ta;
         if (T.len > 2) {
@@ -458,23 +464,18 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
         k.y = T.len == 1 ? R[s + 1].c() : R[e].c() + ri[t] * ta * tb;
         k.rows = ta;
         k.n = ta * tb;
-        most = std::max(most, k.n);
+        hdt[t] = k;
     }
-    TN_CHECK_CUDA(cudaMemcpyAsync(ddt.p, dt.data(), sizeof(DotTask) * dt.size(), cudaMemcpyHostToDevice, ctx->stream));
-    const int64_t parts = std::min<int64_t>((most + 1023) / 1024, 16);
-    DBuf out(ctx, sizeof(cplx) * parts * terms.size());
-    for (size_t t = 0; t < dt.size(); t += 65535) {
-        term_dots_kernel<<<dim3((unsigned)parts, (unsigned)std::min<size_t>(dt.size() - t, 65535)), 128, 0, ctx->stream>>>(
-            static_cast<const DotTask*>(ddt.p) + t, out.c() + parts * t);
+    for (size_t t = 0; t < terms.size(); t += 65535) {
+        term_dots_kernel<<<dim3((unsigned)parts, (unsigned)std::min<size_t>(terms.size() - t, 65535)), 128, 0, ctx->stream>>>(
+            hdt + t, reinterpret_cast<cplx*>(h) + parts * t);
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
-    std::vector<cplx> part(parts * terms.size());
-    TN_CHECK_CUDA(cudaMemcpyAsync(part.data(), out.p, sizeof(cplx) * part.size(), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
     for (size_t t = 0; t < terms.size(); ++t) {
-        cplx v = part[parts * t];
-        for (int64_t k = 1; k < parts; ++k) v = cadd(v, part[parts * t + k]);
+        cplx v = sums[parts * t];
+        for (int64_t k = 1; k < parts; ++k) v = cadd(v, sums[parts * t + k]);
         res[t] = cmul(terms[t].coeff, v);
     }
     return res;
