@@ -72,9 +72,9 @@ void ctx_init(Ctx& c, int device) {
     TN_CHECK_CUDA(cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &thr));
     TN_CHECK_CUDA(cudaMalloc(&c.d_info, sizeof(int)));
     TN_CHECK_CUDA(cudaMalloc(&c.d_bar, 8 * sizeof(unsigned)));
-    TN_CHECK_CUDA(cudaMemset(c.d_bar, 0, 8 * sizeof(unsigned)));
+    TN_CHECK_CUDA(cudaMemsetAsync(c.d_bar, 0, 8 * sizeof(unsigned), c.stream));
     TN_CHECK_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
-    TN_CHECK_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+    TN_CHECK_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
     TN_CHECK_CUDA(cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device));
 }
 

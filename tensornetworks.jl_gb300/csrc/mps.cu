@@ -393,7 +393,9 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
             most = std::max(most, ket->size(i));
         }
     }
-    // the kernels read their tasks from host memory and write the sums there
+    // the kernels' tasks go up by copies on the stream (a kernel reading host memory
+    // that the host wrote just before gave sums from an earlier call's tasks, once);
+    // the sums come back by the kernel's stores
     int64_t parts = 1;
     for (int i = 1; i <= N; ++i)
         parts = std::max(parts, std::min<int64_t>((bra->dr(i) * ket->dr(i) + 1023) / 1024, 16));
@@ -403,9 +405,11 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
     StackTask* hst = reinterpret_cast<StackTask*>(h + nsum);
     DotTask* hdt = reinterpret_cast<DotTask*>(hst + st.size());
     std::copy(st.begin(), st.end(), hst);
+    DBuf dst(ctx, sizeof(StackTask) * st.size()), ddt(ctx, sizeof(DotTask) * terms.size());
+    TN_CHECK_CUDA(cudaMemcpyAsync(dst.p, hst, dst.bytes, cudaMemcpyHostToDevice, ctx->stream));
     for (size_t t = 0; t < st.size(); t += 65535) {
         const dim3 g((unsigned)std::min<int64_t>((most + 127) / 128, 64), (unsigned)std::min<size_t>(st.size() - t, 65535));
-        stack_ops_kernel<<<g, 128, 0, ctx->stream>>>(hst + t, d);
+        stack_ops_kernel<<<g, 128, 0, ctx->stream>>>(dst.as<const StackTask>() + t, d);
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
@@ -466,9 +470,10 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
         k.n = ta * tb;
         hdt[t] = k;
     }
+    TN_CHECK_CUDA(cudaMemcpyAsync(ddt.p, hdt, ddt.bytes, cudaMemcpyHostToDevice, ctx->stream));
     for (size_t t = 0; t < terms.size(); t += 65535) {
         term_dots_kernel<<<dim3((unsigned)parts, (unsigned)std::min<size_t>(terms.size() - t, 65535)), 128, 0, ctx->stream>>>(
-            hdt + t, reinterpret_cast<cplx*>(h) + parts * t);
+            ddt.as<const DotTask>() + t, reinterpret_cast<cplx*>(h) + parts * t);
         ctx->count();
     }
     TN_CHECK_CUDA(cudaGetLastError());
