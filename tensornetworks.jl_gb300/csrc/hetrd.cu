@@ -165,13 +165,13 @@ __device__ __forceinline__ ll to_fix(double x, int s) {
 // x 2^-56 as FP64, |x| < 2^62
 __device__ __forceinline__ double unit56(ll x) { return scale2(__ll2double_rn(x), -56); }
 
-// row warps of a block
-constexpr int row_warps(int form) { return form == CLUSTER ? 8 : 16; }
+template <int FORM>
+constexpr int ROW_WARPS = FORM == CLUSTER ? 8 : 16;  // of a block
 
 template <int FORM>
-__global__ void __launch_bounds__(32 * row_warps(FORM) + 32) hetrd_fix_kernel(TrdIn p) {
+__global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(TrdIn p) {
     constexpr bool GRID = FORM != CLUSTER;
-    constexpr int RW = row_warps(FORM);
+    constexpr int RW = ROW_WARPS<FORM>;
     constexpr int HM = 32 * RW, HT = HM + 32;  // threads of the row warps; the scalar warp
     extern __shared__ __align__(16) unsigned char hsm[];
     __shared__ ShCtl sh;
@@ -727,7 +727,7 @@ void launch(Ctx* ctx, const TrdIn& a, int64_t C, size_t smem) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at;
     cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(32 * row_warps(FORM) + 32);
+    cfg.blockDim = dim3(32 * ROW_WARPS<FORM> + 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cfg.attrs = &at;
@@ -755,7 +755,7 @@ int clusters_fit() {
     at.val.clusterDim.x = HC;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3(HC);
-    cfg.blockDim = dim3(32 * row_warps(CLUSTER) + 32);
+    cfg.blockDim = dim3(32 * ROW_WARPS<CLUSTER> + 32);
     cfg.dynamicSmemBytes = HSMEM;
     cfg.attrs = &at;
     cfg.numAttrs = 1;

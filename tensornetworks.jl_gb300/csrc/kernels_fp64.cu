@@ -253,7 +253,7 @@ void zgemm_dispatch_b(Ctx* ctx, Op opb, dim3 grid, int64_t m, int64_t n, int64_t
 // all entries, as 0 times it is NaN.  parts threads share a column's J.
 // Against all entries of four J at a time by one thread: bond dimension 64, 12 x 12:
 // 41.0 -> 8.2 us; 20 x 20: 104.5 -> 13.4, at 256 204 -> 30.7 (10.7 of them FP64).
-__global__ void __launch_bounds__(128) small_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
+__global__ void __launch_bounds__(128, 8) small_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
                                                           const cplx* __restrict__ M, int nI, int nJ, int64_t na,
                                                           int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o,
                                                           int64_t ldc_o, int accumulate, int parts) {
