@@ -371,7 +371,7 @@ int32_t tn_gate2_apply(tn_ctx* ctx, int64_t chil, int64_t chim, int64_t chir, in
                        const double* A1, const double* A2, const double* G, double* out);
 /* C[m x n] = op(A) B with A column-major (m x k, or k x m when conj_a, where
  * op(A) = A^H), B column-major k x n; precision TN_PREC_FP64 runs the FP64
- * SIMT GEMM, TN_PREC_MIXED the 3xTF32 tcgen05 GEMM.  No reference
+ * product, TN_PREC_MIXED the 3xTF32 tcgen05 GEMM.  No reference
  * counterpart: the contraction primitive under tensors.jl:13-18 exposed for
  * tests and callers. */
 int32_t tn_gemm(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, const double* A, int32_t conj_a,
@@ -386,8 +386,8 @@ int32_t tn_truncate(tn_ctx* ctx, int64_t m, int64_t n, const double* theta,
 /* Top `want` eigenpairs of the Hermitian n x n matrix G (host, interleaved,
  * column-major; the lower triangle is read): lam[g] is the g-th largest
  * eigenvalue, V[:, g] (n x want) its unit eigenvector.  The library's own
- * FP64 eigensolver (Householder tridiagonalisation, bisection, inverse
- * iteration, QR re-orthonormalisation, back-transformation), which sets the
+ * eigensolver (Householder tridiagonalisation in 62-bit fixed point, divide and
+ * conquer, back-transformation), which sets the
  * cut of every truncated split in place of LAPACK's SVD at tensors.jl:191-195;
  * exposed for tests and callers.  n <= 4096. */
 int32_t tn_eigh_top(tn_ctx* ctx, int64_t n, const double* G, int64_t want, double* lam, double* V);

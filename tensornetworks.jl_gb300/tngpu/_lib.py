@@ -112,7 +112,7 @@ _SIGS = {
     "tn_profile_phases": (i32, [P, dp]),
 }
 
-PROF_CLASSES = ("tc_cgemm_kernel (tcgen05 3xTF32)", "zgemm_kernel (FP64)", "eigensolver (own FP64: tridiagonal, bisection, inverse iteration, QR, back-transform)",
+PROF_CLASSES = ("tc_cgemm_kernel (tcgen05 3xTF32)", "zgemm (FP64 complex products)", "eigensolver (own: fixed-point tridiagonal, divide and conquer, back-transform)",
                 "small_apply_kernel (FP64 legs)", "heff_mid_kernel (FP32 leg)",
                 "operand conversion / partial reduction", "Lanczos vector ops",
                 "all launches (count only)")
