@@ -15,20 +15,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Sum over the block (blockDim.x a multiple of 32, at most 1024); the result
-// is valid in every thread.  The warp totals are added as a tree: a serial
-// chain of dependent FP64 additions costs tens of cycles per link on GB300.
-__device__ __forceinline__ double block_sum(double v, double* ws) {
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
-    __syncthreads();
-    if (lane == 0) ws[w] = v;
-    __syncthreads();
-    double t = lane < nw ? ws[lane] : 0.0;
-    t = warp_sum(t);
-    return __shfl_sync(0xffffffffu, t, 0);
-}
-
 // Number of eigenvalues of the symmetric tridiagonal T (diagonal d, squared
 // off-diagonal e2) below x: sign changes of the leading principal minors
 // q_k = det(T[0:k, 0:k] - x I), q_k = (d_k - x) q_{k-1} - e_{k-1}^2 q_{k-2}
