@@ -85,6 +85,9 @@ struct Ctx {
     // split-K FP64 GEMMs draw partial buffers from the pool; callers that must
     // not allocate turn them off
     bool splitk = true;
+    // FP64 DMRG: small splits and sums keep one order of operations, so that its
+    // results are the same to the last bit in every version (eig_fp64.cu)
+    bool ordered = false;
     // a tensor-core kernel of the FP64 path ran since d_err was last read
     bool tc_pending = false;
     double* h_pinned = nullptr;  // small pinned staging area
@@ -242,6 +245,10 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
 // synchronisation; a timed-out grid barrier leaves ctx->d_bar[2] nonzero.
 // psd: G is positive semidefinite (a Gram matrix).
 void eig_top(Ctx* ctx, const cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X, bool psd);
+// The same for a Gram matrix of order up to EIG_FP64_MAX with every operation in FP64
+// and in one order (eig_fp64.cu).
+constexpr int EIG_FP64_MAX = 64, EIG_FP64_MOVE = 16;  // of DMRG's splits, of gauge moves without truncation
+void eig_top_fp64(Ctx* ctx, const cplx* G, int64_t n, int64_t want, double* lam_asc, cplx* X);
 // Householder tridiagonalisation (hetrd.cu): T in (d, e), reflector j in column j
 // of V (rows j+1.., explicit first entry), H_j = I - tau_j v_j v_j^H.
 void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, cplx* V, bool psd, int* perm);

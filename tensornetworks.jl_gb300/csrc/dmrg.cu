@@ -316,13 +316,17 @@ void dmrg_run(tn_mps* psi, const DmrgTerms& terms, const tn_dmrg_opts& o, double
     // the tensor cores for the whole call; restored on every exit path
     struct MixedMode {
         Ctx* c;
-        bool old;
-        ~MixedMode() { c->mixed = old; }
-    } mode_guard{ctx, ctx->mixed};
+        bool mixed, ordered;
+        ~MixedMode() {
+            c->mixed = mixed;
+            c->ordered = ordered;
+        }
+    } mode_guard{ctx, ctx->mixed, ctx->ordered};
     // ctx->mixed: H_eff products and truncation projections on the tensor
     // cores; the environment updates follow EnvCache::env_mixed (FP64 with
     // TN_PREC_MIXED_ENV64)
     ctx->mixed = mixed_heff;
+    ctx->ordered = !mixed_heff;
     movecenter(psi, 1, no_trunc());
     std::vector<std::unique_ptr<EnvCache>> envs;
     std::vector<std::unique_ptr<OvlCache>> ovls;

@@ -143,27 +143,23 @@ __global__ void __launch_bounds__(ZS_T)
             const cplx* bb = B + b * sB + ((OPB == OP_N || OPB == OP_R) ? j * ldb : j);
             const int64_t da = (OPA == OP_N || OPA == OP_R) ? lda : 1;
             const int64_t db = (OPB == OP_N || OPB == OP_R) ? 1 : ldb;
-            cplx acc1 = cmk(0.0, 0.0);
-            auto step = [&](cplx x, cplx y, cplx& s) {
+            auto step = [&](cplx x, cplx y) {
                 if (OPA == OP_C || OPA == OP_R) x.y = -x.y;
                 if (OPB == OP_C || OPB == OP_R) y.y = -y.y;
-                s = cfma(x, y, s);
+                acc = cfma(x, y, acc);
             };
             int64_t l = l0;
-            for (; l + 3 < l1; l += 4) {  // four loads in flight, two FMA chains
+            for (; l + 3 < l1; l += 4) {  // four loads in flight
                 cplx x[4], y[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     x[u] = a[(l + u) * da];
                     y[u] = bb[(l + u) * db];
                 }
-                step(x[0], y[0], acc);
-                step(x[1], y[1], acc1);
-                step(x[2], y[2], acc);
-                step(x[3], y[3], acc1);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) step(x[u], y[u]);
             }
-            for (; l < l1; ++l) step(a[l * da], bb[l * db], acc);
-            acc = cadd(acc, acc1);
+            for (; l < l1; ++l) step(a[l * da], bb[l * db]);
         }
         if (S > 1) {
             part[ty * OX + tx] = acc;
@@ -210,10 +206,12 @@ void zgemm_small_dispatch_b(Ctx* ctx, Op opb, int64_t m, int64_t n, int64_t k, c
     // slices of at least 16 terms up to a full warp, and on to eight warps per
     // SM.
     const int64_t outs = m * n * batch;
+    // DMRG's sums of up to 192 terms stay in one piece (eig_fp64.cu).
     int OX = 32, S = 1;
-    while (OX > 2 && outs < 2 * OX * (int64_t)ctx->sm_count && k >= 16 * (64 / OX)) OX /= 2;
-    while (OX * S < 32 && k >= 32 * S) S *= 2;
-    while (OX * S < ZS_T && outs / OX * ((OX * S + 31) / 32) < 8 * (int64_t)ctx->sm_count && k >= 32 * S) S *= 2;
+    const bool whole = ctx->ordered && k <= 192;
+    while (!whole && OX > 2 && outs < 2 * OX * (int64_t)ctx->sm_count && k >= 16 * (64 / OX)) OX /= 2;
+    while (!whole && OX * S < 32 && k >= 32 * S) S *= 2;
+    while (!whole && OX * S < ZS_T && outs / OX * ((OX * S + 31) / 32) < 8 * (int64_t)ctx->sm_count && k >= 32 * S) S *= 2;
     const unsigned g = (unsigned)std::min<int64_t>((outs + OX - 1) / OX, (int64_t)ctx->sm_count * 64);
     const dim3 th((unsigned)OX, (unsigned)S);
     switch (opb) {
@@ -250,34 +248,38 @@ void zgemm_dispatch_b(Ctx* ctx, Op opb, dim3 grid, int64_t m, int64_t n, int64_t
 // is what bounds this kernel, so every block lists the nonzero entries of M's
 // columns, real ones, imaginary ones (two multiply-adds either) and the rest (four),
 // and a thread multiplies those; a column of the input with an infinity or NaN takes
-// all entries, as 0 times it is NaN.  parts threads share a column's J.
+// all entries, as 0 times it is NaN.  IN_ORDER: by their index instead, which gives the
+// full sum's bits, for small bonds of DMRG (eig_fp64.cu); at bond dimension 256 a sweep
+// of the XXZ chain takes 138 ms that way, 130 by kinds.  parts threads share a column's J.
 // Against all entries of four J at a time by one thread: bond dimension 64, 12 x 12:
 // 41.0 -> 8.2 us; 20 x 20: 104.5 -> 13.4, at 256 204 -> 30.7 (10.7 of them FP64).
+template <bool IN_ORDER>
 __global__ void __launch_bounds__(128, 8) small_apply_kernel(const cplx* __restrict__ in, cplx* __restrict__ out,
                                                           const cplx* __restrict__ M, int nI, int nJ, int64_t na,
                                                           int64_t nc, int64_t lda_i, int64_t ldc_i, int64_t lda_o,
                                                           int64_t ldc_o, int accumulate, int parts) {
     extern __shared__ cplx sM[];
-    unsigned short* li = reinterpret_cast<unsigned short*>(sM + nI * nJ);  // nonzero I of column J
+    unsigned short* li = reinterpret_cast<unsigned short*>(sM + nI * nJ);  // nonzero I of column J, with their kind
     unsigned short* cnt = li + nI * nJ;  // 3 to a column: where each kind ends
     const int lane = threadIdx.x & 31;
     for (int t = threadIdx.x; t < nI * nJ; t += blockDim.x) sM[t] = M[t];
     __syncthreads();
     for (int J = threadIdx.x >> 5; J < nJ; J += blockDim.x >> 5) {
         int c = 0;
-        for (int kind = 0; kind < 3; ++kind) {
+        for (int pass = 1; pass <= (IN_ORDER ? 1 : 3); ++pass) {
             for (int I0 = 0; I0 < nI; I0 += 32) {
                 const int I = I0 + lane;
-                bool on = false;
+                int kind = 0;  // 1 real, 2 imaginary, 3 neither
                 if (I < nI) {
                     const cplx v = sM[I + nI * J];
-                    on = kind == (v.y == 0.0 ? (v.x == 0.0 ? 3 : 0) : v.x == 0.0 ? 1 : 2);
+                    kind = (v.x != 0.0 ? 1 : 0) | (v.y != 0.0 ? 2 : 0);
                 }
+                const bool on = IN_ORDER ? kind != 0 : kind == pass;
                 const unsigned m = __ballot_sync(0xffffffffu, on);
-                if (on) li[nI * J + c + __popc(m & ((1u << lane) - 1u))] = (unsigned short)I;
+                if (on) li[nI * J + c + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(I | kind << 13);
                 c += __popc(m);
             }
-            if (lane == 0) cnt[3 * J + kind] = (unsigned short)c;
+            if (lane == 0) cnt[3 * J + pass - 1] = (unsigned short)c;
         }
     }
     __syncthreads();
@@ -300,21 +302,38 @@ __global__ void __launch_bounds__(128, 8) small_apply_kernel(const cplx* __restr
             } else {
                 const unsigned short* l = li + nI * J;
                 const cplx* m = sM + nI * J;
-                const int n0 = cnt[3 * J], n1 = cnt[3 * J + 1], n2 = cnt[3 * J + 2];
+                const int n0 = cnt[3 * J];
+                if (IN_ORDER) {
 #pragma unroll 4
-                for (int t = 0; t < n0; ++t) {
-                    const cplx v = x[lda_i * l[t]];
-                    const double r = m[l[t]].x;
-                    s = cmk(fma(v.x, r, s.x), fma(v.y, r, s.y));
-                }
+                    for (int t = 0; t < n0; ++t) {
+                        const int I = l[t] & 0x1fff, kind = l[t] >> 13;
+                        const cplx v = x[lda_i * I], w = m[I];
+                        if (kind == 1) s = cmk(fma(v.x, w.x, s.x), fma(v.y, w.x, s.y));
+                        else if (kind == 2) s = cmk(fma(-v.y, w.y, s.x), fma(v.x, w.y, s.y));
+                        else s = cfma(v, w, s);
+                    }
+                } else {
+                    const int n1 = cnt[3 * J + 1], n2 = cnt[3 * J + 2];
+#pragma unroll 4
+                    for (int t = 0; t < n0; ++t) {
+                        const int I = l[t] & 0x1fff;
+                        const cplx v = x[lda_i * I];
+                        const double r = m[I].x;
+                        s = cmk(fma(v.x, r, s.x), fma(v.y, r, s.y));
+                    }
 #pragma unroll 2
-                for (int t = n0; t < n1; ++t) {
-                    const cplx v = x[lda_i * l[t]];
-                    const double r = m[l[t]].y;
-                    s = cmk(fma(-v.y, r, s.x), fma(v.x, r, s.y));
-                }
+                    for (int t = n0; t < n1; ++t) {
+                        const int I = l[t] & 0x1fff;
+                        const cplx v = x[lda_i * I];
+                        const double r = m[I].y;
+                        s = cmk(fma(-v.y, r, s.x), fma(v.x, r, s.y));
+                    }
 #pragma unroll 2
-                for (int t = n1; t < n2; ++t) s = cfma(x[lda_i * l[t]], m[l[t]], s);
+                    for (int t = n1; t < n2; ++t) {
+                        const int I = l[t] & 0x1fff;
+                        s = cfma(x[lda_i * I], m[I], s);
+                    }
+                }
             }
             cplx* dst = y + lda_o * J;
             *dst = accumulate ? cadd(*dst, s) : s;
@@ -931,14 +950,15 @@ void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int
     const size_t smem = (sizeof(cplx) + 2) * nI * nJ + 6 * nJ;
     // the whole operator is staged in shared memory: up to 96 KiB, above the
     // 48 KiB a launch gets without opting in
+    auto kernel = ctx->ordered && na * nc <= 4096 ? small_apply_kernel<true> : small_apply_kernel<false>;
     if (smem > 48 * 1024)
-        TN_CHECK_CUDA(cudaFuncSetAttribute(small_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        TN_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            18 * 4096 + 6 * 4096));
     // threads to a column until two warps are on every scheduler
     int parts = 1;
     while (parts < nJ && na * nc * parts < (int64_t)ctx->sm_count * 256) parts *= 2;
     parts = std::min(parts, nJ);
-    small_apply_kernel<<<grid_for(ctx, na * nc * parts, 128), 128, smem, ctx->stream>>>(
+    kernel<<<grid_for(ctx, na * nc * parts, 128), 128, smem, ctx->stream>>>(
         in, out, M, nI, nJ, na, nc, lda_i, ldc_i, lda_o, ldc_o, accumulate ? 1 : 0, parts);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
@@ -995,9 +1015,11 @@ double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, 
     ProfScope ps(ctx, 6, 32.0 * n * K, 16.0 * n * (3 * K + 5));
     LanczosArgs a{};
     for (int j = 0; j < K; ++j) a.v[j] = hV[j];
+    // Up to 256 entries an SM a thread has one entry and the sums are those of
+    // multi_dot's blocks, in its order (DMRG's results rest on it, eig_fp64.cu).  Above,
     // one warp on every scheduler keeps the FP64 units busy and has the fewest sums;
-    // vectors beyond L2 want more loads in flight
-    const int threads = n <= (1 << 20) ? 128 : 512;
+    // vectors beyond L2 want more loads in flight.
+    const int threads = n <= 256 * (int64_t)ctx->sm_count ? 256 : n <= (1 << 20) ? 128 : 512;
     const int C = (int)std::min<int64_t>(ctx->sm_count, (n + threads - 1) / threads);
     a.partial = ctx->s_dot.c(ctx, (size_t)C * (2 * LMAX + 1));
     double* h = ctx->pinned(2 * (2 * LMAX + 2));
@@ -1120,7 +1142,9 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
     static_assert(sizeof(KeepDev) == 4 * sizeof(double), "four words");
     double* h = ctx->pinned(4);
     KeepDev* dres = reinterpret_cast<KeepDev*>(h);
-    keep_rule_kernel<<<1, one_block(sz), 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
+    // the trace is summed by a thread an entry where its last bit counts
+    const unsigned threads = one_block(ctx->ordered ? std::max(sz, g) : sz);
+    keep_rule_kernel<<<1, threads, 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
                                                   dinfo, ctx->d_err, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());

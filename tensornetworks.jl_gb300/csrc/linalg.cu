@@ -164,7 +164,11 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
     double* lam = ctx->s_eigval.d(ctx, (size_t)want + sz);
     double* dS = lam + want;
     cplx* V = ctx->s_x.c(ctx, (size_t)g * want);  // top eigenvectors, descending
-    eig_top(ctx, G, g, want, lam, V, true);
+    const int64_t fp64 = ctx->ordered ? EIG_FP64_MAX : !ctx->mixed && cutoff == 0.0 && maxdim == 0 ? EIG_FP64_MOVE : 0;
+    if (g <= fp64)
+        eig_top_fp64(ctx, G, g, want, lam, V);
+    else
+        eig_top(ctx, G, g, want, lam, V, true);
     // G's trace gives the weight below the computed values; the eigensolver's barrier
     // status is read back with the keep-rule result
     KeepResult kr = keep_rule(ctx, lam, want, want, cutoff, maxdim, mindim, dS, G, g,
