@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(192, 1)
         // ---- epilogue: warps 2..5, TMEM lane quarter = warp % 4 ----
         const int q = warp & 3;
         const int64_t m = m0 + 32 * q + lane;
-        if (mbar_wait(accf, 0)) {
+        // a warp leaves or goes on as a whole: the loads below are the warp's
+        if (__all_sync(0xffffffffu, mbar_wait(accf, 0))) {
             tc_fence_after();
             const bool ok = !*(volatile int*)abort_flag;
             float* outz = p.out + (size_t)blockIdx.z * p.chunk_stride;
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(192, 1)
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
+        __syncwarp();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(TMEM_COLS));

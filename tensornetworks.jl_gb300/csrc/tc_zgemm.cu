@@ -344,6 +344,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* a
     }
     return true;
 }
+// the same, whatever the other roles did
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    const uint64_t t0 = gtimer();
+    while (!mbar_try(bar, parity))
+        if (gtimer() - t0 > WAIT_NS) return;
+}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y, int z) {
     asm volatile(
@@ -501,11 +507,8 @@ __global__ void __launch_bounds__(GEMM_T, 1)
                 }
             }
             // copies still in flight land before the CTA can retire
-            for (int i = (n > STAGES ? n - STAGES : 0); i < n; ++i) {
-                const uint64_t t0 = gtimer();
-                while (!mbar_try(&full[i % STAGES], (uint32_t)(i / STAGES) & 1u))
-                    if (gtimer() - t0 > WAIT_NS) break;
-            }
+            for (int i = (n > STAGES ? n - STAGES : 0); i < n; ++i)
+                mbar_drain(&full[i % STAGES], (uint32_t)(i / STAGES) & 1u);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -552,6 +555,8 @@ __global__ void __launch_bounds__(GEMM_T, 1)
                     }
                 }
             }
+            // after an abort products in flight end before their TMEM goes back
+            if (!ok && n > 0) mbar_drain(&empty[(n - 1) % STAGES], (uint32_t)((n - 1) / STAGES) & 1u);
         }
     } else {
         // two warps per TMEM lane quarter, 64 columns each
@@ -565,7 +570,9 @@ __global__ void __launch_bounds__(GEMM_T, 1)
             const int ncol = (int)min((int64_t)64, p.N - nb);
             uchar2* out = p.q + ((int64_t)w.mod * p.N + nb) * p.ldq + m;
             for (int ch = 0; ch < nch; ++ch, ++c) {
-                if (!mbar_wait(&accf[c & 1], (uint32_t)(c >> 1) & 1u, abort_flag)) {
+                // a warp leaves or goes on as a whole: the loads below are the warp's
+                if (!__all_sync(0xffffffffu, mbar_wait(&accf[c & 1], (uint32_t)(c >> 1) & 1u, abort_flag))) {
+                    atomicExch(abort_flag, 1);
                     ok = false;
                     break;
                 }
@@ -612,6 +619,7 @@ __global__ void __launch_bounds__(GEMM_T, 1)
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
+        __syncwarp();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(TMEM_COLS));
