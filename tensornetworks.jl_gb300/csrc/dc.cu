@@ -3,16 +3,21 @@
 // S. C. Eisenstat, SIAM J. Matrix Anal. Appl. 16, 1995), steps 2-4 of the
 // eigensolver (eig.cu): top `want` eigenvalues and orthonormal eigenvectors.
 //
-// T is cut into 1 x 1 blocks, T = blockdiag(T1 - rho.., T2 - rho..) + rho v v^T
-// at every cut, and neighbouring blocks merge level by level.  A merge of two
+// T is cut into 1 x 1 blocks, T = blockdiag(T1 - rho a^2 .., T2 - rho b^2 ..) +
+// rho v v^T at every cut, v = (.., a, b, ..) with rho a b = |e| and b / a about the square
+// root of the neighbouring diagonals' ratio, so that what is subtracted from either is
+// no larger than it (Gram matrices are graded, and their small eigenvalues' vectors
+// have to be right to that scale).  Neighbouring blocks merge level by level.  A merge of two
 // eigensystems (D, Q) is the rank-one problem D + rho z z^T with
 // z = Q^T v: its eigenvalues are the roots of 1 / rho + sum z_i^2 / (d_i - x),
 // one between each two poles.
 //
 // Every merge runs the same steps without deflation, so that no step is serial
-// in its size: equal poles are moved an ulp apart and entries of z get a floor of
-// 2^-56 (both a backward error of rounding size), after which all roots are
-// simple.  Roots are kept as an offset from their nearest pole, to full relative
+// in its size: equal poles are moved an ulp apart, entries of v^T Q get a floor of 2^-56
+// of v's, off-diagonals one of 2^-58 of the neighbouring diagonals' mean (all backward
+// errors of rounding size where they act; an absolute floor of 2^-58 mixed pairs of weight
+// 1e-10 closer than 4e-8 of it, 2e-8 in the energy of a chain of 30 sites), after
+// which all roots are simple.  Roots are kept as an offset from their nearest pole, to full relative
 // accuracy, and z is recomputed from them (Loewner's formula), which makes the
 // eigenvectors orthogonal to working precision however close the roots lie.
 //
@@ -56,6 +61,7 @@ struct DcArgs {
     double* mu;   // n: root minus its nearest pole
     int* org;     // n: that pole
     int* idx;     // n: a pole's place in the unsorted merge
+    double* rinv; // n: 1 / rho of the merge around a row
     double *Qa, *Qb;   // n x n, block diagonal
     double* Z;         // n x want
     double* lam_asc;   // want
@@ -72,14 +78,16 @@ __device__ __forceinline__ ll okey(double x) {
 __device__ __forceinline__ double unkey(ll k) {
     return __longlong_as_double(k < 0 ? k ^ 0x7fffffffffffffffll : k);
 }
-// Monotone map to integers whose unit step is an ulp, or 2^-82 below 2^-30; in
-// integers, as FP64 conversions cost 64 clocks each.
-constexpr ll B30 = (1023ll - 30) << 52;
+// Monotone map to integers whose unit step is an ulp, or 2^-112 below 2^-60 (FP32 holds
+// its square root's reciprocal and more); in integers, as FP64 conversions cost 64
+// clocks each.
+constexpr int UEX = 1023 - 60;
+constexpr ll UBITS = (ll)UEX << 52;
 __device__ __forceinline__ ll to_grid(double v) {
     const ll bits = __double_as_longlong(v), a = bits & LLONG_MAX;
-    const int s = 993 - (int)(a >> 52);  // below 2^-30 the mantissa moves down by s
+    const int s = UEX - (int)(a >> 52);  // below 2^-60 the mantissa moves down by s
     ll k;
-    if (s <= 0) k = (1ll << 52) + a - B30;
+    if (s <= 0) k = (1ll << 52) + a - UBITS;
     else if (s > 53) k = 0;
     else k = (((a & ((1ll << 52) - 1)) | (1ll << 52)) + (1ll << (s - 1))) >> s;
     return bits < 0 ? -k : k;
@@ -88,12 +96,12 @@ __device__ __forceinline__ double from_grid(ll k) {
     const ll a = k < 0 ? -k : k;
     ll bits;
     if (a >= (1ll << 52)) {
-        bits = B30 + a - (1ll << 52);
+        bits = UBITS + a - (1ll << 52);
     } else if (a == 0) {
         bits = 0;
     } else {
         const int s = __clzll(a) - 11;  // mantissa's leading bit to bit 52
-        bits = ((ll)(993 - s) << 52) + ((a << s) - (1ll << 52));
+        bits = ((ll)(UEX - s) << 52) + ((a << s) - (1ll << 52));
     }
     return __longlong_as_double(k < 0 ? bits | LLONG_MIN : bits);
 }
@@ -112,6 +120,21 @@ __device__ __forceinline__ double rcp(double x) {
 
 // floor(log2 |x|) of a normal x; zero counts as 2^-1023
 __device__ __forceinline__ int expo(double x) { return ((__double2hiint(x) >> 20) & 0x7ff) - 1023; }
+
+// T's off-diagonal e between diagonals d1 and d2 (all below 1) as rho a b
+struct Cut {
+    double rho, a, b;
+};
+__device__ __forceinline__ double pow2(int s) { return __hiloint2double((1023 + s) << 20, 0); }
+__device__ __forceinline__ Cut cut(double d1, double d2, double e) {
+    const int x1 = expo(d1), x2 = expo(d2), hi = max(x1, x2), lo = min(x1, x2);
+    // the smaller side's factor 2^s: rho stays at the larger diagonal's size where |e|
+    // does, and is |e| where |e| is the largest of the three
+    const int s = max(min(max((lo - hi) / 2, expo(e) - hi), 0), -56);
+    const double r = scale2(fabs(e), -s), f = pow2(max(hi - 58, -112));
+    const double t = pow2(s);
+    return Cut{__double_as_longlong(r) > __double_as_longlong(f) ? r : f, x1 < x2 ? t : 1.0, x1 < x2 ? 1.0 : t};
+}
 
 // sums over aligned groups of g lanes
 __device__ __forceinline__ double gsum(double v, int g) {
@@ -394,7 +417,8 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
     __syncthreads();
     const int ex = min(max((int)(s_max >> 20) - 1022, -900), 900);
     const double down = scalbn(1.0, -ex), up = s_max ? scalbn(1.0, ex) : 0.0;
-    const double rho_min = 0x1p-58;
+    // the cut above row i
+    auto cut_at = [&](int i) { return cut(p.d[i - 1] * down, p.d[i] * down, p.e[i - 1] * down); };
     double *Q = p.Qa, *Qn = p.Qb;
     // ---- base blocks: a warp each, levels 2, 4 and 8 in its shared memory ------------
     for (int B = wid; B * BASE < n; B += W) {
@@ -403,8 +427,14 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
         __syncwarp();
         if (lane < N) {
             double x = p.d[r0 + i] * down;
-            if (r0 + i > 0) x -= fmax(fabs(p.e[r0 + i - 1] * down), rho_min);
-            if (r0 + i + 1 < n) x -= fmax(fabs(p.e[r0 + i] * down), rho_min);
+            if (r0 + i > 0) {
+                const Cut c = cut_at(r0 + i);
+                x = fma(-c.rho, c.b * c.b, x);
+            }
+            if (r0 + i + 1 < n) {
+                const Cut c = cut_at(r0 + i + 1);
+                x = fma(-c.rho, c.a * c.a, x);
+            }
             s.D[i] = x;
         }
         for (int t = lane; t < BASE * BASE; t += 32) s.Q[0][t] = t % BASE == t / BASE ? 1.0 : 0.0;
@@ -424,10 +454,11 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
                     const ll k = s.key[i];
                     rk = 0;
                     for (int t = lo; t < hi; ++t) rk += s.key[t] < k || (s.key[t] == k && t < i);
-                    double z = i < mid ? q[(mid - 1) + BASE * i] : copysign(1.0, p.e[r0 + mid - 1]) * q[mid + BASE * i];
+                    const Cut c = cut_at(r0 + mid);
+                    double z = q[(i < mid ? mid - 1 : mid) + BASE * i];
                     if (expo(z) < -56) z = copysign(0x1p-56, z);
                     s.srt[lo + rk] = k;
-                    s.z[lo + rk] = z;
+                    s.z[lo + rk] = i < mid ? c.a * z : copysign(c.b, p.e[r0 + mid - 1]) * z;
                     s.idx[lo + rk] = i - lo;
                 }
                 __syncwarp();
@@ -447,7 +478,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
                 const bool on = lane / g < N && mid < N;
                 // lanes without a root follow the first
                 const int lo1 = on ? lo : 0, j = on ? jj - lo : 0, K = min(lo1 + K0, N) - lo1;
-                const double rinv = rcp(fmax(fabs(p.e[r0 + lo1 + h - 1] * down), rho_min));
+                const double rinv = rcp(cut_at(r0 + lo1 + h).rho);
                 int o;
                 double mu;
                 find_root<2, true>(s.ds + lo1, s.z + lo1, K, K0, g, j, rinv, s.pf[lane / g], o, mu);
@@ -506,12 +537,13 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
             if (mid >= n) continue;  // an unpaired block goes up as it is
             ll* key = reinterpret_cast<ll*>(dsm);
             ll* srt = key + K;
-            const double ev = p.e[mid - 1];
+            const Cut cm = cut_at(mid);
+            const double cb = copysign(cm.b, p.e[mid - 1]);
+            if (tid == 0) p.rinv[mid] = rcp(cm.rho);
             for (int i = tid; i < K; i += nt) key[i] = okey(__ldcg(p.D + lo + i));
             __syncthreads();
             for (int i = tid; i < K; i += nt) {
-                double z = i < h ? __ldcg(Q + (mid - 1) + (size_t)n * (lo + i))
-                                 : copysign(1.0, ev) * __ldcg(Q + mid + (size_t)n * (lo + i));
+                double z = __ldcg(Q + (i < h ? mid - 1 : mid) + (size_t)n * (lo + i));
                 const ll k = key[i];
                 const int base = i < h ? h : 0;  // the other block; ties: first block first
                 int l = 0, r = i < h ? K - h : h;
@@ -524,7 +556,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
                 const int rk = min((i < h ? i : i - h) + l, K - 1);
                 srt[rk] = k;
                 if (expo(z) < -56) z = copysign(0x1p-56, z);
-                p.z[lo + rk] = z;
+                p.z[lo + rk] = z * (i < h ? cm.a : cb);
                 p.idx[lo + rk] = i;
             }
             __syncthreads();
@@ -566,7 +598,7 @@ __global__ void __launch_bounds__(DT) dc_kernel(DcArgs p) {
                 if (!__any_sync(0xffffffffu, on)) continue;
                 const int G = on ? r : 0, lo = G / K0 * K0, mid = lo + h, K = min(lo + K0, n) - lo, j = G - lo;
                 float2* pf = reinterpret_cast<float2*>(dsm) + (size_t)warp * max(K0, 32) + sub * K0;
-                const double rinv = rcp(fmax(fabs(p.e[mid - 1] * down), rho_min));
+                const double rinv = __ldcg(p.rinv + mid);
                 int o;
                 double mu;
                 if (K0 <= 128) find_root<4, false>(p.ds + lo, p.z + lo, K, K0, g, j, rinv, pf, o, mu);
@@ -661,7 +693,7 @@ void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t 
     auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t n8 = r256(sizeof(double) * n), n4 = r256(sizeof(int) * n),
                  nn = r256(sizeof(double) * (size_t)n * n);
-    char* base = static_cast<char*>(ctx->s_dc.get(ctx, 5 * n8 + 2 * n4 + 2 * nn));
+    char* base = static_cast<char*>(ctx->s_dc.get(ctx, 6 * n8 + 2 * n4 + 2 * nn));
     auto take = [&](size_t b) {
         char* q = base;
         base += b;
@@ -677,6 +709,7 @@ void tridiag_top(Ctx* ctx, int64_t n, const double* d, const double* e, int64_t 
     a.z = reinterpret_cast<double*>(take(n8));
     a.zh = reinterpret_cast<double*>(take(n8));
     a.mu = reinterpret_cast<double*>(take(n8));
+    a.rinv = reinterpret_cast<double*>(take(n8));
     a.org = reinterpret_cast<int*>(take(n4));
     a.idx = reinterpret_cast<int*>(take(n4));
     a.Qa = reinterpret_cast<double*>(take(nn));
