@@ -370,8 +370,9 @@ int32_t tn_env_right(tn_ctx* ctx, int64_t chil, int64_t chir, int32_t d, int64_t
 int32_t tn_gate2_apply(tn_ctx* ctx, int64_t chil, int64_t chim, int64_t chir, int32_t d,
                        const double* A1, const double* A2, const double* G, double* out);
 /* C[m x n] = op(A) B with A column-major (m x k, or k x m when conj_a, where
- * op(A) = A^H), B column-major k x n; precision TN_PREC_FP64 runs the FP64
- * product, TN_PREC_MIXED the 3xTF32 tcgen05 GEMM.  No reference
+ * op(A) = A^H), B column-major k x n; precision TN_PREC_FP64 runs on the FP64
+ * units (every output within k 2^-52 of sum |a| |b|), TN_PREC_MIXED the 3xTF32
+ * tcgen05 GEMM.  No reference
  * counterpart: the contraction primitive under tensors.jl:13-18 exposed for
  * tests and callers. */
 int32_t tn_gemm(tn_ctx* ctx, int64_t m, int64_t n, int64_t k, const double* A, int32_t conj_a,

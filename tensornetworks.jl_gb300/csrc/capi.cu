@@ -949,8 +949,8 @@ int32_t tn_gemm(tn_ctx* h, int64_t m, int64_t n, int64_t k, const double* A, int
         mixed_gemm(ctx, m, n, k, dA.c(), conj_a != 0, dB.c(), dC.c());
     } else {
         const cplx one = cmk(1, 0), zero = cmk(0, 0);
-        zgemm(ctx, conj_a ? OP_C : OP_N, OP_N, m, n, k, one, dA.c(), conj_a ? k : m, 0, dB.c(), k, 0,
-              zero, dC.c(), m, 0);
+        zgemm_fp64(ctx, conj_a ? OP_C : OP_N, OP_N, m, n, k, one, dA.c(), conj_a ? k : m, 0, dB.c(), k, 0,
+                   zero, dC.c(), m, 0);
     }
     d2h(ctx, Cout, dC.p, 16 * (size_t)m * n);
     ctx->sync();

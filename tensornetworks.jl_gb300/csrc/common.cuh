@@ -70,7 +70,7 @@ struct Ctx {
     int sm_count = 0;
     // reusable scratch for the hot path
     Scratch s_gram, s_eigval, s_work, s_x, s_y, s_t1, s_t2, s_dot, s_coef, s_mixa, s_mixb, s_mixc,
-        s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz, s_trd, s_bt, s_dc;
+        s_mixd, s_mixe, s_mixf, s_eig, s_splitk, s_tcz, s_trd, s_bt, s_dc, s_grade;
     int* d_info = nullptr;
     // words of kernels whose blocks wait or count: 0 arrivals and 2 error of the
     // eigensolver's barriers (a bounded wait ran out), 3 blocks done of a dot
@@ -177,14 +177,27 @@ enum Op { OP_N = 0, OP_T = 1, OP_C = 2, OP_R = 3 };  // R: conjugate without tra
 // C[m x n] = alpha * op(A) * op(B) + beta * C, column-major, batched by count.
 void zgemm(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
            int64_t lda, int64_t strideA, const cplx* B, int64_t ldb, int64_t strideB, cplx beta,
-           cplx* C, int64_t ldc, int64_t strideC, int64_t batch = 1, bool lower_only = false);
+           cplx* C, int64_t ldc, int64_t strideC, int64_t batch = 1, bool lower_only = false,
+           const int* kexp = nullptr, int ksign = 1);
 
-// The same product on the tensor cores (tc_zgemm.cu), FP64 accurate, one batch;
-// false when it does not take the call (no room for its operand planes, K
-// above 2^16).
+// The same on the FP64 units whatever the size: every output within K 2^-53 of
+// sum_k |a_ik| |b_kj|.
+void zgemm_fp64(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
+                int64_t lda, int64_t strideA, const cplx* B, int64_t ldb, int64_t strideB, cplx beta,
+                cplx* C, int64_t ldc, int64_t strideC, int64_t batch = 1, bool lower_only = false);
+
+// The same product on the tensor cores (tc_zgemm.cu), one batch: every output within
+// 4 K max_k |a_ik| max_k |b_kj| 2^-T in either part, T = min(57, (122 - ceil log2 K) / 2), and 2^-53 of
+// itself, as if op(A) were op(A) 2^(ksign kexp) and op(B) 2^(-ksign kexp) op(B) when kexp
+// (k integers on the device) is given; false when it does not take the call (no room
+// for its operand planes, K above 2^16).
 bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
               int64_t lda, const cplx* B, int64_t ldb, cplx beta, cplx* C, int64_t ldc,
-              bool lower_only);
+              bool lower_only, const int* kexp = nullptr, int ksign = 1);
+// whether zgemm sends a product of this size there
+bool tc_sized(const Ctx* ctx, int64_t m, int64_t n, int64_t k, bool lower = false);
+// out[i] = half the exponent of G[i, i]: the grading of a Gram matrix' rows
+void grading(Ctx* ctx, const cplx* G, int64_t n, int* out);
 
 // out[a + lda_o*J + ldc_o*c] (=|+=) sum_I in[a + lda_i*I + ldc_i*c] * M[I + nI*J]
 void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int nJ, int64_t na,

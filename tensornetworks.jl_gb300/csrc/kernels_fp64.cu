@@ -667,6 +667,11 @@ __global__ void top_eigvecs_kernel(const cplx* __restrict__ G, int64_t n, int64_
     }
 }
 
+__global__ void grading_kernel(const cplx* __restrict__ G, int64_t n, int* __restrict__ out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (int)((((unsigned)__double2hiint(G[i + n * i].x) >> 20) & 0x7ffu) / 2);
+}
+
 __global__ void scale_cols_kernel(cplx* X, int64_t m, int64_t k, const double* s, int invert) {
     const int64_t total = m * k;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -847,6 +852,9 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
 // five stream operations (27 us at any size up to 256 x 128 x 128 = 4.2 M, where
 // the per-output kernel takes 37 us; at 128^3 = 2.1 M it is 27 us against 23).
 constexpr double ZTC_MIN = 2.5e6;
+inline double gemm_work(int64_t m, int64_t n, int64_t k, int64_t batch, bool lower) {
+    return (lower ? 0.5 : 1.0) * (double)m * n * k * batch;
+}
 
 // Threads of a kernel of one block that scans n values: no more warps than there are
 // values for, as every FP64 instruction of every warp holds its scheduler for 64
@@ -863,9 +871,26 @@ inline int grid_for(Ctx* ctx, int64_t n, int threads = 256) {
 }  // namespace
 
 // -------------------------------------------------------------------------
+// Large products run on the tensor cores.  Thin ones (a side below 16) read more than
+// they multiply: there the operand conversion (64 bytes written per entry) costs more
+// than the FP64 pipe.
+bool tc_sized(const Ctx* ctx, int64_t m, int64_t n, int64_t k, bool lower) {
+    return ctx->splitk && std::min(m, n) >= 16 && k >= 8 && gemm_work(m, n, k, 1, lower) >= ZTC_MIN;
+}
+
 void zgemm(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
            int64_t lda, int64_t sA, const cplx* B, int64_t ldb, int64_t sB, cplx beta, cplx* C,
-           int64_t ldc, int64_t sC, int64_t batch, bool lower_only) {
+           int64_t ldc, int64_t sC, int64_t batch, bool lower_only, const int* kexp, int ksign) {
+    if (batch == 1 && tc_sized(ctx, m, n, k, lower_only)) {
+        ProfScope ps(ctx, 1, 8.0 * gemm_work(m, n, k, 1, lower_only), 16.0 * (double)(m * k + k * n + m * n));
+        if (zgemm_tc(ctx, opa, opb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, kexp, ksign)) return;
+    }
+    zgemm_fp64(ctx, opa, opb, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, lower_only);
+}
+
+void zgemm_fp64(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
+                int64_t lda, int64_t sA, const cplx* B, int64_t ldb, int64_t sB, cplx beta, cplx* C,
+                int64_t ldc, int64_t sC, int64_t batch, bool lower_only) {
     if (m <= 0 || n <= 0 || batch <= 0) return;
     const int lower = lower_only ? 1 : 0;
     TN_REQUIRE((n + GB_N - 1) / GB_N <= 65535 && batch <= 65535, "zgemm: grid too large");
@@ -873,16 +898,9 @@ void zgemm(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha
     if (k <= 0) {  // C = beta * C
         alpha = cmk(0, 0);
     }
-    ProfScope ps(ctx, 1, (lower ? 0.5 : 1.0) * 8.0 * m * n * (double)std::max<int64_t>(k, 0) * batch,
-                 16.0 * (double)(m * k + k * n + m * n) * batch);
-    // Large products run on the tensor cores.  Thin ones (a side below 16) read
-    // more than they multiply: there the operand conversion (64 bytes written
-    // per entry) costs more than the FP64 pipe.
-    const double work = (lower ? 0.5 : 1.0) * (double)m * n * k * batch;
-    const bool tc = ctx->splitk && batch == 1 && std::min(m, n) >= 16 && k >= 8 && work >= ZTC_MIN;
-    if (tc && zgemm_tc(ctx, opa, opb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only)) return;
-    // Otherwise (small products, and callers that must not allocate): a 64 x 64
-    // tile keeps one SM busy for 4.1 us per K entry at two FP64 FMAs per clock
+    const double work = gemm_work(m, n, std::max<int64_t>(k, 0), batch, lower_only);
+    ProfScope ps(ctx, 1, 8.0 * work, 16.0 * (double)(m * k + k * n + m * n) * batch);
+    // A 64 x 64 tile keeps one SM busy for 4.1 us per K entry at two FP64 FMAs per clock
     // (64^3: 263 us), the per-output kernel spreads the same work over the SMs
     // (64^3: 7 us).  Tiles, with their reuse, pay once they fill the SMs.
     if (std::min(m, n) < 48 || work < 6.0e7) {
@@ -1086,6 +1104,12 @@ double znorm2(Ctx* ctx, const cplx* x, int64_t n) {
     multi_dot(ctx, V, 1, x, n, reinterpret_cast<cplx*>(h));
     ctx->sync();
     return h[0];
+}
+
+void grading(Ctx* ctx, const cplx* G, int64_t n, int* out) {
+    grading_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(G, n, out);
+    ctx->count();
+    TN_CHECK_CUDA(cudaGetLastError());
 }
 
 void take_top_eigvecs(Ctx* ctx, const cplx* G, int64_t n, int64_t k, cplx* dst, int64_t ncols) {

@@ -85,7 +85,7 @@ void ctx_release(Ctx& c) {
     Scratch* all[] = {&c.s_gram, &c.s_eigval, &c.s_work, &c.s_x, &c.s_y, &c.s_t1, &c.s_t2,
                       &c.s_dot, &c.s_coef, &c.s_mixa, &c.s_mixb, &c.s_mixc, &c.s_mixd, &c.s_mixe,
                       &c.s_mixf, &c.s_eig, &c.s_splitk, &c.s_tcz,
-                      &c.s_trd, &c.s_bt, &c.s_dc};
+                      &c.s_trd, &c.s_bt, &c.s_dc, &c.s_grade};
     for (Scratch* s : all) s->buf.reset();
     if (c.stream) cudaStreamSynchronize(c.stream);
     if (c.d_info) cudaFree(c.d_info);
@@ -178,6 +178,14 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
     // tensor-core projection in mixed mode, for products large enough to pay
     // for the operand conversion
     const bool use_tc = ctx->mixed && (double)m * n * k >= (double)(1 << 21);
+    // theta's rows (columns) are graded and the vectors against them: |V_li| is at most
+    // about s_i / sqrt(G_ll), so with D = sqrt(G_ll) V^H D has rows of size s_i and D^-1 theta
+    // none smaller than another
+    int* ge = nullptr;
+    if (!use_tc && tc_sized(ctx, k, std::max(m, n), g)) {
+        ge = static_cast<int*>(ctx->s_grade.get(ctx, sizeof(int) * (size_t)g));
+        grading(ctx, G, g, ge);
+    }
     if (left_iso) {
         X = DBuf(ctx, sizeof(cplx) * m * k);
         Y = DBuf(ctx, sizeof(cplx) * k * n);
@@ -185,14 +193,14 @@ SplitResult trunc_split(Ctx* ctx, const cplx* theta, int64_t m, int64_t n, doubl
         if (use_tc)  // the isometry stays exact; the projection on the tensor cores
             mixed_gemm(ctx, k, n, m, X.c(), true, theta, Y.c());
         else
-            zgemm(ctx, OP_C, OP_N, k, n, m, one, X.c(), m, 0, theta, m, 0, zero, Y.c(), k, 0);
+            zgemm(ctx, OP_C, OP_N, k, n, m, one, X.c(), m, 0, theta, m, 0, zero, Y.c(), k, 0, 1, false, ge, 1);
     } else {
         X = DBuf(ctx, sizeof(cplx) * m * k);
         Y = DBuf(ctx, sizeof(cplx) * k * n);
         if (use_tc)
             mixed_gemm(ctx, m, k, n, theta, false, V, X.c());
         else
-            zgemm(ctx, OP_N, OP_N, m, k, n, one, theta, m, 0, V, n, 0, zero, X.c(), m, 0);
+            zgemm(ctx, OP_N, OP_N, m, k, n, one, theta, m, 0, V, n, 0, zero, X.c(), m, 0, 1, false, ge, -1);
         conj_transpose(ctx, V, n, k, Y.c());  // Y = V^H (k x n)
     }
     if (S) {

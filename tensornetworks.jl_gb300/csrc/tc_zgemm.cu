@@ -12,7 +12,12 @@
 //
 //   1. every row of op(A) and column of op(B) gets its own power-of-two scale
 //      and becomes integers of T <= 57 bits relative to its largest entry
-//      (FP64 holds 53 relative to each entry);
+//      (FP64 holds 53 relative to each entry).  The result is good to
+//      4 K max_k|a_ik| max_k|b_kj| 2^-T in either part: where large entries of one side meet small
+//      ones of the other all along K, that is more than FP64's
+//      K 2^-53 sum_k |a_ik||b_kj|.  A caller that knows the operands' grading along K
+//      gives it as kexp: op(A) then counts as op(A) D and op(B) as D^-1 op(B), D = 2^kexp,
+//      in that bound;
 //   2. the integers are reduced modulo p_0 .. p_15 <= 251 (pairwise coprime,
 //      product P = 2^124.9) into BF16 planes, real and imaginary;
 //   3. per modulus, tcgen05 forms the four real products of the complex
@@ -30,6 +35,8 @@
 // each operand plane in shared memory feeds two products, so a 128 x 128 tile
 // needs half the L2 traffic per flop, and conversion writes two planes per
 // modulus instead of three.
+#include <climits>
+
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
@@ -119,6 +126,9 @@ struct Side {
     int64_t rows, K, ld;
     int kmajor, conj;
     unsigned* hmax;          // rows: largest high word of |re|, |im|
+    const int* kexp;         // K: entry (r, k) counts as itself 2^(ksign kexp[k]); null: as itself
+    int ksign;
+    int* ex;                 // rows: largest biased exponent with that, when kexp
     __nv_bfloat16* planes;   // [NP][re, im][rows][ldp]
     int64_t ldp;
     int blocks_max, blocks_cvt;  // grid shares of the two kernels
@@ -133,12 +143,23 @@ __device__ __forceinline__ bool unscaled(unsigned h) {
     return h >= 0x7ff00000u || (h != 0 && h < 0x00100000u);
 }
 
+// biased exponent of the larger part of an entry whose high word of both is h
+__device__ __forceinline__ int exponent(unsigned h, int shift) {
+    return h ? max((int)(h >> 20), 1) + shift : INT_MIN;
+}
+template <bool GRADED>  // with kexp
+__device__ __forceinline__ int row_exponent(const Side& s, int64_t r) {
+    if (GRADED) return s.ex[r] < -100000 ? 1 : s.ex[r];  // a row of zeros: any
+    return max(1, min((int)(s.hmax[r] >> 20), 0x7fe));
+}
+
 constexpr int SEG = 512;    // K per block of the row-maximum kernel
 constexpr int MAX_T = 512;  // its threads
 
 // Largest high word of every row's entries.  Integer maxima, so the order of
 // the atomics that merge several segments does not matter (hmax then starts
 // at zero); one segment stores directly.
+template <bool GRADED>
 __global__ void __launch_bounds__(MAX_T) zrow_max_kernel(Side a, Side b) {
     const bool first = (int)blockIdx.x < a.blocks_max;
     const Side& s = first ? a : b;
@@ -150,38 +171,59 @@ __global__ void __launch_bounds__(MAX_T) zrow_max_kernel(Side a, Side b) {
         const int64_t r = (int64_t)(blk / nseg) * (MAX_T / 32) + warp;
         if (r >= s.rows) return;
         unsigned m = 0;
+        int e = INT_MIN;
 #pragma unroll 4
         for (int64_t k = k0 + lane; k < k1; k += 32) {
             const cplx v = s.src[k + s.ld * r];
-            m = max(m, max(hi_abs(v.x), hi_abs(v.y)));
+            const unsigned h = max(hi_abs(v.x), hi_abs(v.y));
+            m = max(m, h);
+            if (GRADED) e = max(e, exponent(h, s.ksign * s.kexp[k]));
         }
         m = __reduce_max_sync(0xffffffffu, m);
+        if (GRADED) e = __reduce_max_sync(0xffffffffu, e);
         if (lane == 0) {
             if (nseg > 1) atomicMax(s.hmax + r, m);
             else s.hmax[r] = m;
+            if (GRADED) {
+                if (nseg > 1) atomicMax(s.ex + r, e);
+                else s.ex[r] = e;
+            }
         }
     } else {  // 32 rows per block, a lane each; the warps share the segment
         __shared__ unsigned sm[MAX_T / 32][32];
+        __shared__ int se[GRADED ? MAX_T / 32 : 1][32];
         const int64_t r = (int64_t)(blk / nseg) * 32 + lane;
         unsigned m = 0;
+        int e = INT_MIN;
         if (r < s.rows)
 #pragma unroll 8
             for (int64_t k = k0 + warp; k < k1; k += MAX_T / 32) {
                 const cplx v = s.src[r + s.ld * k];
-                m = max(m, max(hi_abs(v.x), hi_abs(v.y)));
+                const unsigned h = max(hi_abs(v.x), hi_abs(v.y));
+                m = max(m, h);
+                if (GRADED) e = max(e, exponent(h, s.ksign * s.kexp[k]));
             }
         sm[warp][lane] = m;
+        if (GRADED) se[warp][lane] = e;
         __syncthreads();
         if (warp == 0 && r < s.rows) {
 #pragma unroll
-            for (int w = 1; w < MAX_T / 32; ++w) m = max(m, sm[w][lane]);
+            for (int w = 1; w < MAX_T / 32; ++w) {
+                m = max(m, sm[w][lane]);
+                if (GRADED) e = max(e, se[w][lane]);
+            }
             if (nseg > 1) atomicMax(s.hmax + r, m);
             else s.hmax[r] = m;
+            if (GRADED) {
+                if (nseg > 1) atomicMax(s.ex + r, e);
+                else s.ex[r] = e;
+            }
         }
     }
 }
 
-// x 2^(T - 1 - e) rounded to an integer, |x| < 2^(e+1) with e the row's exponent
+// x 2^(T - 1 - e) rounded to an integer, |x| < 2^(e+1) with e the row's exponent less
+// what the entry's K index adds
 __device__ __forceinline__ int64_t to_int(double x, int E, int T) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     int e = (int)((b >> 52) & 0x7ff);
@@ -215,7 +257,7 @@ __device__ __forceinline__ float mod_p(float v, float p, float rp) {
 
 // Residues of four consecutive K entries of one row, eight bytes per plane;
 // parts [lo, hi) of (real, imaginary).
-__device__ __forceinline__ void convert4(const cplx* v, int lo, int hi, int E, int T, int conj,
+__device__ __forceinline__ void convert4(const cplx* v, int lo, int hi, const int* E, int T, int conj,
                                          __nv_bfloat16* __restrict__ dst, size_t plane) {
 #pragma unroll 1
     for (int part = lo; part < hi; ++part) {
@@ -223,7 +265,7 @@ __device__ __forceinline__ void convert4(const cplx* v, int lo, int hi, int E, i
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const double x = part ? (conj ? -v[i].y : v[i].y) : v[i].x;
-            l[i] = Limbs(to_int(x, E, T));
+            l[i] = Limbs(to_int(x, E[i], T));
         }
         __nv_bfloat16* d = dst + part * plane;
 #pragma unroll
@@ -243,9 +285,18 @@ __device__ __forceinline__ void convert4(const cplx* v, int lo, int hi, int E, i
     }
 }
 
+// the row's exponent for K entries k .. k + 3
+template <bool GRADED>
+__device__ __forceinline__ void exponents(const Side& s, int64_t r, int64_t k, int* E) {
+    const int e = row_exponent<GRADED>(s, r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) E[i] = GRADED && k + i < s.K ? e - s.ksign * s.kexp[k + i] : e;
+}
+
 // Residue planes.  A half-warp converts 64 consecutive K entries of a row, so
 // that every plane gets 128-byte stores; operands whose rows are contiguous
 // pass through a shared-memory tile of 32 rows x 64 K.
+template <bool GRADED>
 __global__ void __launch_bounds__(256, 2) zconvert_kernel(Side a, Side b, int T) {
     __shared__ cplx tile[32][65];  // row r, K entry k at (k & 3) * 16 + k / 4: no bank conflicts
     const bool first = (int)blockIdx.x < a.blocks_cvt;
@@ -261,7 +312,8 @@ __global__ void __launch_bounds__(256, 2) zconvert_kernel(Side a, Side b, int T)
         const int64_t r = (int64_t)(blk / nk) * 16 + half;
         const int64_t k = (int64_t)(blk % nk) * 64 + 4 * hl;
         if (r >= s.rows || k >= s.ldp) return;
-        const int E = max(1, min((int)(s.hmax[r] >> 20), 0x7fe));
+        int E[4];
+        exponents<GRADED>(s, r, k, E);
         cplx v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = k + i < s.K ? s.src[k + i + s.ld * r] : cmk(0, 0);
@@ -281,7 +333,8 @@ __global__ void __launch_bounds__(256, 2) zconvert_kernel(Side a, Side b, int T)
         for (int rl = half; rl < 32; rl += 16) {
             const int64_t r = r0 + rl;
             if (r >= s.rows) continue;
-            const int E = max(1, min((int)(s.hmax[r] >> 20), 0x7fe));
+            int E[4];
+            exponents<GRADED>(s, r, k, E);
             cplx v[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) v[i] = tile[rl][16 * i + hl];
@@ -684,6 +737,7 @@ constexpr int CRT_T = 128;
 // C = alpha X + beta C from the residues, four consecutive rows per thread.
 // All-integer up to the last scaling: sixteen 32 x 8 bit products per word
 // where FP64 would wait on its two lanes per clock.
+template <bool GRADED>
 __global__ void __launch_bounds__(CRT_T) zcrt_kernel(Out o, Side a, Side b) {
     const int64_t mq = (o.M + 3) / 4, total = mq * o.N;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
@@ -706,13 +760,13 @@ __global__ void __launch_bounds__(CRT_T) zcrt_kernel(Out o, Side a, Side b) {
             }
         }
         const unsigned hb = b.hmax[n];
-        const int eb = max(1, min((int)(hb >> 20), 0x7fe));
+        const int eb = row_exponent<GRADED>(b, n);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             const int64_t m = m0 + v;
             if (m >= o.M || (o.lower && m < n)) continue;
             const unsigned ha = a.hmax[m];
-            const int ea = max(1, min((int)(ha >> 20), 0x7fe));
+            const int ea = row_exponent<GRADED>(a, m);
             const int sc = ea + eb - 2044 - 2 * o.T;
             double x[2];
 #pragma unroll
@@ -778,14 +832,14 @@ void grids(Side& s) {
 
 bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx alpha, const cplx* A,
               int64_t lda, const cplx* B, int64_t ldb, cplx beta, cplx* C, int64_t ldc,
-              bool lower_only) {
+              bool lower_only, const int* kexp, int ksign) {
     if (m > (1 << 24) || n > (1 << 24) || k > (1 << 16)) return false;
     const int64_t ldp = (k + 7) / 8 * 8, ldq = (m + 3) / 4 * 4;
     auto r256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t bA = r256(sizeof(__nv_bfloat16) * 2 * NP * (size_t)m * ldp);
     const size_t bB = r256(sizeof(__nv_bfloat16) * 2 * NP * (size_t)n * ldp);
     const size_t bQ = r256(sizeof(uchar2) * NP * (size_t)n * ldq);
-    const size_t bH = r256(sizeof(unsigned) * (size_t)(m + n));
+    const size_t bH = r256(2 * sizeof(unsigned) * (size_t)(m + n));
     char* base;
     try {
         base = static_cast<char*>(ctx->s_tcz.get(ctx, bA + bB + bQ + bH));
@@ -795,21 +849,26 @@ bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx al
     }
     unsigned* hmax = reinterpret_cast<unsigned*>(base + bA + bB + bQ);
     Side a{A, m, k, lda, (opa == OP_T || opa == OP_C) ? 1 : 0, (opa == OP_C || opa == OP_R) ? 1 : 0,
-           hmax, reinterpret_cast<__nv_bfloat16*>(base), ldp, 0, 0};
+           hmax, kexp, ksign, reinterpret_cast<int*>(hmax + m + n), reinterpret_cast<__nv_bfloat16*>(base), ldp, 0, 0};
     Side b{B, n, k, ldb, (opb == OP_N || opb == OP_R) ? 1 : 0, (opb == OP_C || opb == OP_R) ? 1 : 0,
-           hmax + m, reinterpret_cast<__nv_bfloat16*>(base + bA), ldp, 0, 0};
+           hmax + m, kexp, -ksign, a.ex + m, reinterpret_cast<__nv_bfloat16*>(base + bA), ldp, 0, 0};
     grids(a);
     grids(b);
     // 2 k 2^2T <= P / 2 with P > 2^124
     int lk = 0;
     while (((int64_t)1 << lk) < k) ++lk;
     const int T = std::min(57, (124 - 2 - lk) / 2);
-    if (k > SEG)
+    if (k > SEG) {
         TN_CHECK_CUDA(cudaMemsetAsync(hmax, 0, sizeof(unsigned) * (size_t)(m + n), ctx->stream));
-    zrow_max_kernel<<<a.blocks_max + b.blocks_max, MAX_T, 0, ctx->stream>>>(a, b);
+        if (kexp)  // below any exponent
+            TN_CHECK_CUDA(cudaMemsetAsync(a.ex, 0x80, sizeof(int) * (size_t)(m + n), ctx->stream));
+    }
+    auto row_max = kexp ? zrow_max_kernel<true> : zrow_max_kernel<false>;
+    row_max<<<a.blocks_max + b.blocks_max, MAX_T, 0, ctx->stream>>>(a, b);
     ctx->count();
     const int ncvt = a.blocks_cvt + b.blocks_cvt;
-    zconvert_kernel<<<dim3(ncvt, ncvt < 2 * ctx->sm_count ? 2 : 1), 256, 0, ctx->stream>>>(a, b, T);
+    auto convert = kexp ? zconvert_kernel<true> : zconvert_kernel<false>;
+    convert<<<dim3(ncvt, ncvt < 2 * ctx->sm_count ? 2 : 1), 256, 0, ctx->stream>>>(a, b, T);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
     CUtensorMap ma, mb;
@@ -835,7 +894,8 @@ bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx al
     const bool plain = alpha.x == 1.0 && alpha.y == 0.0 && beta.x == 0.0 && beta.y == 0.0;
     Out o{m, n, ldc, ldq, alpha, beta, C, p.q, lower_only ? 1 : 0, T, plain ? 1 : 0};
     const int64_t blocks = ((m + 3) / 4 * n + CRT_T - 1) / CRT_T;
-    zcrt_kernel<<<(unsigned)std::min<int64_t>(blocks, (int64_t)ctx->sm_count * 16), CRT_T, 0,
+    auto crt = kexp ? zcrt_kernel<true> : zcrt_kernel<false>;
+    crt<<<(unsigned)std::min<int64_t>(blocks, (int64_t)ctx->sm_count * 16), CRT_T, 0,
                   ctx->stream>>>(o, a, b);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
