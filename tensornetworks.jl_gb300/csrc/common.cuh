@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <cstdio>
+#include <cstring>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -119,6 +120,21 @@ struct Ctx {
     }
     double* pinned(size_t n);
 };
+
+// Words that a kernel stores in pinned memory for the host: cleared to a value that no
+// kernel stores (a NaN of its own) before the launch, looked at after the wait, so that a
+// store that did not come about is an error and not the call's before.
+constexpr uint64_t UNSET = 0x7ff4a5a5a5a5a5a5ull;
+inline void unset(double* h, size_t n) {
+    for (size_t i = 0; i < n; ++i) memcpy(h + i, &UNSET, sizeof(double));
+}
+inline void check_set(const double* h, size_t n) {
+    for (size_t i = 0; i < n; ++i) {
+        uint64_t v;
+        memcpy(&v, h + i, sizeof(v));
+        if (v == UNSET) throw Error(TN_ERR_CUDA, "a kernel's result did not arrive");
+    }
+}
 
 // Records a CUDA event pair around the launches in its scope when the
 // context's profiler is on.

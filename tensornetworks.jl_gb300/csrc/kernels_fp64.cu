@@ -1041,7 +1041,7 @@ double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, 
     const int C = (int)std::min<int64_t>(ctx->sm_count, (n + threads - 1) / threads);
     a.partial = ctx->s_dot.c(ctx, (size_t)C * (2 * LMAX + 1));
     double* h = ctx->pinned(2 * (2 * LMAX + 2));
-    h[2 * (2 * LMAX + 1)] = 0.0;
+    unset(h, 2 * (2 * LMAX + 2));
     a.coef = reinterpret_cast<cplx*>(h);
     a.w = w;
     a.n = n;
@@ -1059,6 +1059,9 @@ double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, 
         TN_CHECK_CUDA(cudaMemsetAsync(ctx->d_bar + 4, 0, 3 * sizeof(unsigned), ctx->stream));
         throw Error(TN_ERR_TIMEOUT, "Lanczos: a bounded grid barrier ran out");
     }
+    check_set(h, 2 * K);
+    check_set(h + 2 * LMAX, 2 * K);
+    check_set(h + 4 * LMAX, 2);
     for (int j = 0; j < K; ++j)
         comp[j] = cmk(h[2 * j] + h[2 * (LMAX + j)], h[2 * j + 1] + h[2 * (LMAX + j) + 1]);
     return std::sqrt(h[4 * LMAX]);
@@ -1101,8 +1104,10 @@ void zfill(Ctx* ctx, cplx* dst, int64_t n, cplx v) {
 double znorm2(Ctx* ctx, const cplx* x, int64_t n) {
     const cplx* V[1] = {x};
     double* h = ctx->pinned(2);  // the kernel writes there
+    unset(h, 2);
     multi_dot(ctx, V, 1, x, n, reinterpret_cast<cplx*>(h));
     ctx->sync();
+    check_set(h, 2);
     return h[0];
 }
 
@@ -1166,6 +1171,7 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
     static_assert(sizeof(KeepDev) == 4 * sizeof(double), "four words");
     double* h = ctx->pinned(4);
     KeepDev* dres = reinterpret_cast<KeepDev*>(h);
+    unset(h, 4);
     // the trace is summed by a thread an entry where its last bit counts
     const unsigned threads = one_block(ctx->ordered ? std::max(sz, g) : sz);
     keep_rule_kernel<<<1, threads, 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
@@ -1173,6 +1179,7 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
     ctx->sync();
+    check_set(h, 4);
     ctx->tc_pending = false;
     KeepDev r;
     memcpy(&r, h, sizeof(KeepDev));

@@ -393,9 +393,8 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
             most = std::max(most, ket->size(i));
         }
     }
-    // the kernels' tasks go up by copies on the stream (a kernel reading host memory
-    // that the host wrote just before gave sums from an earlier call's tasks, once);
-    // the sums come back by the kernel's stores
+    // The kernels' tasks go up by copies on the stream, the sums come back by the
+    // kernel's stores.
     int64_t parts = 1;
     for (int i = 1; i <= N; ++i)
         parts = std::max(parts, std::min<int64_t>((bra->dr(i) * ket->dr(i) + 1023) / 1024, 16));
@@ -405,6 +404,7 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
     StackTask* hst = reinterpret_cast<StackTask*>(h + nsum);
     DotTask* hdt = reinterpret_cast<DotTask*>(hst + st.size());
     std::copy(st.begin(), st.end(), hst);
+    unset(h, nsum);
     DBuf dst(ctx, sizeof(StackTask) * st.size()), ddt(ctx, sizeof(DotTask) * terms.size());
     TN_CHECK_CUDA(cudaMemcpyAsync(dst.p, hst, dst.bytes, cudaMemcpyHostToDevice, ctx->stream));
     for (size_t t = 0; t < st.size(); t += 65535) {
@@ -478,6 +478,7 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
     }
     TN_CHECK_CUDA(cudaGetLastError());
     ctx->sync();
+    check_set(h, nsum);
     for (size_t t = 0; t < terms.size(); ++t) {
         cplx v = sums[parts * t];
         for (int64_t k = 1; k < parts; ++k) v = cadd(v, sums[parts * t + k]);
