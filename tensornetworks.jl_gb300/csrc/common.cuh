@@ -119,6 +119,8 @@ struct Ctx {
         if (prof_on) ++prof[TN_PROF_CLASSES - 1].launches;  // class 7 counts every launch
     }
     double* pinned(size_t n);
+    bool reclaim();
+    bool told_oom = false;  // that a product had no room for its planes
 };
 
 // Words that a kernel stores in pinned memory for the host: cleared to a value that no

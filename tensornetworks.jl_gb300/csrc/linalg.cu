@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "mixed.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace tn {
@@ -19,6 +20,7 @@ namespace tn {
 DBuf::DBuf(Ctx* c, size_t b) : ctx(c), bytes(b) {
     if (b == 0) return;
     cudaError_t e = cudaMallocAsync(&p, b, c->stream);
+    if (e != cudaSuccess && c->reclaim()) e = cudaMallocAsync(&p, b, c->stream);
     if (e != cudaSuccess) {
         p = nullptr;
         bytes = 0;
@@ -48,9 +50,17 @@ void* Scratch::get(Ctx* ctx, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (buf.bytes < bytes) {
         buf.reset();
-        buf = DBuf(ctx, bytes + bytes / 4);
+        buf = DBuf(ctx, bytes + std::min<size_t>(bytes / 4, 64 << 20));
     }
     return buf.p;
+}
+
+// An allocation failed: the modular product's operand planes (four times its operands; the
+// next product takes them anew) and the pool's idle blocks go back.
+bool Ctx::reclaim() {
+    (void)cudaGetLastError();
+    s_tcz.buf.reset();
+    return cudaStreamSynchronize(stream) == cudaSuccess && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
 }
 
 double* Ctx::pinned(size_t n) {

@@ -339,10 +339,9 @@ static std::vector<cplx> inner_terms_serial(Ctx* ctx, const tn_mps* bra, const t
     return res;
 }
 
-std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
-                              const std::vector<Term>& terms) {
+static std::vector<cplx> inner_terms_blocks(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
+                                            const std::vector<Term>& terms) {
     const int N = ket->N, d = ket->d;
-    TN_REQUIRE(bra->N == N && bra->d == d, "GMPS must share the same properties.");
     // the operators that a term starts or, from two on, ends with, by site
     std::vector<std::vector<const cplx*>> lops(N + 2), rops(N + 2);
     auto index = [](std::vector<const cplx*>& v, const cplx* op) {
@@ -485,6 +484,17 @@ std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
         res[t] = cmul(terms[t].coeff, v);
     }
     return res;
+}
+
+std::vector<cplx> inner_terms(Ctx* ctx, const tn_mps* bra, const tn_mps* ket,
+                              const std::vector<Term>& terms) {
+    TN_REQUIRE(bra->N == ket->N && bra->d == ket->d, "GMPS must share the same properties.");
+    try {
+        return inner_terms_blocks(ctx, bra, ket, terms);
+    } catch (const Error& e) {
+        if (e.code != TN_ERR_OOM) throw;
+    }
+    return inner_terms_serial(ctx, bra, ket, terms);  // no room for all blocks at once
 }
 
 }  // namespace tn

@@ -845,7 +845,12 @@ bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx al
         base = static_cast<char*>(ctx->s_tcz.get(ctx, bA + bB + bQ + bH));
     } catch (const Error& e) {
         if (e.code != TN_ERR_OOM) throw;
-        return false;  // no room for the residue planes: the SIMT kernel needs none
+        // the FP64 kernels need no planes; up to thirty times slower, so it is said once
+        if (!ctx->told_oom)
+            fprintf(stderr, "tngpu: no room for %zu MB of residue planes, product of %lld x %lld x %lld on the FP64 units\n",
+                    (bA + bB + bQ + bH) >> 20, (long long)m, (long long)n, (long long)k);
+        ctx->told_oom = true;
+        return false;
     }
     unsigned* hmax = reinterpret_cast<unsigned*>(base + bA + bB + bQ);
     Side a{A, m, k, lda, (opa == OP_T || opa == OP_C) ? 1 : 0, (opa == OP_C || opa == OP_R) ? 1 : 0,
