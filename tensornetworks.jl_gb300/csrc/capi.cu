@@ -63,23 +63,21 @@ static thread_local std::string g_noctx_err;
     tn::Ctx* _c = (ctxptr);         \
     try {
 #define TN_API_END                                                  \
-    if (_c && _c->tc_pending) {                                     \
-        _c->tc_pending = false;                                     \
-        tn::tc_check_error(_c);                                     \
-    }                                                               \
     return TN_OK;                                                   \
     }                                                               \
     catch (const tn::Error& e) {                                    \
         if (_c) _c->err = e.what(); else g_noctx_err = e.what();    \
-        if (_c) { cudaGetLastError(); }                             \
+        if (_c) _c->forget();                                       \
         return e.code;                                              \
     }                                                               \
     catch (const std::bad_alloc&) {                                 \
+        if (_c) _c->forget();                                       \
         if (_c) _c->err = "host allocation failed";                 \
         else g_noctx_err = "host allocation failed";                \
         return TN_ERR_OOM;                                          \
     }                                                               \
     catch (const std::exception& e) {                               \
+        if (_c) _c->forget();                                       \
         if (_c) _c->err = e.what(); else g_noctx_err = e.what();    \
         return TN_ERR_INVALID;                                      \
     }

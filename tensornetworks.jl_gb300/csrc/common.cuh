@@ -89,8 +89,9 @@ struct Ctx {
     // FP64 DMRG: small splits and sums keep one order of operations, so that its
     // results are the same to the last bit in every version (eig_fp64.cu)
     bool ordered = false;
-    // a tensor-core kernel of the FP64 path ran since d_err was last read
-    bool tc_pending = false;
+    // pinned: set by a modular product whose bounded wait ran out, looked at after every
+    // host synchronisation (no result reaches the host without one)
+    int* h_err = nullptr;
     double* h_pinned = nullptr;  // small pinned staging area
     size_t h_pinned_n = 0;
     // kernel profiler: CUDA events around launches, per class
@@ -113,7 +114,15 @@ struct Ctx {
     std::vector<cudaEvent_t> ev_pool;
     cudaEvent_t ev_get();
     void prof_flush();  // resolves pending event pairs (synchronises)
-    void sync() { TN_CHECK_CUDA(cudaStreamSynchronize(stream)); }
+    void sync() {
+        TN_CHECK_CUDA(cudaStreamSynchronize(stream));
+        if (h_err && *(volatile int*)h_err) {
+            *h_err = 0;
+            throw Error(TN_ERR_TIMEOUT, "FP64 product: a bounded device wait ran out");
+        }
+    }
+    // after a failed call: its kernels end, and none of its error words stays
+    void forget() noexcept;
     void count() {
         ++launches;
         if (prof_on) ++prof[TN_PROF_CLASSES - 1].launches;  // class 7 counts every launch

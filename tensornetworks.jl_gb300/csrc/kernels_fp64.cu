@@ -743,7 +743,7 @@ __global__ void row_norms_kernel(const cplx* __restrict__ Y, int64_t k, int64_t 
 struct KeepDev {
     int64_t k;
     double total, discarded;
-    int64_t err;  // error words of the kernels before: grid barriers, tensor-core waits
+    int64_t err;  // the eigensolver's barriers ran out
 };
 
 __device__ inline double s2_at(const double* lam, int64_t n, int64_t i) {
@@ -756,7 +756,6 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
                                                          int64_t mindim, double* __restrict__ S_out,
                                                          const cplx* __restrict__ G, int64_t g,
                                                          const int* __restrict__ dinfo,
-                                                         const int* __restrict__ derr,
                                                          KeepDev* __restrict__ res) {
     __shared__ double wsum[32];
     __shared__ long long wcnt[32];
@@ -844,7 +843,7 @@ __global__ void __launch_bounds__(1024) keep_rule_kernel(const double* __restric
         res->k = k;
         res->total = total;
         res->discarded = total > 0 ? d / total : 0.0;
-        res->err = (dinfo ? *dinfo : 0) | *derr;
+        res->err = dinfo ? *dinfo : 0;
     }
 }
 
@@ -1175,19 +1174,16 @@ KeepResult keep_rule(Ctx* ctx, const double* dlam, int64_t n, int64_t sz, double
     // the trace is summed by a thread an entry where its last bit counts
     const unsigned threads = one_block(ctx->ordered ? std::max(sz, g) : sz);
     keep_rule_kernel<<<1, threads, 0, ctx->stream>>>(dlam, n, sz, cutoff, maxdim, mindim, dS, G, g,
-                                                  dinfo, ctx->d_err, dres);
+                                                  dinfo, dres);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
     ctx->sync();
     check_set(h, 4);
-    ctx->tc_pending = false;
     KeepDev r;
     memcpy(&r, h, sizeof(KeepDev));
     if (r.err != 0) {
-        if (dinfo)
-            TN_CHECK_CUDA(cudaMemsetAsync(const_cast<int*>(dinfo), 0, sizeof(int), ctx->stream));
-        TN_CHECK_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-        throw Error(TN_ERR_TIMEOUT, "truncated split: a bounded device wait ran out");
+        TN_CHECK_CUDA(cudaMemsetAsync(const_cast<int*>(dinfo), 0, sizeof(int), ctx->stream));
+        throw Error(TN_ERR_TIMEOUT, "eigensolver: a bounded barrier ran out");
     }
     return KeepResult{r.k, r.total, r.discarded};
 }

@@ -63,6 +63,15 @@ bool Ctx::reclaim() {
     return cudaStreamSynchronize(stream) == cudaSuccess && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
 }
 
+void Ctx::forget() noexcept {
+    if (!stream) return;
+    (void)cudaStreamSynchronize(stream);
+    if (h_err) *h_err = 0;
+    if (d_err) (void)cudaMemsetAsync(d_err, 0, sizeof(int), stream);
+    if (d_bar) (void)cudaMemsetAsync(d_bar, 0, 8 * sizeof(unsigned), stream);
+    (void)cudaGetLastError();
+}
+
 double* Ctx::pinned(size_t n) {
     if (h_pinned_n < n) {
         if (h_pinned) cudaFreeHost(h_pinned);
@@ -85,6 +94,8 @@ void ctx_init(Ctx& c, int device) {
     TN_CHECK_CUDA(cudaMemsetAsync(c.d_bar, 0, 8 * sizeof(unsigned), c.stream));
     TN_CHECK_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
     TN_CHECK_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
+    TN_CHECK_CUDA(cudaMallocHost(&c.h_err, sizeof(int)));
+    *c.h_err = 0;
     TN_CHECK_CUDA(cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device));
 }
 
@@ -102,6 +113,7 @@ void ctx_release(Ctx& c) {
     if (c.d_bar) cudaFree(c.d_bar);
     if (c.d_err) cudaFree(c.d_err);
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
+    if (c.h_err) cudaFreeHost(c.h_err);
     for (auto& r : c.prof_pending) {
         cudaEventDestroy(r.a);
         cudaEventDestroy(r.b);

@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(GEMM_T, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(TMEM_COLS));
     }
-    if (threadIdx.x == 0 && *(volatile int*)abort_flag) atomicExch(p.err, 1);
+    if (threadIdx.x == 0 && *(volatile int*)abort_flag) *(volatile int*)p.err = 1;  // host memory
 }
 
 // ---- reconstruction --------------------------------------------------------------
@@ -889,7 +889,7 @@ bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx al
     p.tiles = p.lower ? p.mt * (p.mt + 1) / 2 : p.mt * p.nt;
     p.q = reinterpret_cast<uchar2*>(base + bA + bB);
     p.ldq = ldq;
-    p.err = ctx->d_err;
+    p.err = ctx->h_err;
     TN_CHECK_CUDA(cudaFuncSetAttribute(zmod_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        SMEM_BYTES));
     const int grid = std::min(NP * p.tiles, ctx->sm_count);
@@ -904,7 +904,6 @@ bool zgemm_tc(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx al
                   ctx->stream>>>(o, a, b);
     ctx->count();
     TN_CHECK_CUDA(cudaGetLastError());
-    ctx->tc_pending = true;
     return true;
 }
 

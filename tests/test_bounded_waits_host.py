@@ -19,3 +19,29 @@ def test_warps_leave_as_a_whole(name, pattern):
     assert waits
     for at in waits:
         assert src[:at].endswith("__all_sync(0xffffffffu, ")
+
+
+def _read(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return f.read()
+
+
+def test_a_failed_call_leaves_no_error_word():
+    """Every way out of a C entry by an exception ends the call's kernels and clears their
+    error words, so that the next call does not report them as its own."""
+    end = re.search(r"#define TN_API_END(.*?)\n\n", _read("capi.cu"), re.S).group(1)
+    catches = re.split(r"catch \(", end)[1:]
+    assert len(catches) == 3
+    for c in catches:
+        assert "_c->forget()" in c
+
+
+def test_results_reach_the_host_through_the_checked_wait():
+    """A modular product's error word is looked at in Ctx::sync; no entry waits for the stream
+    in another way before it hands results out (two destructors wait and return nothing)."""
+    assert "h_err" in re.search(r"void sync\(\) \{(.*?)\n    \}", _read("common.cuh"), re.S).group(1)
+    assert "cudaStreamSynchronize" not in re.search(r"#define TN_API_END(.*?)\n\n", _read("capi.cu"), re.S).group(1)
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith(".cu") and name not in ("linalg.cu", "capi.cu"):
+            assert "cudaStreamSynchronize" not in _read(name), name
+    assert _read("capi.cu").count("cudaStreamSynchronize") == 2
