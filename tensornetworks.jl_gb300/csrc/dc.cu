@@ -310,7 +310,7 @@ __device__ __forceinline__ void find_root(const double* ds, const double* zz, in
     // FP64: Newton on x f(x), which has no pole at the origin, inside the bracket
     // that the signs give.  Steps are compared by their exponents relative to m.
     double m = fmin((double)__uint_as_float(bl + (bh - bl) / 2), half), ml = 0.0, mh = half * 1.001;
-    int before = -20;
+    int before = -20, jumps = 0;
     bool done = false;
     for (int it = 0; it < 48; ++it) {
         const double x = sg * m;
@@ -322,7 +322,12 @@ __device__ __forceinline__ void find_root(const double* ds, const double* zz, in
             const int em = expo(m), st = expo(mn - m) - em;
             const bool noise = expo(f) <= ilogbf(fa) - 51;  // rounding of the sum
             const ll im = __double_as_longlong(mn);
-            if ((im > __double_as_longlong(ml) && im < __double_as_longlong(mh) && st <= -3) || st <= -21) {
+            const bool inside = im > __double_as_longlong(ml) && im < __double_as_longlong(mh);
+            // far below m, where FP32 could not follow the root to its pole, the function
+            // is a line and one long step gets there
+            const bool jump = inside && im < __double_as_longlong(m) && !noise && jumps < 3;
+            if ((inside && st <= -3) || st <= -21 || jump) {
+                jumps += st > -3;
                 m = mn;
                 // converged, or the next step would be (its error is the cube of
                 // this over the square of the last), or as near as the sum allows
