@@ -79,8 +79,9 @@ TN_HD void update(zint& a, int4 wi, int4 vi, int4 wl, int4 vl) {
 }
 
 // Running sum of a v over a row: high products (which may wrap: only the final
-// sum has to fit) and cross products (bounded by Cauchy-Schwarz below 2^63 for
-// a 32nd of any row up to 4096 entries).
+// sum has to fit), cross products (bounded by Cauchy-Schwarz below 2^63 for
+// a 32nd of any row up to 4096 entries) and low products (2^57 an entry whatever the
+// row: dot_carry moves their upper part on after at most 32 entries).
 struct Dot {
     ll mx, my, cx, cy, lx, ly;
 };
@@ -90,6 +91,12 @@ TN_HD void dot_add(Dot& s, zint a, int4 v) {
     s.mx = mw(-l.z, v.z, s.mx), s.cx = mw(-l.z, v.w, s.cx), s.cx = mw(-l.w, v.z, s.cx), s.lx = mw(-l.w, v.w, s.lx);
     s.my = mw(l.x, v.z, s.my), s.cy = mw(l.x, v.w, s.cy), s.cy = mw(l.y, v.z, s.cy), s.ly = mw(l.y, v.w, s.ly);
     s.my = mw(l.z, v.x, s.my), s.cy = mw(l.z, v.y, s.cy), s.cy = mw(l.w, v.x, s.cy), s.ly = mw(l.w, v.y, s.ly);
+}
+TN_HD void dot_carry(Dot& s) {
+    s.cx += s.lx >> 29;
+    s.lx &= (1ll << 29) - 1;
+    s.cy += s.ly >> 29;
+    s.ly &= (1ll << 29) - 1;
 }
 TN_HD zint dot_value(const Dot& s) {  // unit 2^-61 F
     return zint{(ll)((ull)s.mx << 5) + ((s.cx + (s.lx >> 29) + (1ll << 23)) >> 24),

@@ -477,7 +477,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                     dot_add(s, x, vD[l]);
                 };
                 zint x0 = a[min(l, n - 1)], x1 = a[min(l + 32, n - 1)];
-                for (; l - lane < n; l += dl) {
+                for (int t = 0; l - lane < n; l += dl, ++t) {
+                    if (FORM == GRID_GLOBAL && (t & 15) == 15) dot_carry(s);  // others: up to 36 entries in all
                     const zint y0 = a[min(l + dl, n - 1)], y1 = a[min(l + dl + 32, n - 1)];
                     one(x0, l);
                     one(x1, l + 32);

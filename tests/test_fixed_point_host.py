@@ -1,0 +1,51 @@
+"""The reduction's running sums on the CPU (csrc/fixp.cuh compiles for both): a lane's 128
+products at order 4096, with every low limb at its largest and of one sign, against exact
+integers; one unit for the rounding of the sum and one for the parts carried on."""
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "tensornetworks.jl_gb300", "csrc")
+
+SOURCE = r"""
+#include "fixp.cuh"
+using namespace tn::fixp;
+int main() {
+    int bad = 0;
+    unsigned long long r = 88172645463325252ull;
+    auto rnd = [&] { r ^= r << 13; r ^= r >> 7; r ^= r << 17; return r; };
+    for (int trial = 0; trial < 2000; ++trial) {
+        Dot s{0, 0, 0, 0, 0, 0};
+        i128 ex = 0, ey = 0;
+        const ll al = trial % 3 == 0 ? (1ll << 28) - 1 : trial % 3 == 1 ? -(1ll << 28) : (ll)(rnd() >> 36) - (1ll << 27);
+        for (int t = 0; t < 128; ++t) {
+            const ll hi = (ll)(rnd() >> 40) - (1ll << 23), vh = (ll)(rnd() >> 43) - (1ll << 20);
+            // entries in units of 2^-61 (their limbs hold the upper 61 bits but three), v 2^-56
+            const zint a{((hi << 29) + al) * 8, ((vh << 29) + al) * 8}, v{(vh << 29) + al, (hi % 1048576 << 29) - al};
+            dot_add(s, a, limbs29(v));
+            if ((t & 31) == 31) dot_carry(s);
+            ex += (i128)a.x * v.x - (i128)a.y * v.y;
+            ey += (i128)a.x * v.y + (i128)a.y * v.x;
+        }
+        const zint p = dot_value(s);
+        const i128 dx = ((i128)p.x << 56) - ex, dy = ((i128)p.y << 56) - ey, tol = (i128)2 << 56;
+        bad += dx > tol || dx < -tol || dy > tol || dy < -tol;
+    }
+    printf("%d\n", bad);
+    return 0;
+}
+"""
+
+
+def test_low_limbs_of_one_sign(tmp_path):
+    nvcc = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    src, exe = tmp_path / "dot.cu", tmp_path / "dot"
+    src.write_text(SOURCE)
+    subprocess.run([nvcc, "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, str(src), "-o", str(exe)], check=True,
+                   capture_output=True)
+    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "0\n"
