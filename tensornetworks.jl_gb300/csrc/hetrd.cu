@@ -593,7 +593,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                     const zint v = zsft(x, shf - d);
                     p.o.V[(size_t)j * n + l] = cmk(unit56(v.x), unit56(v.y));
                 }
-                vm = max(vm, max(bits64(x.x), bits64(x.y)) + shf - 2 * d - 56);
+                const int bits = max(bits64(x.x), bits64(x.y));
+                if (bits) vm = max(vm, bits + shf - 2 * d - 56);  // zeros have no size, whatever the shift
             }
             vm = __reduce_max_sync(0xffffffffu, vm);
             if (lane == 0) atomicMax(&sh.vm[j % 3], vm);
