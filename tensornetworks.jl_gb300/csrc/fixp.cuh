@@ -127,7 +127,6 @@ TN_HD ll prod1(const Prod& p, int s) {
 TN_HD ll prod2(const Prod& p, int s) {
     return (ll)((ull)p.m << (64 - s)) + ((p.x + (p.l >> 31) + (1ll << (s - 33))) >> (s - 32));
 }
-TN_HD limb32 neg(limb32 a) { return limb32{-a.h, -a.l}; }
 
 // x 2^s (s negative: rounded), componentwise; zero beyond |s| = 62 (upwards only a
 // zero gets there)
@@ -164,7 +163,8 @@ TN_HD ll re_dot(zint v, zint p) {
 // w = tau p - al v: tau in units of 2^-59, al 2^-57, p 2^-61 F, v 2^-56; w 2^-57 F
 TN_HD zint make_w(zint tau, zint p, ll al, zint v) {
     const limb32 tx = split32(tau.x), ty = split32(tau.y), px = split32(p.x), py = split32(p.y), la = split32(al);
-    return zint{prod2(mul32(tx, px, mul32(neg(ty), py)), 63) - prod1(mul32(split32(v.x), la), 56),
+    const limb32 ny = split32(-tau.y);  // not ty's limbs negated: the lower one may be -2^31
+    return zint{prod2(mul32(tx, px, mul32(ny, py)), 63) - prod1(mul32(split32(v.x), la), 56),
                 prod2(mul32(tx, py, mul32(ty, px)), 63) - prod1(mul32(split32(v.y), la), 56)};
 }
 

@@ -40,12 +40,36 @@ int main() {
 """
 
 
-def test_low_limbs_of_one_sign(tmp_path):
+def build(src, exe):
     nvcc = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("no nvcc")
+    subprocess.run([nvcc, "-O2", "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True, capture_output=True)
+
+
+def test_low_limbs_of_one_sign(tmp_path):
     src, exe = tmp_path / "dot.cu", tmp_path / "dot"
     src.write_text(SOURCE)
-    subprocess.run([nvcc, "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, str(src), "-o", str(exe)], check=True,
-                   capture_output=True)
+    build(src, exe)
     assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "0\n"
+
+
+def test_a_limb_that_has_no_negative(tmp_path):
+    """make_w with the lower limb of tau's imaginary part at -2^31, against exact integers."""
+    src, exe = tmp_path / "w.cu", tmp_path / "w"
+    src.write_text(r"""
+#include "fixp.cuh"
+using namespace tn::fixp;
+int main() {
+    const zint tau{(1ll << 60) - 12345, (1ll << 60) - (1ll << 31)}, p{(3ll << 55) + 77, (1ll << 57) + 5}, v{1ll << 49, 3ll << 48};
+    const ll al = (1ll << 58) + 9;
+    const zint w = make_w(tau, p, al, v);
+    const i128 x = (i128)tau.x * p.x - (i128)tau.y * p.y, y = (i128)tau.x * p.y + (i128)tau.y * p.x;
+    const ll wx = (ll)(x >> 63) - (ll)((i128)al * v.x >> 56), wy = (ll)(y >> 63) - (ll)((i128)al * v.y >> 56);
+    printf("%d\n", llabs(w.x - wx) <= 4 && llabs(w.y - wy) <= 4);
+    return 0;
+}
+""")
+    build(src, exe)
+    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "1\n"
