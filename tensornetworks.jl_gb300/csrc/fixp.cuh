@@ -10,11 +10,11 @@
 // eigenvalues need every entry to that scale's precision, as FP64 keeps it.  Row l
 // therefore has an exponent e_l >= 0 that keeps its scaled diagonal at 1/2 or
 // below; all quantities below are bounded by that (Cauchy-Schwarz), and with
-// F >= |A|_F a power of two their units are
+// F >= |A|_F a power of two their units are (m = min e less guard_bits)
 //   entries             A_il 2^(e_i + e_l)                     2^-61 F
 //   column              x_l 2^(e_l + c)                        2^-61 F
 //   reflector v, |column| scaled to [1/2, 1)                   2^-56
-//   product             p_l 2^(e_l + m), p = A v, m = min e    2^-61 F
+//   product             p_l 2^(e_l + m), p = A v               2^-61 F
 //   v^H p               2^(2 m)                                2^-60 F
 //   update vectors      v_l 2^(e_l + h - m), h = log2 sqrt(v^H p)   2^-56
 //                       w_l 2^(e_l - h + m)                    2^-57 F
@@ -243,10 +243,10 @@ TN_HD unsigned norm_carry(unsigned l, unsigned below) { return l + (below >> 22)
 TN_HD int norm_shift(int bl) { return 56 - ((bl - 56 + 401) / 2 - 200); }
 
 // The new exponent of a row from its scaled diagonal a before the update and the
-// float estimates d of 2 Re(w conj v), b of 2 |w||v| and v2 of |v|^2 in the same
-// scale: unchanged while the larger of the diagonals before and after and v2 / 32
-// lies in [2^-14, 1/2], else such that it is at most 1/4, and never above cap.
-// v2 matters where q is below its floor only.
+// float estimates d of 2 Re(w conj v), b of 2 |w||v| and v2 of the larger of |v|^2 and
+// |w|^2 in the same scale: unchanged while the larger of the diagonals before and after
+// and v2 / 32 lies in [2^-14, 1/2], else such that it is at most 1/4, and never above cap.
+// v2 matters where q is below its floor or the row holds rounding errors only.
 constexpr int EXP_MAX = 28;   // 2^-56 F on the diagonal
 constexpr int EXP_GAIN = 18;  // a row's rounding errors stay 2^-20 of its scale
 TN_HD int next_exponent(int e, int cap, float a, float d, float b, float v2) {
@@ -273,14 +273,20 @@ TN_HD int bits64(ll x) {  // of |x|
 #endif
 }
 
-// h = log2 sqrt(q), q = v^H A v in units of 2^-60, with the floor that rounding
-// errors of the product need, from the largest entry 2^vm of v 2^-e.
+// h = log2 sqrt(q) of the largest that v^H A v can be, q in units of 2^-60 and off by
+// two of them a row at most (a q that rounds to zero says nothing of p, which is
+// bounded by sqrt of the true one), with the floor that rounding errors of the
+// product need, from the largest entry 2^vm of v 2^-e.
+// Rows' exponents bound the scaled matrix' diagonal, not its norm, which can be the sum of
+// n of them; v^H A v 2^(2 m) and the product stay in range with m this much below the
+// smallest exponent (4^g >= n / 2, and none where that is zero: |A| is below F).
+TN_HD int guard_bits(int n) { return bits64(n - 1) / 2; }
 constexpr int Q_FLOOR = 12;
-TN_HD int q_exponent(ll q, int vm) {
-    const int lo = vm - Q_FLOOR;
-    if (q <= 0) return lo;
-    const int h = (bits64(q) - 61) >> 1;
-    return h < lo ? lo : h;
+// Where rows hold nothing but rounding errors the matrix is not positive, and p, of at most
+// pm bits, has to bound h itself.
+TN_HD int q_exponent(ll q, int vm, int pm, int n) {
+    const int lo = vm - Q_FLOOR, h = (bits64((q > 0 ? q : 0) + 4ll * n) - 61) >> 1, hp = pm - 62;
+    return h > lo ? (h > hp ? h : hp) : lo > hp ? lo : hp;
 }
 // al = |tau|^2 / 2 q 2^(-2 h), unit 2^-57, from |tau|^2 / 2 in units of 2^-59
 TN_HD ll q_scaled(ll c2, ll q, int h) { return prod1(mul32(split32(c2), split32(sft(q, -2 * h))), 62); }

@@ -68,6 +68,7 @@ struct TrdIn {
     zint* ma;
     ll* md;
     ull* mq;          // grid form: v^H A v, triple buffered by step
+    int* mx;          // grid form: the products' largest number of bits, likewise
     zint* xr;         // rows in global memory: a block's copy of the column
     unsigned* part;   // grid form: per-block scale partials
     unsigned* bar;    // grid form: arrival counter (zero at launch)
@@ -126,11 +127,12 @@ __device__ __forceinline__ ll warp_sum64(ll v) {
 }
 
 struct ShCtl {
-    ull q;               // grid form: the block's share of v^H A v
+    ull q;               // grid form: the block's share of v^H A v, its rows' largest product
+    int pm;
     zint sum[HROWS];     // products of row segments with v
     zint first[HROWS];   // rows' entries of column j+1
     ll diag[HROWS];
-    ll qt[2][8 * HC];    // cluster form: every warp's share, from every block
+    alignas(16) zint qt[2][8 * HC];  // cluster form: every warp's share and largest product, from every block
     uint64_t mbar[2];    // cluster form: a step's exchange has arrived
     int abort;
     unsigned S[3][NORM_LIMBS];  // squared norm, limbs, triple buffered by step
@@ -204,11 +206,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
     if (tid == 0) {
         sh.abort = 0;
         sh.q = 0;
+        sh.pm = 0;
         for (int k = 0; k < 3; ++k) {
             sh.emin[k] = INT_MAX;
             sh.vm[k] = INT_MIN;
             sh.shift[k] = 0;
-            if (GRID && b == 0) p.mq[k] = 0;
+            if (GRID && b == 0) p.mq[k] = 0, p.mx[k] = 0;
         }
         if (!GRID) {  // seen by the others after the cluster barrier below
             for (int k = 0; k < 2; ++k)
@@ -395,6 +398,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
         em = sh.em;
         c = sh.c;
         const int l0 = j + 1, s0 = ee[l0] - em;  // first row left
+        const int gb = p.psd ? min(em, guard_bits(n - j)) : 0;
         const int cn = max(0, em - 6);  // its new exponent: its diagonal is at most the trace, n 2^(-2 em)
         const int buf = j & 1, nb = (j + 1) % 3;
         if (warp == RW) {
@@ -420,7 +424,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                 if (!GRID)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                      (uint32_t)__cvta_generic_to_shared(&sh.mbar[buf])),
-                                 "r"(40 * (n - j - 1) + 8 * RW * C)
+                                 "r"(40 * (n - j - 1) + 16 * RW * C)
                                  : "memory");
                 ar = scale2(__ll2double_rn(al.x), -56);
                 ai = scale2(__ll2double_rn(al.y), -56);
@@ -456,7 +460,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
             if (sh.abort) break;
         } else {
             // column -> v's limbs for the products (the first entry still alpha)
-            for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em)));
+            for (int l = l0 + tid; l < n; l += HM) vD[l] = limbs29(zsft(xr[l], shf - 2 * (ee[l] - em) - gb));
             __syncwarp();
             bar_named(1, HM);
             // ---- A. rows: pending update, product with v ------------------------
@@ -511,9 +515,11 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                 bar_named(2, HT);  // beta and the first entry of v
                 const int io = w0 + RW * C * lane;
                 ll q = 0;
+                int pm = 0;
                 if (lane < k) {
-                    P = minus_real(P, Aj, sh.beta, s0);
-                    q = re_dot(io == l0 ? zsft(sh.v1, -s0) : value29(vD[io]), P);
+                    P = minus_real(P, Aj, sh.beta, s0 + gb);
+                    pm = max(bits64(P.x), bits64(P.y));
+                    q = re_dot(io == l0 ? zsft(sh.v1, -s0 - gb) : value29(vD[io]), P);
                 }
                 // every warp sends its share of q, rows or not: a block that has
                 // everybody's share knows that nobody reads the buffer it will
@@ -531,7 +537,8 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                         st_async(rmd + 8 * ir, dr, rbar + 8 * buf);
                     }
                 }
-                if (lane < C) st_async(rqt + 8 * (8 * HC * buf + RW * b + warp), qs, rbar + 8 * buf);
+                pm = __reduce_max_sync(0xffffffffu, pm);
+                if (lane < C) st_async(rqt + 16 * (8 * HC * buf + RW * b + warp), zint{qs, pm}, rbar + 8 * buf);
             } else {
                 // Local row r is matrix row i0 + C r; 2^ls warps share a row while there
                 // are more warps than rows (a warp alone on its scheduler takes 1,900
@@ -557,6 +564,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                 }
                 bar_named(2, HT);  // the rows' sums; beta and the first entry of v
                 ll qs = 0;
+                int pm = 0;
                 for (int r = warp; r < nrows; r += RW) {  // a warp finishes a row
                     const int i = i0 + C * r, ir = buf * n + i;
                     zint P{0, 0};
@@ -565,27 +573,33 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                         P = zint{P.x + u.x, P.y + u.y};
                     }
                     const zint Aj = sh.first[r];
-                    P = minus_real(P, Aj, sh.beta, s0);
+                    P = minus_real(P, Aj, sh.beta, s0 + gb);
                     if (lane == 0) {
                         mp[ir] = P;
                         ma[ir] = Aj;
                         md[ir] = sh.diag[r];
                     }
-                    qs += re_dot(i == l0 ? zsft(sh.v1, -s0) : value29(vD[i]), P);
+                    pm = max(pm, max(bits64(P.x), bits64(P.y)));
+                    qs += re_dot(i == l0 ? zsft(sh.v1, -s0 - gb) : value29(vD[i]), P);
                 }
-                if (qs && lane == 0) atomicAdd(&sh.q, (ull)qs);
+                if (lane == 0) {
+                    if (qs) atomicAdd(&sh.q, (ull)qs);
+                    if (pm) atomicMax(&sh.pm, pm);
+                }
                 __syncwarp();
                 bar_named(1, HM);
                 arrivals += (unsigned)C;
                 if (tid == 0) {
                     atomicAdd(p.mq + j % 3, sh.q);
+                    if (sh.pm) atomicMax(p.mx + j % 3, sh.pm);
                     sh.q = 0;
+                    sh.pm = 0;
                     grid_arrive(p.bar);
                 }
             }
             // while the results travel: v for the back-transformation, the largest
             // entry of v 2^-e
-            int vm = -s0;
+            int vm = -s0 - gb;
             for (int l = l0 + tid; l < n; l += HM) {
                 const int d = ee[l] - em;
                 const zint x = xr[l];
@@ -594,7 +608,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                     p.o.V[(size_t)j * n + l] = cmk(unit56(v.x), unit56(v.y));
                 }
                 const int bits = max(bits64(x.x), bits64(x.y));
-                if (bits) vm = max(vm, bits + shf - 2 * d - 56);  // zeros have no size, whatever the shift
+                if (bits) vm = max(vm, bits + shf - 2 * d - gb - 56);  // zeros have no size, whatever the shift
             }
             vm = __reduce_max_sync(0xffffffffu, vm);
             if (lane == 0) atomicMax(&sh.vm[j % 3], vm);
@@ -602,7 +616,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
             if (GRID) {
                 if (tid == 0) {
                     if (!grid_wait(p.bar, p.err, arrivals)) sh.abort = 1;
-                    if (b == 0) p.mq[(j + 2) % 3] = 0;  // every block has read step j - 1's
+                    if (b == 0) p.mq[(j + 2) % 3] = 0, p.mx[(j + 2) % 3] = 0;  // every block has read step j - 1's
                 }
             } else if (!mbar_wait(&sh.mbar[buf], (uint32_t)(j >> 1) & 1u)) {
                 sh.abort = 1;
@@ -627,21 +641,28 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                 df = GRID ? __ldcg(md + o) : md[o];
             }
             ll q = 0;
+            int pm = 0;
             if (GRID) {
                 q = (ll)__ldcg(p.mq + j % 3);
+                pm = __ldcg(p.mx + j % 3);
             } else {  // every warp adds all shares itself
 #pragma unroll
                 for (int t = 0; t < RW * HC; t += 32)
-                    if (t + lane < RW * C) q += sh.qt[buf][t + lane];
+                    if (t + lane < RW * C) {
+                        const zint s = sh.qt[buf][t + lane];
+                        q += s.x;
+                        pm = max(pm, (int)s.y);
+                    }
                 q = warp_sum64(q);
+                pm = __reduce_max_sync(0xffffffffu, pm);
             }
             // h = log2 sqrt(v^H A v): w and v scaled by its powers stay bounded
-            const int h = p.psd ? q_exponent(q, sh.vm[j % 3]) : 0;
+            const int h = p.psd ? q_exponent(q, sh.vm[j % 3], pm, n - j) : 0;
             const ll al2 = q_scaled(sh.c2, q, h);
             const zint tau = sh.tau;
             // float copies for the exponents' estimate
             const float tx = (float)(int)(tau.x >> 32) * 0x1p-27f, ty = (float)(int)(tau.y >> 32) * 0x1p-27f;
-            const float fp = __int_as_float((127 - 61 - h) << 23), fv = __int_as_float((127 + shf + h - 56) << 23);
+            const float fp = __int_as_float((127 - 61 - h) << 23), fv = __int_as_float((127 + shf + h + gb - 56) << 23);
             const float fa = (float)(int)(al2 >> 32) * 0x1p-25f, ft = fabsf(tx) + fabsf(ty);
             int emn = INT_MAX, any = 0;
             for (int l = l0 + tid; l < n; l += HM) {
@@ -657,11 +678,11 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                     const float av = fabsf(vx) + fabsf(vy);
                     const float a = __ll2float_rn(l == l0 + tid ? df : GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
                     en = next_exponent(el, cap[l], a, 2.f * (wx * vx + wy * vy),
-                                       2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), vx * vx + vy * vy);
+                                       2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), fmaxf(vx * vx + vy * vy, wx * wx + wy * wy));
                     if (top) en = cn;  // its row becomes column j+1
                 }
                 const int d = en - el;
-                const zint vt = zsft(top ? sh.v1 : x, top ? cn + h - em : shf + h + d);
+                const zint vt = zsft(top ? sh.v1 : x, (top ? cn + h - em : shf + h + d) + gb);
                 wU[l] = limbs31(make_w(tau, zsft(pl, d - h), al2, vt));
                 vU[l] = limbs29(vt);
                 ee[l] = (signed char)en;
@@ -807,6 +828,7 @@ void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, 
     a.bar = ctx->d_bar;
     if (grid) {
         a.mq = reinterpret_cast<ull*>(take(256));
+        a.mx = reinterpret_cast<int*>(a.mq + 4);
         a.mp = reinterpret_cast<zint*>(take(nz));
         a.ma = reinterpret_cast<zint*>(take(nz));
         a.md = reinterpret_cast<ll*>(take(2 * n8));

@@ -1,6 +1,12 @@
-"""The reduction's running sums on the CPU (csrc/fixp.cuh compiles for both): a lane's 128
-products at order 4096, with every low limb at its largest and of one sign, against exact
-integers; one unit for the rounding of the sum and one for the parts carried on."""
+"""The reduction's fixed-point arithmetic on the CPU (csrc/fixp.cuh compiles for both).
+
+Running sums: a lane's 128 products at order 4096, with every low limb at its largest and of
+one sign, against exact integers; one unit for the rounding of the sum and one for the
+parts carried on.
+
+The whole reduction (host/reduction.cu has its steps): random positive semidefinite matrices
+with sectors, zeros, rank deficiency, grading and rounding-size entries keep a backward error
+of 64 n 2^-53 and stay within the range of their integers."""
 
 import os
 import shutil
@@ -51,6 +57,51 @@ def build(src, exe):
 def test_low_limbs_of_one_sign(tmp_path):
     src, exe = tmp_path / "dot.cu", tmp_path / "dot"
     src.write_text(SOURCE)
+    build(src, exe)
+    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "0\n"
+
+
+@pytest.fixture(scope="module")
+def reduction(tmp_path_factory):
+    exe = tmp_path_factory.mktemp("reduction") / "reduction"
+    build(os.path.join(os.path.dirname(os.path.abspath(__file__)), "host", "reduction.cu"), exe)
+    return exe
+
+
+@pytest.mark.parametrize("count,order,flat", [(150000, 6, 0), (150000, 12, 1), (1500, 60, 1), (40, 300, 1)])
+def test_backward_error(reduction, count, order, flat):
+    out = subprocess.run([str(reduction), "1", str(count), str(order), str(flat)], check=True, capture_output=True, text=True)
+    assert out.stdout.startswith("0 of "), out.stdout
+
+
+@pytest.mark.parametrize("n", [3, 8, 40, 150, 300])
+def test_equal_rows(reduction, n):
+    """Rows that are all alike below a larger one: the norm of what is left is the sum of its
+    diagonal, while every row's exponent goes by its own."""
+    out = subprocess.run([str(reduction), str(n)], check=True, capture_output=True, text=True)
+    assert out.stdout == "0 of 7\n"
+
+
+def test_scale_of_a_product_that_rounds_to_zero(tmp_path):
+    """q_exponent from v^H A v known to two units a row: the root of the true value, and so the
+    update vectors, stay within a factor of two of the scale."""
+    src, exe = tmp_path / "q.cu", tmp_path / "q"
+    src.write_text(r"""
+#include "fixp.cuh"
+using namespace tn::fixp;
+int main() {
+    int bad = 0;
+    for (int n = 2; n <= 4096; n = 2 * n - 1)
+        for (int k = 0; k < 62; ++k)
+            for (ll off = -2; off <= 2; ++off) {
+                const ll q = k ? 1ll << (k - 1) : 0;
+                const int h = q_exponent(q + off * n, -1000, 0, n);
+                bad += ldexp((double)q, -60) > 4.0 * ldexp(1.0, 2 * h);
+            }
+    printf("%d\n", bad);
+    return 0;
+}
+""")
     build(src, exe)
     assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "0\n"
 

@@ -78,6 +78,23 @@ def test_splits(tn, lo, hi, count, direction):
         assert np.linalg.norm(A - X @ Y) ** 2 <= tail + 2 * k * tol * top ** 2, (it, m, n, k)
 
 
+@pytest.mark.parametrize("n", [3, 20, 60, 150, 300, 1200])
+@pytest.mark.parametrize("s", [1e-1, 1e-2, 1e-4])
+def test_equal_rows(tn, n, s):
+    """Rows that are all alike beside a larger one: two singular values, each to 64 n 2^-52."""
+    ctx = tn.context()
+    A = np.zeros((n, 2), complex)
+    A[0, 0], A[1:, 1] = np.sqrt(n), s
+    th = np.asfortranarray(A)
+    X, Y, S, k = np.zeros(2 * n, complex), np.zeros(4, complex), np.zeros(2), C.c_int64(2)
+    t = tn._lib.trunc(0.0, 2, 1)
+    ctx.check(ctx.lib.tn_truncate(ctx.h, n, 2, dp(th), C.byref(t), 0, dp(X), dp(Y), dp(S), C.byref(k)))
+    assert k.value == 2
+    tol = 64 * n * EPS
+    assert np.abs(S - [np.sqrt(n), s * np.sqrt(n - 1)]).max() <= tol * np.sqrt(n)
+    assert np.abs(X.reshape((n, 2), order="F") @ Y.reshape((2, 2), order="F") - A).max() <= tol * np.sqrt(n)
+
+
 @pytest.mark.parametrize("seed", range(8))
 def test_quench_from_a_product_state(tn, seed):
     N, dt, steps = 10, 0.05, 6
