@@ -244,7 +244,7 @@ TN_HD int norm_shift(int bl) { return 56 - ((bl - 56 + 401) / 2 - 200); }
 
 // The new exponent of a row from its scaled diagonal a before the update and the
 // float estimates d of 2 Re(w conj v), b of 2 |w||v| and v2 of the larger of |v|^2 and
-// |w|^2 in the same scale: unchanged while the larger of the diagonals before and after
+// 2 |w|^2 in the same scale: unchanged while the larger of the diagonals before and after
 // and v2 / 32 lies in [2^-14, 1/2], else such that it is at most 1/4, and never above cap.
 // v2 matters where q is below its floor or the row holds rounding errors only.
 constexpr int EXP_MAX = 28;   // 2^-56 F on the diagonal

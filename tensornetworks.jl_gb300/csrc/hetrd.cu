@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS<FORM> + 32) hetrd_fix_kernel(Tr
                     const float av = fabsf(vx) + fabsf(vy);
                     const float a = __ll2float_rn(l == l0 + tid ? df : GRID ? __ldcg(md + off + l) : md[off + l]) * 0x1p-61f;
                     en = next_exponent(el, cap[l], a, 2.f * (wx * vx + wy * vy),
-                                       2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), fmaxf(vx * vx + vy * vy, wx * wx + wy * wy));
+                                       2.f * av * (ft * (fabsf(px) + fabsf(py)) + fa * av), fmaxf(vx * vx + vy * vy, 2.f * (wx * wx + wy * wy)));
                     if (top) en = cn;  // its row becomes column j+1
                 }
                 const int d = en - el;

@@ -2,11 +2,13 @@
 // (csrc/fixp.cuh), and their backward error on random positive semidefinite matrices
 // of the kinds that truncated splits meet.
 //   reduction <order>: n beside s in every other place, s = 10^-2 .. 10^-8, likewise
+//   reduction file <path>: a matrix, its order and lower triangle by rows
 //   reduction <seed> <matrices> <largest order> <flat>: prints how many are off by more
 //   than 64 n 2^-53 of the norm or leave the numbers' range, and the largest error
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstdio>
 #include <cstdlib>
 #include <random>
 #include <vector>
@@ -124,7 +126,7 @@ static Reduced reduce(const std::vector<C>& G, int n) {
             const float wx = tx * px - ty * py - fa * vx, wy = tx * py + ty * px - fa * vy, av = std::fabs(vx) + std::fabs(vy);
             en[l] = l == l0 ? cn
                             : next_exponent(e[l], cap[l], (float)unfix(dg[l], -61), 2.f * (wx * vx + wy * vy),
-                                            2.f * av * (ft * (std::fabs(px) + std::fabs(py)) + fa * av), std::max(vx * vx + vy * vy, wx * wx + wy * wy));
+                                            2.f * av * (ft * (std::fabs(px) + std::fabs(py)) + fa * av), std::max(vx * vx + vy * vy, 2.f * (wx * wx + wy * wy)));
             dl[l] = en[l] - e[l];
             const zint vt = zsft(l == l0 ? v1 : x[l], (l == l0 ? cn + h - em : sh + h + dl[l]) + g);
             const zint w = make_w(tau, zsft(p[l], dl[l] - h), al2, vt);
@@ -181,6 +183,23 @@ static bool off(const Reduced& r, double err, int n) {
 }
 
 int main(int argc, char** argv) {
+    if (argc == 3) {  // a matrix from a file: its order and lower triangle by rows
+        FILE* f = std::fopen(argv[2], "r");
+        int n = 0;
+        if (!f || std::fscanf(f, "%d", &n) != 1) return 1;
+        std::vector<C> P((size_t)n * n);
+        for (int i = 0; i < n; ++i)
+            for (int l = 0; l <= i; ++l) {
+                double x, y;
+                if (std::fscanf(f, "%la %la", &x, &y) != 2) return 1;
+                P[i + (size_t)n * l] = C(x, y);
+                P[l + (size_t)n * i] = C(x, -y);
+            }
+        std::fclose(f);
+        const Reduced r = reduce(P, n);
+        printf("%d of 1, p %.2f\n", (int)off(r, backward(P, n, r), n), r.pmax);
+        return 0;
+    }
     if (argc == 2) {
         const int n = std::atoi(argv[1]);
         int bad = 0;

@@ -82,6 +82,14 @@ def test_equal_rows(reduction, n):
     assert out.stdout == "0 of 7\n"
 
 
+def test_products_of_rows_left_small(reduction):
+    """A 12-row matrix whose update raises a row's products by more than |w|^2 says: they
+    have to stay within their range of four (4.004 where the exponents minded |w|^2 once)."""
+    case = os.path.join(os.path.dirname(os.path.abspath(__file__)), "host", "lifted_products.txt")
+    out = subprocess.run([str(reduction), "file", case], check=True, capture_output=True, text=True)
+    assert out.stdout.startswith("0 of 1"), out.stdout
+
+
 def test_scale_of_a_product_that_rounds_to_zero(tmp_path):
     """q_exponent from v^H A v known to two units a row: the root of the true value, and so the
     update vectors, stay within a factor of two of the scale."""
