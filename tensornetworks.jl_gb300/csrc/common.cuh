@@ -83,8 +83,8 @@ struct Ctx {
     // mixed precision on: environment updates and truncation projections run
     // on the tensor cores (set for the duration of a mixed-precision sweep)
     bool mixed = false;
-    // split-K FP64 GEMMs draw partial buffers from the pool; callers that must
-    // not allocate turn them off
+    // split-K partials and the tensor-core products' planes draw scratch;
+    // callers that must not allocate turn both off
     bool splitk = true;
     // FP64 DMRG: small splits and sums keep one order of operations, so that its
     // results are the same to the last bit in every version (eig_fp64.cu)
@@ -233,8 +233,10 @@ void small_apply(Ctx* ctx, const cplx* in, cplx* out, const cplx* M, int nI, int
 
 // out[j] = <v_j, w> for K vectors; result left in device memory dout (K cplx).
 void multi_dot(Ctx* ctx, const cplx* const* dV, int K, const cplx* w, int64_t n, cplx* dout);
-// w += sum_j coef[j] * v_j, coef on the device (K cplx); sign applied to coefs.
+// w orthogonalised against the v_j in two passes and normalised: the summed components
+// in comp, the norm returned; waits for the stream.
 double lanczos_orth(Ctx* ctx, const cplx* const* hV, int K, cplx* w, int64_t n, cplx* comp);
+// w += sum_j coef[j] * v_j, coef on the device (K cplx); sign applied to coefs.
 void multi_axpy(Ctx* ctx, cplx* w, const cplx* const* dV, const cplx* dcoef, int K, int64_t n,
                 double sign);
 void zscale(Ctx* ctx, cplx* x, int64_t n, cplx a);

@@ -24,8 +24,8 @@
 // What it replaced is serial in the order: a Sturm count is n steps of four FP64
 // instructions of 64 clocks each, an inverse iteration six such sweeps, the QR
 // of the vectors n grid barriers; at order 256, 128 vectors: bisection 1,071 us,
-// inverse iteration 731, QR and its Q 1,114.  Here all of it takes 72 us at order
-// 32, 94 at 64, 152 at 128, 210 at 256.
+// inverse iteration 731, QR and its Q 1,114.  Here all of it takes 69 us at order
+// 32, 92 at 64, 153 at 128, 195 at 256.
 //
 // A level is a chain of FP64 instructions that cost the same for one lane as for
 // 32, so a warp finds several roots at once where merges are small (32 / K lanes),

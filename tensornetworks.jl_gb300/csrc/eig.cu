@@ -13,7 +13,8 @@
 // GB300 issues FP64 at two FMAs per clock per SM and each FP64 instruction of a
 // warp takes 64 clocks, so serial recurrences and reductions cost most; steps 1
 // and 2 say how each avoids them.  Order 16 with 8 vectors takes 0.15 ms, 64 with 32
-// 0.41, 128 with 64 0.86, 256 with 128 2.3 (reduction 1.9), 512 with 256 5.4 (4.4).
+// 0.43, 128 with 64 0.86, 256 with 128 2.3 (reduction 1.8), 512 with 256 5.1 (4.2).
+// Small splits of FP64 DMRG keep another solver, for their values (eig_fp64.cu).
 #include <cmath>
 
 #include "common.cuh"

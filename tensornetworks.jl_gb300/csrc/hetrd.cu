@@ -25,7 +25,9 @@
 // 32-bit limbs, the new exponent of row j+1 from the last step's smallest exponent
 // (so that w needs one pass) and work that nobody waits for behind the exchange took
 // order 64 from 308 to 245 us, 128 from 699 to 571, 256 from 2,069 to 1,646, 512
-// from 6,574 to 3,830, 1024 from 21.3 to 12.0 ms, 2048 from 98 to 58 ms.
+// from 6,574 to 3,830, 1024 from 21.3 to 12.0 ms, 2048 from 98 to 58 ms.  With all bounds
+// of the update vectors' scale (q_exponent) they take 262, 577, 1,826 and 4,198 us, 13.0
+// and 59.6 ms.
 //
 // Reflector j is kept as V[j n + i] (i > j, the first entry explicit) and tau[j]:
 // H_j = I - tau_j v_j v_j^H.  Results become FP64 while the exchange travels, or by
@@ -798,8 +800,9 @@ void hetrd(Ctx* ctx, const cplx* G, int64_t n, double* d, double* e, cplx* tau, 
     // Blocks of the cluster: the row work of a step (n^2 / 3 entries on average at
     // 180 clocks per 32) against the exchange with more blocks.  The grid's barrier
     // and vectors through L2 cost 4 us a step more, its rows next to nothing: order
-    // 160 takes 837 us in a cluster and 1,069 on the grid, 200 1,179 and 1,329, 256
-    // 1,900 and 1,646.
+    // 160 took 837 us in a cluster and 1,069 on the grid, 200 1,179 and 1,329, 256
+    // 1,900 and 1,646 when the line was drawn (now 200 takes 1,210 in its cluster, 256
+    // 1,826 on the grid).
     int64_t C = n <= 16 ? 1 : n <= 32 ? 4 : n <= 64 ? 8 : HC;
     const bool grid = n > 208 || ctx->trd_clusters == 0;
     if (grid) C = ctx->sm_count;

@@ -3,10 +3,12 @@
 // shuffles) and the truncation keep rule.
 //
 // GB300 executes FP64 on the SIMT pipes at a small fraction of its tensor
-// rate, so these kernels are compute-bound at modest tile sizes: a 64x64
-// complex tile per 256-thread block with a 4x4 complex register tile per
-// thread keeps the DFMA pipe busy while shared-memory traffic stays far below
-// its bandwidth.
+// rate.  Large products of the library's own paths therefore run on the
+// tensor cores (tc_zgemm.cu, chosen by tc_sized).  Here are the small ones,
+// one output per thread or group of lanes, and a 64x64 complex tile per
+// 256-thread block with a 4x4 complex register tile per thread, which keeps
+// the DFMA pipe busy: it serves products that a caller wants on FP64 units
+// and those whose operand planes find no room.
 #include "common.cuh"
 #include "grid_dev.cuh"
 
@@ -913,8 +915,8 @@ void zgemm_fp64(Ctx* ctx, Op opa, Op opb, int64_t m, int64_t n, int64_t k, cplx 
         TN_CHECK_CUDA(cudaGetLastError());
         return;
     }
-    // Split K when the tiles cannot fill the SMs (the Gram and projection
-    // products of bond dimensions 128-512): S chunks of at least 128, each
+    // Split K when the tiles cannot fill the SMs (a long
+    // inner dimension under a small result): S chunks of at least 128, each
     // into its own partial, summed in chunk order by a second kernel.
     const int64_t tiles = (int64_t)grid.x * grid.y;
     int64_t S = 1;
